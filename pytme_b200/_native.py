@@ -36,7 +36,7 @@ EXPORTED = (
     "tm_version", "tm_last_error", "tm_set_device_memory_limit", "tm_rigid_transform", "tm_normalize_template_workspace",
     "tm_normalize_template", "tm_norm_scores", "tm_max_score_over_rotations",
     "tm_fft_plan_create", "tm_fft_plan_destroy", "tm_fft_r2c", "tm_fft_c2r",
-    "tm_scan_create", "tm_scan_destroy", "tm_scan_device_bytes", "tm_scan_set_template",
+    "tm_scan_create", "tm_scan_create_any_length", "tm_scan_destroy", "tm_scan_device_bytes", "tm_scan_set_template",
     "tm_scan_set_target", "tm_scan_run", "tm_scan_set_timing", "tm_scan_set_graph",
     "tm_scan_get_timing",
     "tm_scan_stage_bytes", "tm_max_filter_peaks",
@@ -115,6 +115,7 @@ def _load():
         "tm_fft_r2c": (c_int, [vp, vp, vp, vp]),
         "tm_fft_c2r": (c_int, [vp, vp, vp, c_double, vp]),
         "tm_scan_create": (c_int, [POINTER(ScanDesc), POINTER(c_void_p)]),
+        "tm_scan_create_any_length": (c_int, [POINTER(ScanDesc), POINTER(c_void_p)]),
         "tm_scan_destroy": (c_int, [vp]),
         "tm_scan_device_bytes": (c_int64, [vp]),
         "tm_scan_set_template": (c_int, [vp, f32p, f32p, f32p, vp]),

@@ -14,6 +14,7 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
@@ -44,7 +45,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     nvcc = _nvcc()
     os.makedirs(BUILD, exist_ok=True)
     hdr = _newest_header()
-    objs, changed = [], force or not os.path.exists(LIB)
+    objs, jobs, changed = [], [], force or not os.path.exists(LIB)
     for src in sorted(glob.glob(os.path.join(CSRC, "*.cu"))):
         obj = os.path.join(BUILD, os.path.basename(src)[:-3] + ".o")
         objs.append(obj)
@@ -54,8 +55,12 @@ def build(force: bool = False, verbose: bool = False) -> str:
         cmd = [nvcc, *ARCH, *FLAGS, "-I", INCLUDE, "-I", CSRC, "-c", src, "-o", obj]
         if verbose:
             print(" ".join(cmd), flush=True)
-        subprocess.check_call(cmd)
+        jobs.append((os.path.getsize(src), cmd))
         changed = True
+    # one nvcc per source, several at a time: the line-FFT passes compile every radix
+    with ThreadPoolExecutor(max_workers=max(1, min(8, os.cpu_count() or 1))) as pool:
+        for done in [pool.submit(subprocess.check_call, cmd) for _, cmd in sorted(jobs, reverse=True)]:
+            done.result()
     if changed:
         cmd = [nvcc, *ARCH, "-shared", "-o", LIB, *objs, "-lcufft", "-lcudart"]
         if verbose:

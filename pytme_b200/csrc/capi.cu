@@ -198,6 +198,15 @@ int tm_scan_create(const tm_scan_desc* desc, tm_scan** plan) {
   return TM_OK;
 }
 
+int tm_scan_create_any_length(const tm_scan_desc* desc, tm_scan** plan) {
+  TM_REQUIRE(plan, "tm_scan_create_any_length: null plan pointer");
+  *plan = nullptr;
+  tmb::Scan* impl = nullptr;
+  TM_TRY(tmb::scan_create(desc, &impl, true));
+  *plan = new tm_scan{impl};
+  return TM_OK;
+}
+
 int tm_scan_destroy(tm_scan* plan) {
   if (!plan) return TM_OK;
   tmb::scan_destroy(plan->impl);

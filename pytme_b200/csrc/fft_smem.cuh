@@ -320,8 +320,9 @@ __device__ __forceinline__ void fft_lines_ct(float2* buf, int nlines, int ls, in
 }
 
 // ---- small DFTs of compile-time size in registers (DIR -1 forward, +1 inverse)
-// 16 = 4 x 4 Cooley-Tukey with its constant twiddles; 6, 10, 12, 15, 20 = Good-Thomas
-// prime-factor forms (coprime factors, no twiddles).
+// 16 = 4 x 4 and 9 = 3 x 3 Cooley-Tukey with their constant twiddles; 7, 11, 13 by the
+// symmetry of an odd prime; 6, 10, 12, 14, 15, 20 = Good-Thomas prime-factor forms (coprime
+// factors, no twiddles).
 template <int DIR>
 __device__ __forceinline__ void dft16(float2* v) {
   const float c1 = 0.92387953251128675613f, s1 = 0.38268343236508977173f;
@@ -354,6 +355,86 @@ __device__ __forceinline__ void dft16(float2* v) {
   }
 }
 
+// 9 = 3 x 3 Cooley-Tukey with its constant twiddles w9^1, w9^2, w9^4.
+template <int DIR>
+__device__ __forceinline__ void dft9(float2* v) {
+  const float sg = DIR < 0 ? -1.f : 1.f;
+  const float2 w1 = make_float2(0.76604444311897803520f, sg * 0.64278760968653932632f);
+  const float2 w2 = make_float2(0.17364817766693034885f, sg * 0.98480775301220805937f);
+  const float2 w4 = make_float2(-0.93969262078590838405f, sg * 0.34202014332566873304f);
+  float2 a[3][3];
+#pragma unroll
+  for (int n1 = 0; n1 < 3; ++n1) {
+#pragma unroll
+    for (int n2 = 0; n2 < 3; ++n2) a[n1][n2] = v[3 * n2 + n1];
+    dft3<DIR>(a[n1]);
+  }
+  a[1][1] = cmul(a[1][1], w1);
+  a[1][2] = cmul(a[1][2], w2);
+  a[2][1] = cmul(a[2][1], w2);
+  a[2][2] = cmul(a[2][2], w4);
+#pragma unroll
+  for (int k2 = 0; k2 < 3; ++k2) {
+    float2 b[3] = {a[0][k2], a[1][k2], a[2][k2]};
+    dft3<DIR>(b);
+#pragma unroll
+    for (int k1 = 0; k1 < 3; ++k1) v[k2 + 3 * k1] = b[k1];
+  }
+}
+
+// Odd prime P by its symmetry: with a_k = v[k] + v[P-k], b_k = v[k] - v[P-k],
+// X[j], X[P-j] = v[0] + sum_k cos(2 pi jk/P) a_k  +- DIR i sum_k sin(2 pi jk/P) b_k.
+template <int P, int DIR>
+__device__ __forceinline__ void dft_odd_prime(float2* v) {
+  static_assert(P == 7 || P == 11 || P == 13, "unsupported prime");
+  constexpr int H = (P - 1) / 2;
+  // cos and sin of 2 pi j / P
+  const float c7[4] = {1.f, 0.62348980185873353053f, -0.22252093395631440429f,
+                       -0.90096886790241912624f};
+  const float s7[4] = {0.f, 0.78183148246802980871f, 0.97492791218182360702f,
+                       0.43388373911755812048f};
+  const float c11[6] = {1.f, 0.84125353283118116886f, 0.41541501300188642553f,
+                        -0.14231483827328514044f, -0.65486073394528506406f,
+                        -0.95949297361449738989f};
+  const float s11[6] = {0.f, 0.54064081745559758211f, 0.90963199535451837141f,
+                        0.98982144188093273237f, 0.75574957435425828378f,
+                        0.28173255684142969771f};
+  const float c13[7] = {1.f, 0.88545602565320989590f, 0.56806474673115580251f,
+                        0.12053668025532305335f, -0.35460488704253562597f,
+                        -0.74851074817110109863f, -0.97094181742605202716f};
+  const float s13[7] = {0.f, 0.46472317204376854566f, 0.82298386589365639458f,
+                        0.99270887409805399280f, 0.93501624268541482344f,
+                        0.66312265824079520238f, 0.23931566428755776715f};
+  float2 a[H + 1], b[H + 1];
+  float2 sum = v[0];
+#pragma unroll
+  for (int k = 1; k <= H; ++k) {
+    a[k] = cadd(v[k], v[P - k]);
+    b[k] = csub(v[k], v[P - k]);
+    sum = cadd(sum, a[k]);
+  }
+  const float2 v0 = v[0];
+#pragma unroll
+  for (int j = 1; j <= H; ++j) {
+    float2 m = v0, n = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int k = 1; k <= H; ++k) {
+      const int e = (j * k) % P;
+      const int f = e <= H ? e : P - e;
+      const float c = P == 7 ? c7[f & 3] : P == 11 ? c11[f % 6] : c13[f];
+      const float s = (DIR < 0 ? -1.f : 1.f) * (e <= H ? 1.f : -1.f) *
+                      (P == 7 ? s7[f & 3] : P == 11 ? s11[f % 6] : s13[f]);
+      m.x += c * a[k].x;
+      m.y += c * a[k].y;
+      n.x -= s * b[k].y;  // i s b
+      n.y += s * b[k].x;
+    }
+    v[j] = cadd(m, n);
+    v[P - j] = csub(m, n);
+  }
+  v[0] = sum;
+}
+
 constexpr int modinv(int a, int m) {
   for (int x = 1; x < m; ++x)
     if ((a * x) % m == 1) return x;
@@ -366,6 +447,7 @@ __device__ __forceinline__ void dft_prime_or_pow2(float2* v) {
   else if constexpr (R == 3) dft3<DIR>(v);
   else if constexpr (R == 4) dft4<DIR>(v);
   else if constexpr (R == 5) dft5<DIR>(v);
+  else if constexpr (R == 7 || R == 11 || R == 13) dft_odd_prime<R, DIR>(v);
   else if constexpr (R == 8) dft8<DIR>(v);
   else dft16<DIR>(v);
 }
@@ -396,9 +478,12 @@ __device__ __forceinline__ void dft_pfa(float2* v) {
 template <int N, int DIR>
 __device__ __forceinline__ void dft_small(float2* v) {
   if constexpr (N == 1) {
-  } else if constexpr (N == 2 || N == 3 || N == 4 || N == 5 || N == 8 || N == 16) {
+  } else if constexpr (N == 2 || N == 3 || N == 4 || N == 5 || N == 7 || N == 8 || N == 11 ||
+                       N == 13 || N == 16) {
     dft_prime_or_pow2<N, DIR>(v);
-  } else if constexpr (N == 6) dft_pfa<2, 3, DIR>(v);
+  } else if constexpr (N == 9) dft9<DIR>(v);
+  else if constexpr (N == 14) dft_pfa<2, 7, DIR>(v);
+  else if constexpr (N == 6) dft_pfa<2, 3, DIR>(v);
   else if constexpr (N == 10) dft_pfa<2, 5, DIR>(v);
   else if constexpr (N == 12) dft_pfa<4, 3, DIR>(v);
   else if constexpr (N == 15) dft_pfa<3, 5, DIR>(v);

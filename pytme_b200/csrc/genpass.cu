@@ -1,0 +1,68 @@
+// Plans, tiles and shared memory of the fused scan passes over axes of any length.
+#include "genpass_dev.cuh"
+
+namespace tmb {
+
+namespace {
+
+size_t smem_template(const Plan& p, int w, int t1, int t2) {
+  return 16 * p.pairs + sizeof(float2) * (size_t)w * (p.rows + t1 + t2) +
+         sizeof(float) * (size_t)t1 * (t2 | 1);
+}
+// the tile, the target's column and two buffers of t0 inputs; for FLC three tiles
+size_t smem_x(const Plan& p, int w, int t0, bool flc) {
+  return 16 * p.pairs + sizeof(float2) * (size_t)w * (flc ? 3 * p.rows : 2 * (p.rows + t0));
+}
+size_t even_tile(const Plan& p, int w, int tiles) {
+  return 16 * p.pairs + sizeof(float2) * (((size_t)w * p.rows * tiles + 1) & ~(size_t)1);
+}
+size_t smem_y(const Plan& p, int w, size_t elem) { return even_tile(p, w, 1) + elem * w * p.n; }
+// z pass: tiles, the staged rows, and per voxel of 2 w rows the maximum, its rotation and (not
+// for FLC) the inverse denominator
+size_t smem_z(const Plan& p, int w, int hp, bool flc, bool half) {
+  const size_t wide = sizeof(float2) * staged_pitch<float2>(hp);
+  const size_t own = half ? sizeof(__half2) * staged_pitch<__half2>(hp) : wide;
+  return even_tile(p, w, flc ? 3 : 1) + 2 * w * ((flc ? 2 * wide : 0) + own) +
+         2 * (size_t)w * z_pitch(p.n) * (flc ? 6 : 10);
+}
+
+}  // namespace
+
+GenConfig gen_config(int n0, int n1, int n2, int t0, int t1, int t2, int hp, bool flc, bool half) {
+  GenConfig c;
+  // the most lines, up to eight, whose tile fits
+  auto pick = [](GenTile& g, int n, int regs, auto size) {
+    g.plan = make_plan(n);
+    if (!g.plan.ns) return false;
+    for (int lines : {8, 4, 2, 1}) {
+      g.plan.w = lines;
+      g.smem = size(g.plan, lines);
+      if (g.smem <= kSmemMax) {
+        choose_slots(g.plan, g.smem, regs);
+        return true;
+      }
+    }
+    return false;
+  };
+  c.ok = pick(c.t, n1, 80, [&](const Plan& p, int w) { return smem_template(p, w, t1, t2); }) &&
+         pick(c.x, n0, flc ? 128 : 80,
+              [&](const Plan& p, int w) { return smem_x(p, w, t0, flc); }) &&
+         pick(c.y, n1, 80, [&](const Plan& p, int w) { return smem_y(p, w, 8); }) &&
+         pick(c.z, n2, 80, [&](const Plan& p, int w) { return smem_z(p, w, hp, flc, half); });
+  if (c.ok) c.smem_y_half = smem_y(c.y.plan, c.y.plan.w, 4);
+  return c;
+}
+
+int gen_prepare_cols(const GenConfig& c, bool half);
+int gen_prepare_x(const GenConfig& c, bool half);
+int gen_prepare_xflc(const GenConfig& c, bool half);
+int gen_prepare_z(const GenConfig& c, bool half);
+int gen_prepare_zflc(const GenConfig& c, bool half);
+
+int gen_prepare(const GenConfig& c, bool flc, bool half) {
+  TM_TRY(gen_prepare_cols(c, half));
+  TM_TRY(flc ? gen_prepare_xflc(c, half) : gen_prepare_x(c, half));
+  return flc ? gen_prepare_zflc(c, half) : gen_prepare_z(c, half);
+}
+
+}  // namespace tmb

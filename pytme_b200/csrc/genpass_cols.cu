@@ -1,0 +1,212 @@
+// Template rows and the y pass of the scan over axes of any length (see genpass_dev.cuh).
+#include "genpass_dev.cuh"
+#include "scan.cuh"
+
+namespace tmb {
+
+namespace {
+
+// ------------------------------------------------------------------ template pass
+// grid (hp / w, ceil(t0 / kXPlanes), nb). Direct real DFT along z of the t1 x t2 plane for
+// the tile's w columns (t2 of n2 inputs are non-zero), then the zero-padded FFT along y.
+template <int W>
+__global__ void __launch_bounds__(kMaxThreads, 2)
+gen_template_kernel(const float* __restrict__ tmpl, int t0, int t1, int t2, int n2, int h2,
+                    const Plan p, const float4* __restrict__ tw1_g,
+                    const float2* __restrict__ tw2_g, float2* __restrict__ G) {
+  extern __shared__ float4 smem_raw[];
+  const int w = lines<W>(p), tid = threadIdx.x, nt = blockDim.x, l = tid % w, slot = tid / w;
+  float4* tw = smem_raw;
+  float2* sm = reinterpret_cast<float2*>(tw + p.pairs);
+  float2* twz = sm + p.rows * w;   // t2 x w roots of the tile's columns
+  float2* zrow = twz + t2 * w;     // t1 x w
+  float* plane = reinterpret_cast<float*>(zrow + t1 * w);
+  const int k2_0 = blockIdx.x * w, k2 = k2_0 + l, b = blockIdx.z;
+  const int pt = t2 | 1;  // odd row pitch of the plane
+  for (int i = tid; i < p.pairs; i += nt) tw[i] = tw1_g[i];
+  for (int i = tid; i < t2 * w; i += nt) {
+    const int z = i / w, c = k2_0 + i % w;
+    twz[i] = c < h2 ? tw2_g[(int)(((int64_t)z * c) % n2)] : make_float2(0.f, 0.f);
+  }
+  const int x1 = min(t0, (int)(blockIdx.y + 1) * kXPlanes);
+  for (int x = blockIdx.y * kXPlanes; x < x1; ++x) {
+    const float* src = tmpl + ((int64_t)b * t0 + x) * t1 * t2;
+    for (int y = slot; y < t1; y += p.slots)
+      for (int z = l; z < t2; z += w) plane[y * pt + z] = src[y * t2 + z];
+    __syncthreads();
+    for (int y = slot; y < t1; y += 4 * p.slots) {
+      float2 acc[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[i] = make_float2(0.f, 0.f);
+      if (y + p.slots < t1) {
+        int row[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) row[i] = min(y + i * p.slots, t1 - 1) * pt;
+        for (int z = 0; z < t2; ++z) {
+          const float2 rt = twz[z * w + l];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float a = plane[row[i] + z];
+            acc[i].x += a * rt.x;
+            acc[i].y += a * rt.y;
+          }
+        }
+      } else {
+        const float* row = plane + y * pt;
+        for (int z = 0; z < t2; ++z) {
+          const float2 rt = twz[z * w + l];
+          acc[0].x += row[z] * rt.x;
+          acc[0].y += row[z] * rt.y;
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (y + i * p.slots < t1) zrow[(y + i * p.slots) * w + l] = acc[i];
+    }
+    __syncthreads();
+    TM_RADIX(p.r[0], (first_stage<W, RR, -1, true>(p, sm, tw, l, slot, t1, [&](int q) {
+      return [a = zrow + q * w + l, step = p.lr[0] * w](int r) { return a[r * step]; };
+    })));
+    __syncthreads();
+    mid_stages<W, -1>(p, sm, tw, l, slot);
+    float2* dst = G + ((int64_t)b * t0 + x) * p.n * h2 + k2;
+    TM_RADIX(p.rl, (last_stage<W, RR, -1>(p, sm, l, slot,
+                                          [&](int q, const float2(&v)[RR], float2*) {
+      if (k2 >= h2) return;
+      float2* d = dst + (int64_t)out_base(p, q) * h2;
+      const int64_t step = (int64_t)(p.n / RR) * h2;
+      _Pragma("unroll")
+      for (int r = 0; r < RR; ++r) d[r * step] = v[r];
+    })));
+    // the next plane's first stage writes the tile after two more barriers
+  }
+}
+
+// Self test: y[i][:] = FFT_dir(x[i][:]) for w lines of length p.n, one CTA.
+__global__ void __launch_bounds__(kMaxThreads, 2)
+line_fft_test_kernel(const float2* x, float2* y, const Plan p, const float4* tw_g, int dir) {
+  extern __shared__ float4 smem_raw[];
+  const int w = p.w, tid = threadIdx.x, l = tid % w, slot = tid / w;
+  float4* tw = smem_raw;
+  float2* sm = reinterpret_cast<float2*>(tw + p.pairs);
+  for (int i = tid; i < p.pairs; i += blockDim.x) tw[i] = tw_g[i];
+  __syncthreads();
+  auto in = [&](int q) { return [&, q](int r) { return x[l * p.n + q + r * p.lr[0]]; }; };
+  if (dir < 0) TM_RADIX(p.r[0], (first_stage<0, RR, -1, false>(p, sm, tw, l, slot, 0, in)));
+  if (dir > 0) TM_RADIX(p.r[0], (first_stage<0, RR, 1, false>(p, sm, tw, l, slot, 0, in)));
+  __syncthreads();
+  if (dir < 0) mid_stages<0, -1>(p, sm, tw, l, slot);
+  else mid_stages<0, 1>(p, sm, tw, l, slot);
+  auto out = [&](int q, const auto& v, int n) {
+    const int k0 = out_base(p, q);
+    for (int r = 0; r < n; ++r) y[l * p.n + k0 + r * (p.n / n)] = v[r];
+  };
+  if (dir < 0)
+    TM_RADIX(p.rl, (last_stage<0, RR, -1>(p, sm, l, slot, [&](int q, const float2(&v)[RR],
+                                                              float2*) { out(q, v, RR); })));
+  if (dir > 0)
+    TM_RADIX(p.rl, (last_stage<0, RR, 1>(p, sm, l, slot, [&](int q, const float2(&v)[RR],
+                                                             float2*) { out(q, v, RR); })));
+}
+
+// ------------------------------------------------------------------ y pass
+// grid (hp / w, ceil(n0 / kYPlanes), nb): inverse FFT along y, in place. The next plane's
+// columns are copied to shared memory (16 bytes at a time) while the later stages of the
+// current one run.
+template <int W, typename HT>
+__global__ void __launch_bounds__(kMaxThreads, 2)
+gen_ypass_kernel(HT* __restrict__ H, int n0, const Plan p, const float4* __restrict__ tw_g,
+                 const HLayout hl) {
+  extern __shared__ float4 smem_raw[];
+  const int w = lines<W>(p), tid = threadIdx.x, nt = blockDim.x, l = tid % w, slot = tid / w;
+  float4* tw = smem_raw;
+  float2* sm = reinterpret_cast<float2*>(tw + p.pairs);
+  HT* stage = reinterpret_cast<HT*>(sm + ((p.rows * w + 1) & ~1));  // n x w
+  const int k2 = blockIdx.x * w;
+  const int x0 = blockIdx.y * kYPlanes, x1 = min(n0, x0 + kYPlanes);
+  HT* base = H + blockIdx.z * hl.sb + k2;
+  auto fetch = [&](const HT* src) {
+    if constexpr (W == 8) {
+      constexpr int PER = 16 / sizeof(HT), PIECES = 8 / PER;
+      const int piece = tid % PIECES * PER;
+      const int64_t step = nt / PIECES * hl.sr;
+      const HT* s = src + tid / PIECES * hl.sr + piece;
+      for (int row = tid / PIECES; row < p.n; row += nt / PIECES, s += step)
+        async_copy16(stage + row * 8 + piece, s);
+    } else {
+      for (int row = slot; row < p.n; row += p.slots) stage[row * w + l] = src[row * hl.sr + l];
+    }
+    async_commit();
+  };
+  fetch(base + x0 * hl.sx);
+  for (int i = tid; i < p.pairs; i += nt) tw[i] = tw_g[i];
+  for (int x = x0; x < x1; ++x) {
+    HT* col = base + x * hl.sx;
+    async_wait_all();
+    __syncthreads();  // plane x is in; the plane before has left the tile
+    TM_RADIX(p.r[0], (first_stage<W, RR, 1, false>(p, sm, tw, l, slot, 0, [&](int q) {
+      return [a = stage + q * w + l, step = p.lr[0] * w](int r) { return load_c<HT>(a + r * step); };
+    })));
+    __syncthreads();
+    if (x + 1 < x1) fetch(col + hl.sx);
+    mid_stages<W, 1>(p, sm, tw, l, slot);
+    TM_RADIX(p.rl, (last_stage<W, RR, 1>(p, sm, l, slot,
+                                         [&](int q, const float2(&v)[RR], float2*) {
+      HT* d = col + out_base(p, q) * hl.sr + l;
+      const int64_t step = (p.n / RR) * hl.sr;
+      _Pragma("unroll")
+      for (int r = 0; r < RR; ++r) store_c(d + r * step, v[r]);
+    })));
+  }
+}
+
+}  // namespace
+
+int gen_prepare_cols(const GenConfig& c, bool half) {
+  TM_LINES(c.t.plan, TM_TRY(raise(gen_template_kernel<WW>)));
+  TM_LINES(c.y.plan, TM_TRY((raise(gen_ypass_kernel<WW, float2>))));
+  if (half) TM_LINES(c.y.plan, TM_TRY((raise(gen_ypass_kernel<WW, __half2>))));
+  return TM_OK;
+}
+
+int gen_template(const GenConfig& c, const float* tmpl, int nb, int t0, int t1, int t2, int n1,
+                 int n2, int h2, int hp, const float4* tw1, const float2* tw2, float2* G,
+                 cudaStream_t st) {
+  const dim3 g(hp / c.t.plan.w, (unsigned)ceil_div(t0, kXPlanes), nb);
+  TM_LINES(c.t.plan, (gen_template_kernel<WW><<<g, c.t.threads(), c.t.smem, st>>>(
+                     tmpl, t0, t1, t2, n2, h2, c.t.plan, tw1, tw2, G)));
+  return check_launch("gen_template_kernel");
+}
+
+int gen_ypass(const GenConfig& c, void* H, bool half, int nb, int n0, int hp,
+              const float4* tw1, const HLayout& hl, cudaStream_t st) {
+  const dim3 g(hp / c.y.plan.w, (unsigned)ceil_div(n0, kYPlanes), nb);
+  TM_STORE(half, TM_LINES(c.y.plan, (gen_ypass_kernel<WW, HT><<<g, c.y.threads(), half ? c.smem_y_half : c.y.smem, st>>>(
+                                    static_cast<HT*>(H), n0, c.y.plan, tw1, hl))));
+  return check_launch("gen_ypass_kernel");
+}
+
+int line_fft_test(const void* x, void* y, int n, int lines, int dir, cudaStream_t st) {
+  Plan p = make_plan(n);
+  TM_REQUIRE(p.ns > 0, "line_fft_test: length %d not supported", n);
+  TM_REQUIRE(lines >= 1 && lines <= kMaxThreads && (int64_t)n * lines <= kMaxLength,
+             "line_fft_test: tile too large");
+  p.w = lines;
+  p.slots = std::max(1, std::min(kMaxSlots, kMaxThreads / lines));
+  const auto t = twiddle_rows(p);
+  const size_t smem = 16 * p.pairs + sizeof(float2) * (size_t)p.rows * lines;
+  float4* tw = nullptr;
+  TM_TRY(cuda_status(cudaMalloc(&tw, sizeof(float2) * t.size() + 16), "line_fft_test: alloc"));
+  cudaMemcpy(tw, t.data(), sizeof(float2) * t.size(), cudaMemcpyHostToDevice);
+  int rc = raise(line_fft_test_kernel);
+  if (rc == TM_OK) {
+    line_fft_test_kernel<<<1, p.slots * lines, smem, st>>>(
+        static_cast<const float2*>(x), static_cast<float2*>(y), p, tw, dir);
+    rc = check_launch("line_fft_test_kernel");
+  }
+  cudaStreamSynchronize(st);
+  cudaFree(tw);
+  return rc;
+}
+
+}  // namespace tmb

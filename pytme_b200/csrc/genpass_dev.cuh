@@ -1,0 +1,120 @@
+// What the kernels of the fused scan passes over axes of any length share. The passes of
+// scan.cu's scheme live in genpass_cols.cu (template rows, y pass), genpass_x.cu,
+// genpass_xflc.cu, genpass_z.cu and genpass_zflc.cu, one file each because every kernel
+// holds all radices; genpass.cu chooses plans and tiles.
+//
+// Every pass moves tiles of W = 8 neighbouring k2 columns (one 64-byte segment of complex64,
+// 32 bytes of half2). Tiles of fewer lines serve the lengths whose eight-line tile does not fit in shared memory.
+#pragma once
+
+#include <cuda_fp16.h>
+
+#include <algorithm>
+#include <type_traits>
+
+#include "common.cuh"
+#include "genpass.cuh"
+
+namespace tmb {
+
+using namespace linefft;
+
+namespace {
+
+constexpr int kMaxThreads = 8 * kMaxSlots;
+constexpr int kXPlanes = 4;  // x planes per CTA of the template pass
+constexpr int kYPlanes = 8;  // x' planes per CTA of the y pass
+constexpr size_t kSmemMax = 220 * 1024;
+
+template <typename T>
+__device__ __forceinline__ float2 load_c(const T* p);
+template <>
+__device__ __forceinline__ float2 load_c<float2>(const float2* p) { return *p; }
+template <>
+__device__ __forceinline__ float2 load_c<__half2>(const __half2* p) { return __half22float2(*p); }
+__device__ __forceinline__ void store_c(float2* p, float2 v) { *p = v; }
+__device__ __forceinline__ void store_c(__half2* p, float2 v) { *p = __float22half2_rn(v); }
+
+// asynchronous copies global -> shared
+__device__ __forceinline__ void async_copy8(void* smem, const void* gmem) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void async_copy16(void* smem, const void* gmem) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void async_commit() {
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+__device__ __forceinline__ void async_wait_all() {
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+}
+
+// Pitch of a staged H row, in elements: hp and 16 bytes, so that eight rows' values of four
+// neighbouring k fall on distinct banks.
+template <typename HT>
+__host__ __device__ constexpr int staged_pitch(int hp) {
+  return hp + 16 / (int)sizeof(HT);
+}
+
+// Stage `nrows` rows of hp values, sx apart, w lanes and `slots` rows at a time.
+template <typename HT>
+__device__ __forceinline__ void stage_rows(HT* dst, const HT* src, int nrows, int hp, int64_t sx,
+                                           int l, int w, int slot, int slots) {
+  constexpr int PER = 16 / sizeof(HT);
+  for (int rho = slot; rho < nrows; rho += slots)
+    for (int k = l * PER; k < hp; k += w * PER)
+      async_copy16(dst + rho * staged_pitch<HT>(hp) + k, src + rho * sx + k);
+}
+
+// c2r along z of two real lines by one complex FFT of length n2: with A and B the half
+// spectra of two rows (imaginary parts of bin 0 and, for even n2, of bin n2 / 2 dropped, as
+// numpy's irfft does), Z[k] = A[k] + i B[k] and Z[n2 - k] = conj(A[k]) + i conj(B[k]) have the
+// inverse transform a + i b. Any n2 works, odd ones included. Input r of a first-stage
+// butterfly q of radix R is Z[q + r * lr]: whether it is mirrored is known from r alone but
+// for the middle r of an odd R, and bins 0 and n2 / 2 can only be at r = 0 and r = R / 2.
+template <int R, typename TA, typename TB>
+__device__ __forceinline__ float2 pair_input(const TA* a, const TB* b, int q, int r, int lr,
+                                             int n2) {
+  const int i = q + r * lr;
+  const bool mirror = R % 2 && r == R / 2 ? 2 * i > n2 : r >= (R + 1) / 2;
+  const int k = mirror ? n2 - i : i;
+  float2 u = load_c<TA>(a + k), v = load_c<TB>(b + k);
+  if ((r == 0 && i == 0) || (r == R / 2 && 2 * i == n2)) { u.y = 0.f; v.y = 0.f; }
+  return mirror ? make_float2(u.x + v.y, v.x - u.y) : make_float2(u.x - v.y, u.y + v.x);
+}
+
+// pitch of a row of z voxels: 4 mod 32 words, so eight rows times four voxels are 32 banks
+inline int z_pitch(int n2) { return (n2 + 27) / 32 * 32 + 4; }
+
+// Rotations are split over more CTAs where the columns alone leave the chip idle: the
+// target's column is then read once per chunk, from the L2.
+inline int rotations_per_cta(int64_t columns, int nb) {
+  const int64_t want = 148 * 6;
+  const int64_t chunks = std::min<int64_t>(nb, std::max<int64_t>(1, want / columns));
+  return (int)ceil_div(nb, chunks);
+}
+
+#define TM_LINES(p, CALL)                                 \
+  do {                                                    \
+    if ((p).w == 8) { constexpr int WW = 8; CALL; }         \
+    else { constexpr int WW = 0; CALL; }                  \
+  } while (0)
+#define TM_STORE(half, CALL)                              \
+  do {                                                    \
+    if (half) { using HT = __half2; CALL; }               \
+    else { using HT = float2; CALL; }                     \
+  } while (0)
+
+template <class K>
+int raise(K kernel) {
+  return cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)kSmemMax),
+                     "shared memory limit");
+}
+
+
+}  // namespace
+
+}  // namespace tmb

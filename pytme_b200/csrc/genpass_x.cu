@@ -1,0 +1,97 @@
+// The x pass of the scan over axes of any length (see genpass_dev.cuh).
+#include "genpass_dev.cuh"
+
+namespace tmb {
+
+namespace {
+
+// grid (hp / w, n1, rotation chunks): forward FFT along x of the t0 non-zero rows, product
+// with the target spectrum, inverse FFT, H written. The column of the target, times the scale
+// of H, stays in shared memory for all rotations, in the order of the tile: the product reads
+// it at constant offsets. The next rotation's few input rows are copied in meanwhile.
+template <int W, typename HT>
+__global__ void __launch_bounds__(kMaxThreads, 2)
+gen_xpass_kernel(const float2* __restrict__ G, const float2* __restrict__ Ft, int B, int per,
+                 int t0, int n1, int h2, const Plan p, const float4* __restrict__ tw_g,
+                 float scale, HT* __restrict__ H, const HLayout hl) {
+  extern __shared__ float4 smem_raw[];
+  const int w = lines<W>(p), tid = threadIdx.x, nt = blockDim.x, l = tid % w, slot = tid / w;
+  float4* tw = smem_raw;
+  float2* sm = reinterpret_cast<float2*>(tw + p.pairs);
+  const int tile = p.rows * w;
+  float2* stage = sm + 2 * tile;  // two buffers of t0 x w inputs
+  const int k2 = blockIdx.x * w + l, k1 = blockIdx.y;
+  const bool valid = k2 < h2;  // the row padding is transformed as zeros
+  const int64_t row_s = (int64_t)n1 * h2;
+  const float2* g = G + (int64_t)k1 * h2 + k2;
+  const int b0 = blockIdx.z * per, b1 = min(B, b0 + per);
+  auto fetch = [&](int b) {
+    if (valid) {
+      const float2* src = g + ((int64_t)b * t0 + slot) * row_s;
+      float2* dst = stage + ((b & 1) * t0 + slot) * w + l;
+      for (int x = slot; x < t0; x += p.slots, src += p.slots * row_s, dst += p.slots * w)
+        async_copy8(dst, src);
+    }
+    async_commit();
+  };
+  fetch(b0);
+  for (int i = tid; i < p.pairs; i += nt) tw[i] = tw_g[i];
+  if (!valid)
+    for (int x = slot; x < 2 * t0; x += p.slots) stage[x * w + l] = make_float2(0.f, 0.f);
+  const float2* f = Ft + (int64_t)k1 * h2 + k2;
+  for (int q = slot; q < p.nb[p.ns - 1]; q += p.slots)
+    for (int r = 0; r < p.rl; ++r) {
+      const float2 c = valid ? f[(out_base(p, q) + r * p.nb[p.ns - 1]) * row_s]
+                             : make_float2(0.f, 0.f);
+      sm[tile + (q * p.pitch + r) * w + l] = make_float2(c.x * scale, c.y * scale);
+    }
+  async_wait_all();
+  __syncthreads();
+  for (int b = b0; b < b1; ++b) {
+    TM_RADIX(p.r[0], (first_stage<W, RR, -1, true>(p, sm, tw, l, slot, t0, [&](int q) {
+      return [a = stage + ((b & 1) * t0 + q) * w + l, step = p.lr[0] * w](int r) {
+        return a[r * step];
+      };
+    })));
+    if (b + 1 < b1) fetch(b + 1);
+    __syncthreads();
+    mid_stages<W, -1>(p, sm, tw, l, slot);
+    TM_RADIX(p.rl, (last_stage<W, RR, -1>(p, sm, l, slot, [&](int, float2(&v)[RR], float2* d) {
+      _Pragma("unroll")
+      for (int r = 0; r < RR; ++r) v[r] = fft::cmul(v[r], d[tile + r * w]);
+      fft::dft_small<RR, 1>(v);
+      _Pragma("unroll")
+      for (int r = 0; r < RR; ++r) d[r * w] = v[r];
+    })));
+    async_wait_all();  // the next inputs, for every thread after the barrier
+    __syncthreads();
+    mid_adjoints<W>(p, sm, tw, l, slot);
+    HT* h = H + b * hl.sb + k1 * hl.sr + k2;
+    // the next rotation's first stage writes the rows this thread reads here
+    TM_RADIX(p.r[0], (first_adjoint<W, RR>(p, sm, tw, l, slot, [&](int q) {
+      return [a = h + q * hl.sx, step = p.lr[0] * hl.sx](int r, float2 v) {
+        store_c(a + r * step, v);
+      };
+    })));
+  }
+}
+
+}  // namespace
+
+int gen_prepare_x(const GenConfig& c, bool half) {
+  TM_STORE(half, TM_LINES(c.x.plan, TM_TRY((raise(gen_xpass_kernel<WW, HT>)))));
+  return TM_OK;
+}
+
+int gen_xpass(const GenConfig& c, const float2* G, const float2* Ft, int nb, int t0, int n1,
+              int h2, int hp, const float4* tw0, float scale, void* H, bool half,
+              const HLayout& hl, cudaStream_t st) {
+  const int per = rotations_per_cta((int64_t)(hp / c.x.plan.w) * n1, nb);
+  const dim3 g(hp / c.x.plan.w, n1, (unsigned)ceil_div(nb, per));
+  TM_STORE(half, TM_LINES(c.x.plan, (gen_xpass_kernel<WW, HT><<<g, c.x.threads(), c.x.smem, st>>>(
+                                    G, Ft, nb, per, t0, n1, h2, c.x.plan, tw0, scale,
+                                    static_cast<HT*>(H), hl))));
+  return check_launch("gen_xpass_kernel");
+}
+
+}  // namespace tmb

@@ -1,0 +1,97 @@
+// The z pass of the scan over axes of any length (see genpass_dev.cuh).
+#include "genpass_dev.cuh"
+
+namespace tmb {
+
+namespace {
+
+// grid (n1, ceil(n0 / (2 w))): the rows (x', y') of 2 w consecutive x', all rotations of the
+// group. Row rho pairs with row rho + w. The running maximum, its rotation and the scaled
+// inverse denominator of the CTA's voxels stay in shared memory.
+template <int W, typename HT>
+__global__ void __launch_bounds__(kMaxThreads, 2)
+gen_zpass_kernel(const HT* __restrict__ H, int B, int n0, int n1, int n2, int hp,
+                 const Plan p, const float4* __restrict__ tw_g, float scale,
+                 const float* __restrict__ inv_den, int32_t first, const int32_t* __restrict__ first_dev,
+                 float* __restrict__ state_max, int32_t* __restrict__ state_rot,
+                 const HLayout hl, int zp) {
+  if (first_dev) first = *first_dev;
+  extern __shared__ float4 smem_raw[];
+  const int w = lines<W>(p), tid = threadIdx.x, nt = blockDim.x, l = tid % w, slot = tid / w;
+  const int rows2 = 2 * w;
+  float4* tw = smem_raw;
+  float2* sm = reinterpret_cast<float2*>(tw + p.pairs);
+  const int pitch = staged_pitch<HT>(hp);
+  HT* rows = reinterpret_cast<HT*>(sm + ((p.rows * w + 1) & ~1));  // rows2 staged rows
+  float* den = reinterpret_cast<float*>(rows + rows2 * pitch);
+  float* best = den + rows2 * zp;
+  uint16_t* arg = reinterpret_cast<uint16_t*>(best + rows2 * zp);
+  const int y = blockIdx.x, x0 = blockIdx.y * rows2, nrows = min(rows2, n0 - x0);
+  const HT* src = H + x0 * hl.sx + y * hl.sr;
+  stage_rows<HT>(rows, src, nrows, hp, hl.sx, l, w, slot, p.slots);
+  async_commit();
+  // rows past the edge repeat the last one; their voxels are not stored
+  const HT *ha = rows + min(l, nrows - 1) * pitch, *hb = rows + min(l + w, nrows - 1) * pitch;
+  for (int i = tid; i < p.pairs; i += nt) tw[i] = tw_g[i];
+  for (int rho = slot; rho < rows2; rho += p.slots)
+    for (int z = l; z < n2; z += w) {
+      const int64_t v = ((int64_t)(x0 + rho) * n1 + y) * n2 + z;
+      den[rho * zp + z] = (inv_den && rho < nrows ? inv_den[v] : 1.f) * scale;
+      best[rho * zp + z] = -INFINITY;
+    }
+  for (int b = 0; b < B; ++b) {
+    async_wait_all();
+    __syncthreads();  // rotation b's rows are in; the tile is free
+    TM_RADIX(p.r[0], (first_stage<W, RR, 1, false>(p, sm, tw, l, slot, 0, [&](int q) {
+      return [=, lr = p.lr[0]](int r) { return pair_input<RR>(ha, hb, q, r, lr, n2); };
+    })));
+    __syncthreads();
+    if (b + 1 < B) {
+      stage_rows<HT>(rows, src + (b + 1) * hl.sb, nrows, hp, hl.sx, l, w, slot, p.slots);
+      async_commit();
+    }
+    mid_stages<W, 1>(p, sm, tw, l, slot);
+    TM_RADIX(p.rl, (last_stage<W, RR, 1>(p, sm, l, slot,
+                                         [&](int q, const float2(&v)[RR], float2*) {
+      const int at = l * zp + out_base(p, q), step = n2 / RR, half = w * zp;
+      _Pragma("unroll")
+      for (int r = 0; r < RR; ++r) {
+        const int i = at + r * step, j = i + half;
+        const float s0 = v[r].x * den[i], s1 = v[r].y * den[j];
+        if (s0 > best[i]) { best[i] = s0; arg[i] = (uint16_t)b; }
+        if (s1 > best[j]) { best[j] = s1; arg[j] = (uint16_t)b; }
+      }
+    })));
+  }
+  __syncthreads();
+  for (int rho = slot; rho < nrows; rho += p.slots)
+    for (int z = l; z < n2; z += w) {
+      const int64_t v = ((int64_t)(x0 + rho) * n1 + y) * n2 + z;
+      const float s = best[rho * zp + z];
+      if (s > state_max[v]) {
+        state_max[v] = s;
+        state_rot[v] = first + (int32_t)arg[rho * zp + z];
+      }
+    }
+}
+
+}  // namespace
+
+int gen_prepare_z(const GenConfig& c, bool half) {
+  TM_STORE(half, TM_LINES(c.z.plan, TM_TRY((raise(gen_zpass_kernel<WW, HT>)))));
+  return TM_OK;
+}
+
+int gen_zpass(const GenConfig& c, const void* H, bool half, int nb, int n0, int n1, int n2,
+              int hp, const float4* tw2, float scale, const float* inv_den, int32_t first,
+              const int32_t* first_dev, float* state_max, int32_t* state_rot, const HLayout& hl,
+              cudaStream_t st) {
+  const dim3 g(n1, (unsigned)ceil_div(n0, 2 * c.z.plan.w));
+  TM_STORE(half, TM_LINES(c.z.plan, (gen_zpass_kernel<WW, HT><<<g, c.z.threads(), c.z.smem, st>>>(
+                                    static_cast<const HT*>(H), nb, n0, n1, n2, hp,
+                                    c.z.plan, tw2, scale, inv_den, first, first_dev, state_max, state_rot, hl,
+                                    z_pitch(n2)))));
+  return check_launch("gen_zpass_kernel");
+}
+
+}  // namespace tmb

@@ -1,0 +1,140 @@
+// The z pass of the FLC scan over axes of any length (see genpass_dev.cuh).
+#include "genpass_dev.cuh"
+
+namespace tmb {
+
+namespace {
+
+// Grid (n1, ceil(n0 / (2 w))): the rows (x', y') of 2 w consecutive x', all rotations of the
+// group; three complex transforms a rotation for each two rows rho and rho + w: (local mean,
+// local mean square) of either row as a pair, and the numerators of both rows as the third.
+// The thread that ends with two rows' numerators also holds their statistics. Only values of
+// one rotation share a transform: a rotation whose template normalises to NaN (an empty
+// rotated mask) leaves the others alone. Variance and quotient in double, as norm_scores
+// takes them (tme/backends/npfftw_backend.py:537-587), the quotient by rsqrt.
+template <int W, typename HT>
+__global__ void __launch_bounds__(kMaxThreads, 2)
+gen_zpass_flc_kernel(const HT* __restrict__ Ht, const float2* __restrict__ Hm,
+                     const float2* __restrict__ Hm2, int B, int n0, int n1, int n2, int hp,
+                     const Plan p, const float4* __restrict__ tw_g, float scale_t, float scale_m,
+                     const double* __restrict__ stats, double eps, int32_t first,
+                     const int32_t* __restrict__ first_dev, float* __restrict__ state_max,
+                     int32_t* __restrict__ state_rot, const HLayout hl, int zp) {
+  if (first_dev) first = *first_dev;
+  extern __shared__ float4 smem_raw[];
+  const int w = lines<W>(p), tid = threadIdx.x, nt = blockDim.x, l = tid % w, slot = tid / w;
+  const int rows2 = 2 * w;
+  float4* tw = smem_raw;
+  // tiles: statistics of rows 0..w-1, of rows w..2w-1, numerators
+  float2* sm = reinterpret_cast<float2*>(tw + p.pairs);
+  const int tile = p.rows * w;
+  const int pm = staged_pitch<float2>(hp), pt = staged_pitch<HT>(hp);
+  float2* rm = sm + ((3 * tile + 1) & ~1);  // staged rows of Hm, of Hm2, of Ht
+  float2* rm2 = rm + rows2 * pm;
+  HT* rt = reinterpret_cast<HT*>(rm2 + rows2 * pm);
+  float* best = reinterpret_cast<float*>(rt + rows2 * pt);
+  uint16_t* arg = reinterpret_cast<uint16_t*>(best + rows2 * zp);
+  const int y = blockIdx.x, x0 = blockIdx.y * rows2, nrows = min(rows2, n0 - x0);
+  const int64_t off = x0 * hl.sx + y * hl.sr;
+  auto stage = [&](int b) {
+    const int64_t o = off + b * hl.sb;
+    stage_rows<float2>(rm, Hm + o, nrows, hp, hl.sx, l, w, slot, p.slots);
+    stage_rows<float2>(rm2, Hm2 + o, nrows, hp, hl.sx, l, w, slot, p.slots);
+    stage_rows<HT>(rt, Ht + o, nrows, hp, hl.sx, l, w, slot, p.slots);
+    async_commit();
+  };
+  stage(0);
+  // rows past the edge repeat the last one; their voxels are not stored
+  const int ra = min(l, nrows - 1), rb = min(l + w, nrows - 1);
+  for (int i = tid; i < p.pairs; i += nt) tw[i] = tw_g[i];
+  for (int i = tid; i < rows2 * zp; i += nt) best[i] = -INFINITY;
+  const double eps2 = eps * eps;
+  for (int b = 0; b < B; ++b) {
+    async_wait_all();
+    __syncthreads();  // rotation b's rows are in; the tiles are free
+    TM_RADIX(p.r[0], ({
+      first_stage<W, RR, 1, false>(p, sm, tw, l, slot, 0, [&](int q) {
+        return [=, lr = p.lr[0]](int r) {
+          return pair_input<RR>(rm + ra * pm, rm2 + ra * pm, q, r, lr, n2);
+        };
+      });
+      first_stage<W, RR, 1, false>(p, sm + tile, tw, l, slot, 0, [&](int q) {
+        return [=, lr = p.lr[0]](int r) {
+          return pair_input<RR>(rm + rb * pm, rm2 + rb * pm, q, r, lr, n2);
+        };
+      });
+      first_stage<W, RR, 1, false>(p, sm + 2 * tile, tw, l, slot, 0, [&](int q) {
+        return [=, lr = p.lr[0]](int r) {
+          return pair_input<RR>(rt + ra * pt, rt + rb * pt, q, r, lr, n2);
+        };
+      });
+    }));
+    __syncthreads();
+    if (b + 1 < B) stage(b + 1);
+    for (int s = 1; s < p.ns - 1; ++s) {
+      TM_RADIX(p.r[s], ({
+        for (int i = 0; i < 3; ++i) mid_stage<W, RR, 1>(p, s, sm + i * tile, tw, l, slot);
+      }));
+      __syncthreads();
+    }
+    const double nobs = stats[b * 4 + 2];
+    const double sm_n = (double)scale_m / nobs, st_n = (double)scale_t / nobs;
+    // st = (CC(f, m), CC(f^2, m)), u the numerator
+    auto update = [&](int i, float2 st, float u) {
+      const double e1 = (double)st.x * sm_n, var = (double)st.y * sm_n - e1 * e1;
+      const double inv = var >= eps2 ? rsqrt(var) : 1.0;
+      const float s = (float)((double)u * st_n * inv);
+      if (s > best[i]) { best[i] = s; arg[i] = (uint16_t)b; }
+    };
+    TM_RADIX(p.rl, ({
+      for (int i = 0; i < 2; ++i)
+        last_stage<W, RR, 1>(p, sm + i * tile, l, slot,
+                             [&](int, const float2(&v)[RR], float2* d) {
+          _Pragma("unroll")
+          for (int r = 0; r < RR; ++r) d[r * w] = v[r];
+        });
+      last_stage<W, RR, 1>(p, sm + 2 * tile, l, slot,
+                           [&](int q, const float2(&v)[RR], float2* d) {
+        const int at = l * zp + out_base(p, q);
+        _Pragma("unroll")
+        for (int r = 0; r < RR; ++r) {
+          const int i = at + r * (n2 / RR);
+          update(i, d[r * w - 2 * tile], v[r].x);
+          update(i + w * zp, d[r * w - tile], v[r].y);
+        }
+      });
+    }));
+  }
+  __syncthreads();
+  for (int rho = slot; rho < nrows; rho += p.slots)
+    for (int z = l; z < n2; z += w) {
+      const int64_t v = ((int64_t)(x0 + rho) * n1 + y) * n2 + z;
+      const float s = best[rho * zp + z];
+      if (s > state_max[v]) {
+        state_max[v] = s;
+        state_rot[v] = first + (int32_t)arg[rho * zp + z];
+      }
+    }
+}
+
+}  // namespace
+
+int gen_prepare_zflc(const GenConfig& c, bool half) {
+  TM_STORE(half, TM_LINES(c.z.plan, TM_TRY((raise(gen_zpass_flc_kernel<WW, HT>)))));
+  return TM_OK;
+}
+
+int gen_zpass_flc(const GenConfig& c, const void* Ht, bool half, const float2* Hm,
+                  const float2* Hm2, int nb, int n0, int n1, int n2, int hp, const float4* tw2,
+                  float scale_t, float scale_m, const double* stats, double eps, int32_t first,
+                  const int32_t* first_dev, float* state_max, int32_t* state_rot,
+                  const HLayout& hl, cudaStream_t st) {
+  const dim3 g(n1, (unsigned)ceil_div(n0, 2 * c.z.plan.w));
+  TM_STORE(half, TM_LINES(c.z.plan, (gen_zpass_flc_kernel<WW, HT><<<g, c.z.threads(), c.z.smem, st>>>(
+                                    static_cast<const HT*>(Ht), Hm, Hm2, nb, n0, n1, n2, hp,
+                                    c.z.plan, tw2, scale_t, scale_m, stats, eps,
+                                    first, first_dev, state_max, state_rot, hl, z_pitch(n2)))));
+  return check_launch("gen_zpass_flc_kernel");
+}
+
+}  // namespace tmb

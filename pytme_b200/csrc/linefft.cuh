@@ -1,0 +1,352 @@
+// Line FFTs of any length 2^a 3^b 5^c 7^d 11^e 13^f up to 4096 for the fused scan passes.
+//
+// A CTA transforms W interleaved lines of length N held in one shared-memory tile. N is
+// split into two to five radices of at most 16 (host: make_plan); a thread computes whole
+// radix-R butterflies in registers, so a transform of up to 256 points exchanges its data
+// through shared memory once, one of up to 4096 points twice (more often where no three
+// radices fit). The radix of a stage is a run-time value that selects a compile-time
+// butterfly: one kernel serves every length, and the branch is uniform over the CTA.
+//
+// Decimation in frequency, in place: stage s works on sub-problems of length L (N, then
+// N / R_0, ...), butterfly b = p * LR + q (LR = L / R, q < LR) reads positions
+// p * L + q + LR * r, takes the R-point DFT, multiplies output j by w_L^(j q) and writes
+// it back to position p * L + q + LR * j. The last stage leaves frequency
+// j_0 + R_0 j_1 + R_0 R_1 j_2 + ... at position ((j_0 R_1 + j_1) R_2 + j_2) ..., i.e. the
+// butterfly b of the last stage holds the frequencies out_base(b) + r * (N / R_last). The
+// adjoint stages in reverse order go back to natural order (unnormalised inverse), so a
+// forward transform, a product and an inverse transform need no reordering, and the last
+// forward stage, the product and the first adjoint stage share their registers.
+//
+// Twiddles come from tables in shared memory (no recurrences: a value is one rounding from
+// the exact root), for each stage a row of R roots, padded to an even count, per q: a
+// butterfly reads two of its roots at a time, at constant offsets. Lanes of a warp cover W = 8
+// lines and 4 neighbouring butterflies, so a table read is a broadcast, and rows of the tile (8 complex values, 16
+// banks) are grouped by R_last with an odd group pitch, which lets the four butterflies
+// alternate between the two halves of the banks in every stage.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <algorithm>
+#include <cmath>
+#include <cstdint>
+#include <vector>
+
+#include "fft_smem.cuh"
+
+namespace tmb {
+namespace linefft {
+
+constexpr int kMaxStages = 5;
+constexpr int kMaxRadix = 16;
+constexpr int kMaxLength = 4096;
+constexpr int kMaxSlots = 48;
+
+struct Plan {
+  int n = 0, ns = 0;       // length, stages
+  int r[kMaxStages] = {};  // radices
+  int nb[kMaxStages] = {};    // butterflies of a stage
+  int lr[kMaxStages] = {};    // positions between a butterfly's values
+  int step[kMaxStages] = {};  // N / L
+  int tw4[kMaxStages] = {};   // first pair of a stage's twiddles in the table
+  int rrow[kMaxStages] = {};  // tile rows between a butterfly's values
+  int grow[kMaxStages] = {};  // (L - LR) / R_last: groups added per sub-problem p
+  uint32_t mlr[kMaxStages] = {};  // ceil(2^32 / lr)
+  uint32_t mrl = 0, mr1 = 0;  // the same of R_last and r[1]
+  int rl = 1, pitch = 1;   // R_last and the odd number of rows a group of R_last takes
+  int rows = 0;            // rows of the tile
+  int pairs = 0;           // pairs of roots in the twiddle table
+  int slots = 1;           // butterflies in flight: the CTA has slots * W threads
+  int w = 8;               // lines of the tile where they are no compile-time constant
+};
+
+// lines of a tile: W, or the plan's count for W = 0
+template <int W>
+__device__ __forceinline__ int lines(const Plan& p) {
+  return W ? W : p.w;
+}
+
+// quotient of b / d for b, d <= 4096 with m = ceil(2^32 / d), d >= 2
+__device__ __forceinline__ int fast_div(int b, uint32_t m) {
+  return (int)__umulhi((uint32_t)b, m);
+}
+
+// frequency (or output index) of value 0 of the last stage's butterfly b
+__device__ __forceinline__ int out_base(const Plan& p, int b) {
+  if (p.ns == 2) return b;
+  if (p.ns == 3) {
+    const int j0 = fast_div(b, p.mr1);
+    return j0 + p.r[0] * (b - j0 * p.r[1]);
+  }
+  int t = b, k = 0;
+  for (int s = p.ns - 2; s >= 1; --s) {
+    const int u = t / p.r[s];
+    k += (t - u * p.r[s]) * p.step[s];
+    t = u;
+  }
+  return k + t;
+}
+
+// tile row of value 0 of butterfly b of a stage before the last, and its place q in the
+// sub-problem
+__device__ __forceinline__ int stage_row(const Plan& p, int s, int b, int& q) {
+  const int o = fast_div(b, p.mrl), pp = s == 0 ? 0 : fast_div(b, p.mlr[s]);
+  q = b - pp * p.lr[s];
+  return (o + pp * p.grow[s]) * p.pitch + (b - o * p.rl);
+}
+
+// v[j] *= w_L^(j q), conjugated for the inverse direction; t points to the q-th row of the
+// stage's table
+template <int R, int DIR>
+__device__ __forceinline__ void twiddle_row(float2 (&v)[R], const float4* t) {
+#pragma unroll
+  for (int i = 0; i < (R + 1) / 2; ++i) {
+    const float4 w = t[i];
+    if (i > 0)
+      v[2 * i] = fft::cmul(v[2 * i], make_float2(w.x, DIR < 0 ? w.y : -w.y));
+    if (2 * i + 1 < R)
+      v[2 * i + 1] = fft::cmul(v[2 * i + 1], make_float2(w.z, DIR < 0 ? w.w : -w.w));
+  }
+}
+
+// First stage: ld(b) gives a functor of r for the natural-order inputs b + r * lr. With NZ,
+// inputs from nz on are zero (and not asked for); where a butterfly then has one non-zero
+// input only, its DFT is that value.
+template <int W, int R, int DIR, bool NZ, class Load>
+__device__ __forceinline__ void first_stage(const Plan& p, float2* sm, const float4* tw, int l,
+                                            int slot, int nz, Load ld) {
+  for (int b = slot; b < p.nb[0]; b += p.slots) {
+    auto in = ld(b);
+    float2 v[R];
+    if (NZ && nz <= p.lr[0]) {
+      const float2 x = b < nz ? in(0) : make_float2(0.f, 0.f);
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = x;
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        v[r] = !NZ || b + r * p.lr[0] < nz ? in(r) : make_float2(0.f, 0.f);
+      fft::dft_small<R, DIR>(v);
+    }
+    int q;
+    float2* d = sm + stage_row(p, 0, b, q) * lines<W>(p) + l;
+    const int step = p.rrow[0] * lines<W>(p);
+    twiddle_row<R, DIR>(v, tw + p.tw4[0] + q * ((R + 1) / 2));
+#pragma unroll
+    for (int j = 0; j < R; ++j) d[j * step] = v[j];
+  }
+}
+
+// A stage between the first and the last, in place.
+template <int W, int R, int DIR>
+__device__ __forceinline__ void mid_stage(const Plan& p, int s, float2* sm, const float4* tw,
+                                          int l, int slot) {
+  const int step = p.rrow[s] * lines<W>(p);
+  for (int b = slot; b < p.nb[s]; b += p.slots) {
+    int q;
+    float2* d = sm + stage_row(p, s, b, q) * lines<W>(p) + l;
+    float2 v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = d[r * step];
+    fft::dft_small<R, DIR>(v);
+    twiddle_row<R, DIR>(v, tw + p.tw4[s] + q * ((R + 1) / 2));
+#pragma unroll
+    for (int j = 0; j < R; ++j) d[j * step] = v[j];
+  }
+}
+
+// Last stage: f(b, v, d) with the R values after the DFT; d is the tile column they came
+// from (value r at d[r * lines<W>(p)]).
+template <int W, int R, int DIR, class F>
+__device__ __forceinline__ void last_stage(const Plan& p, float2* sm, int l, int slot, F f) {
+  const int nb = p.nb[p.ns - 1];
+  for (int b = slot; b < nb; b += p.slots) {
+    float2* d = sm + b * p.pitch * lines<W>(p) + l;
+    float2 v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = d[r * lines<W>(p)];
+    fft::dft_small<R, DIR>(v);
+    f(b, v, d);
+  }
+}
+
+// Adjoints (inverse direction): conjugate twiddles, then the inverse DFT.
+template <int W, int R>
+__device__ __forceinline__ void mid_adjoint(const Plan& p, int s, float2* sm, const float4* tw,
+                                            int l, int slot) {
+  const int step = p.rrow[s] * lines<W>(p);
+  for (int b = slot; b < p.nb[s]; b += p.slots) {
+    int q;
+    float2* d = sm + stage_row(p, s, b, q) * lines<W>(p) + l;
+    float2 v[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j) v[j] = d[j * step];
+    twiddle_row<R, 1>(v, tw + p.tw4[s] + q * ((R + 1) / 2));
+    fft::dft_small<R, 1>(v);
+#pragma unroll
+    for (int r = 0; r < R; ++r) d[r * step] = v[r];
+  }
+}
+
+// The first stage's adjoint: st(b) gives a functor that takes (r, value) of the natural-order
+// outputs b + r * lr.
+template <int W, int R, class Store>
+__device__ __forceinline__ void first_adjoint(const Plan& p, const float2* sm, const float4* tw,
+                                              int l, int slot, Store st) {
+  const int step = p.rrow[0] * lines<W>(p);
+  for (int b = slot; b < p.nb[0]; b += p.slots) {
+    int q;
+    const float2* d = sm + stage_row(p, 0, b, q) * lines<W>(p) + l;
+    float2 v[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j) v[j] = d[j * step];
+    twiddle_row<R, 1>(v, tw + p.tw4[0] + q * ((R + 1) / 2));
+    fft::dft_small<R, 1>(v);
+    auto out = st(b);
+#pragma unroll
+    for (int r = 0; r < R; ++r) out(r, v[r]);
+  }
+}
+
+// run-time radix -> compile-time butterfly
+#define TM_RADIX(r, CALL)                        \
+  switch (r) {                                   \
+    case 1: { constexpr int RR = 1; CALL; } break;   \
+    case 2: { constexpr int RR = 2; CALL; } break;   \
+    case 3: { constexpr int RR = 3; CALL; } break;   \
+    case 4: { constexpr int RR = 4; CALL; } break;   \
+    case 5: { constexpr int RR = 5; CALL; } break;   \
+    case 6: { constexpr int RR = 6; CALL; } break;   \
+    case 7: { constexpr int RR = 7; CALL; } break;   \
+    case 8: { constexpr int RR = 8; CALL; } break;   \
+    case 9: { constexpr int RR = 9; CALL; } break;   \
+    case 10: { constexpr int RR = 10; CALL; } break; \
+    case 11: { constexpr int RR = 11; CALL; } break; \
+    case 12: { constexpr int RR = 12; CALL; } break; \
+    case 13: { constexpr int RR = 13; CALL; } break; \
+    case 14: { constexpr int RR = 14; CALL; } break; \
+    case 15: { constexpr int RR = 15; CALL; } break; \
+    case 16: { constexpr int RR = 16; CALL; } break; \
+    default: break;                              \
+  }
+
+template <int W, int DIR>
+__device__ __forceinline__ void mid_stages(const Plan& p, float2* sm, const float4* tw, int l,
+                                           int slot) {
+  for (int s = 1; s < p.ns - 1; ++s) {
+    TM_RADIX(p.r[s], (mid_stage<W, RR, DIR>(p, s, sm, tw, l, slot)));
+    __syncthreads();
+  }
+}
+
+template <int W>
+__device__ __forceinline__ void mid_adjoints(const Plan& p, float2* sm, const float4* tw, int l,
+                                             int slot) {
+  for (int s = p.ns - 2; s >= 1; --s) {
+    TM_RADIX(p.r[s], (mid_adjoint<W, RR>(p, s, sm, tw, l, slot)));
+    __syncthreads();
+  }
+}
+
+// ------------------------------------------------------------------ host
+namespace detail {
+inline uint32_t recip(int d) { return d < 2 ? 0u : (uint32_t)((0x100000000ull + d - 1) / d); }
+
+inline void search(int n, int left, int hi, int* cur, int depth, int stages, int* best,
+                   double* best_cost) {
+  if (depth == stages - 1) {
+    if (left > hi) return;
+    cur[depth] = left;
+    // fewest operations: a radix-R butterfly costs about log2 R per value for smooth R and
+    // more for the primes; the largest radix sets the registers
+    double cost = 0;
+    for (int i = 0; i < stages; ++i) {
+      const int r = cur[i];
+      cost += r * 0.25 + (r == 7 || r == 14 ? 2.0 : r == 11 ? 4.0 : r == 13 ? 5.0 : 0.0);
+    }
+    if (cost < *best_cost) {
+      *best_cost = cost;
+      for (int i = 0; i < stages; ++i) best[i] = cur[i];
+    }
+    return;
+  }
+  for (int r = hi; r >= 1; --r)
+    if (left % r == 0 && (r > 1 || stages == 2)) {
+      cur[depth] = r;
+      search(n, left / r, r, cur, depth + 1, stages, best, best_cost);
+    }
+}
+}  // namespace detail
+
+// The plan of a length (ns = 0 where the length is not supported), but for its slots. Radices ascend, so the first stage, which reads global memory, has
+// the most butterflies and the shortest non-zero part of a zero-padded input.
+inline Plan make_plan(int n) {
+  Plan p;
+  if (n < 2 || n > kMaxLength) return p;
+  int best[kMaxStages] = {}, cur[kMaxStages] = {};
+  int ns = 0;
+  for (int s = 2; s <= kMaxStages && !ns; ++s) {
+    double cost = 1e30;
+    detail::search(n, n, kMaxRadix, cur, 0, s, best, &cost);
+    if (cost < 1e30) ns = s;
+  }
+  if (!ns) return p;
+  p.n = n;
+  p.ns = ns;
+  for (int i = 0; i < ns; ++i) p.r[i] = best[ns - 1 - i];
+  p.rl = p.r[ns - 1];
+  p.pitch = p.rl | 1;
+  p.rows = n / p.rl * p.pitch;
+  int l = n, before = 1;
+  for (int s = 0; s < ns; ++s) {
+    p.nb[s] = n / p.r[s];
+    p.lr[s] = l / p.r[s];
+    p.step[s] = before;
+    p.rrow[s] = s == ns - 1 ? 1 : p.lr[s] / p.rl * p.pitch;
+    p.grow[s] = s == ns - 1 ? 0 : (l - p.lr[s]) / p.rl;
+    p.mlr[s] = detail::recip(p.lr[s]);
+    p.tw4[s] = p.pairs;
+    if (s < ns - 1) p.pairs += p.lr[s] * ((p.r[s] + 1) / 2);
+    before *= p.r[s];
+    l = p.lr[s];
+  }
+  p.mrl = detail::recip(p.rl);
+  p.mr1 = detail::recip(p.r[1]);
+  return p;
+}
+
+// Butterfly slots of a CTA: a multiple of 4 (whole warps at eight lines) with few idle lanes
+// over the stages and with enough warps on an SM, given the CTA's shared memory and the
+// registers of a thread. Several small CTAs hide each other's barriers and memory waits.
+inline void choose_slots(Plan& p, size_t smem, int regs) {
+  double most = 0;
+  for (int s = 4; s <= kMaxSlots; s += 4) {
+    double spent = 0, work = 0;
+    for (int i = 0; i < p.ns; ++i) {
+      spent += (double)((p.nb[i] + s - 1) / s) * s * (p.r[i] + 2);
+      work += (double)p.nb[i] * (p.r[i] + 2);
+    }
+    const int threads = s * p.w;
+    const int ctas = (int)std::min<size_t>(
+        std::min<size_t>(32, 227 * 1024 / (smem + 1024)), 65536 / (regs * threads));
+    const double warps = ctas * threads / 32.0;
+    const double rate = work / spent * std::min(1.0, (warps + 4) / 24);
+    if (rate > most * 1.01) { most = rate; p.slots = s; }
+  }
+}
+
+// The twiddle table of a plan: p.pairs pairs of roots.
+inline std::vector<float2> twiddle_rows(const Plan& p) {
+  std::vector<float2> t(2 * (size_t)p.pairs, make_float2(1.f, 0.f));
+  for (int s = 0; s < p.ns - 1; ++s)
+    for (int q = 0; q < p.lr[s]; ++q)
+      for (int j = 0; j < p.r[s]; ++j) {
+        const int64_t e = (int64_t)j * q * p.step[s] % p.n;
+        const double a = -2.0 * 3.14159265358979323846 * (double)e / p.n;
+        t[2 * (p.tw4[s] + (size_t)q * ((p.r[s] + 1) / 2)) + j] =
+            make_float2((float)std::cos(a), (float)std::sin(a));
+      }
+  return t;
+}
+
+}  // namespace linefft
+}  // namespace tmb

@@ -30,6 +30,7 @@
 #include "colfft.cuh"
 #include "common.cuh"
 #include "fft_smem.cuh"
+#include "genpass.cuh"
 #include "ops.cuh"
 #include "scan.cuh"
 #include "tc_common.cuh"
@@ -121,134 +122,6 @@ __device__ __forceinline__ void cp_async_wait() {
 constexpr int kThreads = 512;
 constexpr int kMaxE = 8;             // complex elements per thread in a line-FFT tile
 constexpr int kTile = kThreads * kMaxE;  // elements per tile (4096)
-
-// ------------------------------------------------------------------ K1: template z/y
-// grid (ceil(h2/W), t0, B); tile: n1 lines-fast rows x W lines (k2).
-__global__ void __launch_bounds__(kThreads, 1)
-tmpl_zy_kernel(const float* __restrict__ tmpl, int t0, int t1, int t2, int n1, int n2, int h2,
-               int W, LinePlan p1, const float2* __restrict__ tw1_g, const float2* __restrict__ tw2_g,
-               float2* __restrict__ G) {
-  extern __shared__ float4 smem_raw[];
-  float2* tw1 = reinterpret_cast<float2*>(smem_raw);
-  float2* tw2 = tw1 + n1;
-  float2* buf = tw2 + n2;
-  float* plane = reinterpret_cast<float*>(buf + (int64_t)n1 * W);
-  const int tid = threadIdx.x;
-  const int k2_0 = blockIdx.x * W;
-  const int x = blockIdx.y;
-  const int b = blockIdx.z;
-  for (int i = tid; i < n1; i += kThreads) tw1[i] = tw1_g[i];
-  for (int i = tid; i < n2; i += kThreads) tw2[i] = tw2_g[i];
-  const float* src = tmpl + ((int64_t)b * t0 + x) * t1 * t2;
-  for (int i = tid; i < t1 * t2; i += kThreads) plane[i] = src[i];
-  __syncthreads();
-  // G1[y][k2] = sum_z plane[y][z] * exp(-2 pi i z k2 / n2), rows y >= t1 are zero
-  for (int e = tid; e < n1 * W; e += kThreads) {
-    int y = e / W, l = e % W;
-    int k2 = k2_0 + l;
-    float2 acc = make_float2(0.f, 0.f);
-    if (y < t1 && k2 < h2) {
-      const float* row = plane + y * t2;
-      int idx = 0;
-      for (int z = 0; z < t2; ++z) {
-        float v = row[z];
-        float2 w = tw2[idx];
-        acc.x += v * w.x;
-        acc.y += v * w.y;
-        idx += k2;
-        if (idx >= n2) idx -= n2;
-      }
-    }
-    buf[e] = acc;
-  }
-  __syncthreads();
-  fft::fft_lines<-1, kMaxE, true>(buf, p1, W, 1, W, tw1, n1, tid, kThreads);
-  float2* dst = G + ((int64_t)b * t0 + x) * n1 * h2;
-  for (int e = tid; e < n1 * W; e += kThreads) {
-    int k1 = e / W, l = e % W;
-    int k2 = k2_0 + l;
-    if (k2 < h2) dst[(int64_t)k1 * h2 + k2] = buf[e];
-  }
-}
-
-// ------------------------------------------------------------------ K2: x pass
-// grid (ceil(h2/W), n1); loops over the B rotations of the group.
-template <typename HT>
-__global__ void __launch_bounds__(kThreads, 1)
-xpass_kernel(const float2* __restrict__ G, const float2* __restrict__ Ft, int B, int t0, int n0,
-             int n1, int h2, int W, LinePlan p0, const float2* __restrict__ tw0_g, float scale,
-             HT* __restrict__ H, int hp) {
-  extern __shared__ float4 smem_raw[];
-  float2* tw0 = reinterpret_cast<float2*>(smem_raw);
-  float2* buf = tw0 + n0;
-  const int tid = threadIdx.x;
-  const int k2_0 = blockIdx.x * W;
-  const int k1 = blockIdx.y;
-  for (int i = tid; i < n0; i += kThreads) tw0[i] = tw0_g[i];
-  const int tile = n0 * W;
-  // target-spectrum tile: re-read through L1 for every rotation of the group
-  const float2* ft_col = Ft + (int64_t)k1 * h2 + k2_0;
-  const int64_t ft_row = (int64_t)n1 * h2;
-  const int64_t S = (int64_t)n0 * n1 * h2;
-  const int64_t SH = (int64_t)n0 * n1 * hp;
-  for (int b = 0; b < B; ++b) {
-    const float2* g = G + (int64_t)b * t0 * n1 * h2;
-    for (int e = tid; e < tile; e += kThreads) {
-      int x = e / W, l = e % W;
-      int k2 = k2_0 + l;
-      float2 v = make_float2(0.f, 0.f);
-      if (x < t0 && k2 < h2) v = g[((int64_t)x * n1 + k1) * h2 + k2];
-      buf[e] = v;
-    }
-    __syncthreads();
-    fft::fft_lines<-1, kMaxE, true>(buf, p0, W, 1, W, tw0, n0, tid, kThreads);
-    for (int e = tid; e < tile; e += kThreads) {
-      int k0 = e / W, l = e % W;
-      float2 f = make_float2(0.f, 0.f);
-      if (k2_0 + l < h2) f = __ldg(ft_col + k0 * ft_row + l);
-      buf[e] = fft::cmul(buf[e], make_float2(f.x * scale, f.y * scale));
-    }
-    __syncthreads();
-    fft::fft_lines<1, kMaxE, true>(buf, p0, W, 1, W, tw0, n0, tid, kThreads);
-    HT* h = H + (int64_t)b * SH;
-    for (int e = tid; e < tile; e += kThreads) {
-      int x = e / W, l = e % W;
-      int k2 = k2_0 + l;
-      if (k2 < h2) Store<HT>::store(h + ((int64_t)x * n1 + k1) * hp + k2, buf[e]);
-    }
-    __syncthreads();
-  }
-}
-
-// ------------------------------------------------------------------ K3: y pass
-// grid (ceil(h2/W), n0, B): inverse FFT along axis 1, in place.
-template <typename HT>
-__global__ void __launch_bounds__(kThreads, 1)
-ypass_kernel(HT* __restrict__ H, int n0, int n1, int h2, int W, LinePlan p1,
-             const float2* __restrict__ tw1_g, int hp) {
-  extern __shared__ float4 smem_raw[];
-  float2* tw1 = reinterpret_cast<float2*>(smem_raw);
-  float2* buf = tw1 + n1;
-  const int tid = threadIdx.x;
-  const int k2_0 = blockIdx.x * W;
-  const int x = blockIdx.y;
-  const int b = blockIdx.z;
-  for (int i = tid; i < n1; i += kThreads) tw1[i] = tw1_g[i];
-  const int tile = n1 * W;
-  HT* h = H + (int64_t)b * n0 * n1 * hp + (int64_t)x * n1 * hp;
-  for (int e = tid; e < tile; e += kThreads) {
-    int y = e / W, l = e % W;
-    int k2 = k2_0 + l;
-    buf[e] = (k2 < h2) ? Store<HT>::load(h + (int64_t)y * hp + k2) : make_float2(0.f, 0.f);
-  }
-  __syncthreads();
-  fft::fft_lines<1, kMaxE, true>(buf, p1, W, 1, W, tw1, n1, tid, kThreads);
-  for (int e = tid; e < tile; e += kThreads) {
-    int y = e / W, l = e % W;
-    int k2 = k2_0 + l;
-    if (k2 < h2) Store<HT>::store(h + (int64_t)y * hp + k2, buf[e]);
-  }
-}
 
 // ------------------------------------------------------------------ register-resident passes
 // Power-of-two axis lengths use the column codelet of colfft.cuh: T = N/8 threads
@@ -621,103 +494,9 @@ static bool reg_supported(int n) {
 // with the imaginary parts of X[0] and X[m] dropped, as numpy/pocketfft's c2r does.
 constexpr int kMaxV = 8;   // output voxels per thread
 
-template <typename HT, int M = 0>
-__global__ void __launch_bounds__(kThreads, 1)
-zpass_kernel(const HT* __restrict__ H, int B, int64_t rows, int n2, int hp, int R, LinePlan pm,
-             const float2* __restrict__ tw2_g, float scale, const float* __restrict__ inv_den,
-             int32_t first_index, float* __restrict__ state_max, int32_t* __restrict__ state_rot,
-             int64_t S, const int32_t* __restrict__ first_dev) {
-  if (first_dev) first_index = *first_dev;
-  extern __shared__ float4 smem_raw[];
-  const int m = n2 / 2;
-  float2* tw2 = reinterpret_cast<float2*>(smem_raw);
-  float2* raw = tw2 + n2;
-  float2* buf = raw + (int64_t)R * hp;
-  const int tid = threadIdx.x;
-  const int64_t row0 = (int64_t)blockIdx.x * R;
-  const int nrows = (int)min((int64_t)R, rows - row0);
-  for (int i = tid; i < n2; i += kThreads) tw2[i] = tw2_g[i];
-  const int nout = nrows * n2;
-  const int64_t vox0 = row0 * n2;
-  float den[kMaxV], best[kMaxV];
-  int32_t arg[kMaxV];
-#pragma unroll
-  for (int c = 0; c < kMaxV; ++c) {
-    int v = tid + c * kThreads;
-    den[c] = (v < nout) ? (inv_den ? inv_den[vox0 + v] : 1.f) * scale : 0.f;
-    best[c] = -INFINITY;
-    arg[c] = -1;
-  }
-  for (int b = 0; b < B; ++b) {
-    const HT* src = H + (int64_t)b * S + row0 * hp;
-    for (int e = tid; e < nrows * hp; e += kThreads) raw[e] = Store<HT>::load(src + e);
-    __syncthreads();
-    for (int e = tid; e < nrows * m; e += kThreads) {
-      int r = e / m, k = e % m;
-      const float2* xr = raw + (int64_t)r * hp;
-      float2 a = xr[k], c = xr[m - k];
-      if (k == 0) { a.y = 0.f; c.y = 0.f; }
-      float2 cc = fft::cconj(c);
-      float2 E = fft::cadd(a, cc);
-      float2 O = fft::cmul(fft::csub(a, cc), fft::cconj(tw2[k]));
-      buf[e] = make_float2(E.x - O.y, E.y + O.x);
-    }
-    __syncthreads();
-    if constexpr (M > 0)
-      fft::fft_lines_ct<M, 1, kMaxE, false>(buf, nrows, M, 1, tw2, 2 * M, tid, kThreads);
-    else
-      fft::fft_lines<1, kMaxE, false>(buf, pm, nrows, m, 1, tw2, n2, tid, kThreads);
-    const float* outv = reinterpret_cast<const float*>(buf);
-#pragma unroll
-    for (int c = 0; c < kMaxV; ++c) {
-      int v = tid + c * kThreads;
-      if (v < nout) {
-        float s = outv[v] * den[c];
-        if (s > best[c]) {
-          best[c] = s;
-          arg[c] = first_index + b;
-        }
-      }
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int c = 0; c < kMaxV; ++c) {
-    int v = tid + c * kThreads;
-    if (v < nout && arg[c] >= 0) {
-      int64_t g = vox0 + v;
-      if (best[c] > state_max[g]) {
-        state_max[g] = best[c];
-        state_rot[g] = arg[c];
-      }
-    }
-  }
-}
-
 // K4'' (FLC): c2r of the numerator and both statistics rows, then
 // norm_scores (tme/backends/npfftw_backend.py:537-587) in double precision with the
 // rotation's own n_obs = sum(rotated mask), and the strict-> update.
-template <int M, typename RT = float2>
-__device__ __forceinline__ void c2r_rows(const RT* raw, float2* buf, const float2* tw2, int nrows,
-                                         int n2, int hp, const LinePlan& pm, int tid) {
-  const int m = n2 / 2;
-  for (int e = tid; e < nrows * m; e += kThreads) {
-    int r = e / m, k = e % m;
-    const RT* xr = raw + (int64_t)r * hp;
-    float2 a = Store<RT>::load(xr + k), c = Store<RT>::load(xr + (m - k));
-    if (k == 0) { a.y = 0.f; c.y = 0.f; }
-    float2 cc = fft::cconj(c);
-    float2 E = fft::cadd(a, cc);
-    float2 O = fft::cmul(fft::csub(a, cc), fft::cconj(tw2[k]));
-    buf[e] = make_float2(E.x - O.y, E.y + O.x);
-  }
-  __syncthreads();
-  if constexpr (M > 0)
-    fft::fft_lines_ct<M, 1, kMaxE, false>(buf, nrows, M, 1, tw2, 2 * M, tid, kThreads);
-  else
-    fft::fft_lines<1, kMaxE, false>(buf, pm, nrows, m, 1, tw2, n2, tid, kThreads);
-}
-
 // The FLC z pass transforms, for every rotation, the local mean (Hm), the local mean
 // square (Hm2) and the numerator (H) of a block of R rows as one batch of 3 R lines (one
 // set of barriers per rotation). The next rotation's rows are copied (cp.async, 16-byte
@@ -1124,12 +903,13 @@ struct Scan {
   float2* tw0 = nullptr;
   float2* tw1 = nullptr;
   float2* tw2 = nullptr;
-  LinePlan p0{}, p1{}, pm{};
+  LinePlan pm{};
   bool reg0 = false, reg1 = false;  // register-resident column kernels for n0 / n1
-  int W1 = 1, W2 = 1, W3 = 1, R4 = 1;
+  bool z4 = false;                  // four-step z pass for n2 / 2
+  GenConfig gen{};                  // passes over axes of any other length
+  float4* gtw[3] = {};              // their twiddle tables
   int R4f = 1;  // rows per block of the FLC z pass (three parts per row)
   size_t smem4f = 0;
-  size_t smem1 = 0, smem2 = 0, smem3 = 0, smem4 = 0;
   cufftHandle fwd = 0, inv = 0, tfwd = 0, tinv = 0;
   bool have_fwd = false, have_tfwd = false;
   // CUDA-graph replay of a full launch group (see scan_set_graph)
@@ -1176,6 +956,25 @@ static bool x_inner(const Scan* s) {
   return s->H2 && s->ytc && !s->yinplace && !y_stage1_tc(s) && x_writes_stage1(s);
 }
 
+// Which passes run over axes of any length (genpass.cuh): those without tensor cores whose
+// length has no kernel of its own. FLC takes the power-of-two kernels for both x and y or
+// for neither.
+static bool flc_reg(const Scan* s) { return s->reg0 && s->reg1; }
+static bool gen_x(const Scan* s) {
+  return s->d.score == TM_SCORE_FLC ? !flc_reg(s) : !s->xtc && !s->reg0;
+}
+static bool gen_y(const Scan* s) {
+  return s->d.score == TM_SCORE_FLC ? !flc_reg(s) : !s->ytc && !s->reg1;
+}
+static bool gen_z(const Scan* s) {
+  return s->d.score == TM_SCORE_FLC ? !flc_reg(s) : !(s->ztc && s->half) && !s->z4;
+}
+// H is k1-outer where all three run so, row-major otherwise.
+static HLayout h_layout(const Scan* s) {
+  return gen_x(s) && gen_y(s) && gen_z(s) ? h_k1_outer(s->n0, s->n1, s->hp)
+                                          : h_row_major(s->n0, s->n1, s->hp);
+}
+
 // Stage timing: record an event before a stage and accumulate after it.
 struct StageTimer {
   Scan* s;
@@ -1211,6 +1010,12 @@ static void launch_zpass_flc(Scan* s, HT* H, int nb, int64_t rows, float out_sca
                              int32_t first, float* state_max, int32_t* state_rot,
                              cudaStream_t st) {
   const double* stats = s->stats_ws + (int64_t)nb * kStatChunks * 3;
+  if (gen_z(s)) {
+    gen_zpass_flc(s->gen, H, std::is_same<HT, __half2>::value, s->Hm, s->Hm2, nb, s->n0, s->n1,
+                  s->n2, s->hp, s->gtw[2], out_scale, out_scale, stats, 1.1920928955078125e-07,
+                  first, s->graph_first, state_max, state_rot, h_layout(s), st);
+    return;
+  }
   dim3 g4f(ceil_div(rows, s->R4f));
   TM_DISPATCH_M(s->n2 / 2, (zpass_flc_kernel<HT, MM><<<g4f, kThreads, s->smem4f, st>>>(
                                H, s->Hm, s->Hm2, nb, rows, s->n2, s->hp, s->R4f, s->pm, s->tw2,
@@ -1218,24 +1023,17 @@ static void launch_zpass_flc(Scan* s, HT* H, int nb, int64_t rows, float out_sca
                                state_max, state_rot, s->SH, s->graph_first)));
 }
 
-static void set_zpass_attrs(int m, int smem) {
-  (void)smem;
+static void set_zpass_attrs(int m) {
   TM_DISPATCH_M(m, (cudaFuncSetAttribute(zpass_flc_kernel<float2, MM>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max()),
                     cudaFuncSetAttribute(zpass_flc_kernel<__half2, MM>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max())));
-  TM_DISPATCH_M(m, (cudaFuncSetAttribute(zpass_kernel<float2, MM>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max()),
-                    cudaFuncSetAttribute(zpass_kernel<__half2, MM>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max())));
 }
 
 #define TM_DISPATCH_4STEP(m, CALL)                                  \
   switch (m) {                                                      \
     case 32: { constexpr int A1 = 4, A2 = 8; CALL; } break;         \
-    case 50: { constexpr int A1 = 5, A2 = 10; CALL; } break;        \
     case 64: { constexpr int A1 = 8, A2 = 8; CALL; } break;         \
-    case 80: { constexpr int A1 = 4, A2 = 20; CALL; } break;        \
     case 100: { constexpr int A1 = 10, A2 = 10; CALL; } break;      \
     case 128: { constexpr int A1 = 8, A2 = 16; CALL; } break;       \
     case 200: { constexpr int A1 = 10, A2 = 20; CALL; } break;      \
@@ -1243,9 +1041,12 @@ static void set_zpass_attrs(int m, int smem) {
     default: break;                                                 \
   }
 
+// Half-lengths whose four-step kernel beats the z pass over any length (us for 32 rotations of
+// 160 x 160 x n2, four-step / any length: n2 = 128 209 / 280, 200 383 / 567, 256 538 / 624,
+// 400 1241 / 1341, 512 900 / 1787; for 8 rotations of 64 x 64 x 64 24 / 30. It does not at
+// n2 = 100 and 160: 238 / 211, 429 / 312).
 static bool zpass4_supported(int m) {
-  return m == 32 || m == 50 || m == 64 || m == 80 || m == 100 || m == 128 || m == 200 ||
-         m == 256;
+  return m == 32 || m == 64 || m == 100 || m == 128 || m == 200 || m == 256;
 }
 
 template <typename HT>
@@ -1268,7 +1069,7 @@ static void set_zpass4_attrs(int m) {
 }
 
 template <typename HT>
-static void launch_zpass(Scan* s, dim3 g4, HT* H, int nb, int64_t rows, float out_scale,
+static void launch_zpass(Scan* s, HT* H, int nb, int64_t rows, float out_scale,
                          int32_t first, float* state_max, int32_t* state_rot, cudaStream_t st) {
   if (s->ztc && std::is_same<HT, __half2>::value) {
     zpass_tc_run(s->zcfg, H, nb, rows, s->n2, s->h2, s->hp, s->ztable, out_scale, s->inv_den,
@@ -1276,13 +1077,13 @@ static void launch_zpass(Scan* s, dim3 g4, HT* H, int nb, int64_t rows, float ou
                  s->wait_iters, seg_layout(s));
     return;
   }
-  if (zpass4_supported(s->n2 / 2) && !getenv("PYTME_B200_GENERIC_FFT")) {
+  if (s->z4) {
     launch_zpass4<HT>(s, H, nb, rows, out_scale, first, state_max, state_rot, st);
     return;
   }
-  TM_DISPATCH_M(s->n2 / 2, (zpass_kernel<HT, MM><<<g4, kThreads, s->smem4, st>>>(
-                               H, nb, rows, s->n2, s->hp, s->R4, s->pm, s->tw2, out_scale,
-                               s->inv_den, first, state_max, state_rot, s->SH, s->graph_first)));
+  gen_zpass(s->gen, H, std::is_same<HT, __half2>::value, nb, s->n0, s->n1, s->n2, s->hp,
+            s->gtw[2], out_scale, s->inv_den, first, s->graph_first, state_max, state_rot,
+            h_layout(s), st);
 }
 
 // ---- launch helpers for the register-resident kernels
@@ -1370,32 +1171,36 @@ static int launch_template_x_y(Scan* s, int nb, float hs, HT* H, StageTimer& tmr
   // rounds them to FP16 for its MMAs anyway), so the template pass writes them so
   const bool half_g = s->reg1 && x_writes_stage1(s);
   tmr.begin();
-  if (s->reg1) {
+  const HLayout hl = h_layout(s);
+  const bool half = std::is_same<HT, __half2>::value;
+  if (gen_y(s) && !half_g) {
+    TM_TRY(gen_template(s->gen, s->rot_t, nb, s->t0, s->t1, s->t2, s->n1, s->n2, s->h2, s->hp,
+                        s->gtw[1], s->tw2, s->G, stream));
+    if (flc)
+      TM_TRY(gen_template(s->gen, s->rot_m, nb, s->t0, s->t1, s->t2, s->n1, s->n2, s->h2, s->hp,
+                          s->gtw[1], s->tw2, s->Gm, stream));
+  } else {
     TM_DISPATCH_N(s->n1, (launch_tmpl_reg<NN>(s, nb, stream, nullptr, nullptr, half_g)));
     if (flc) TM_DISPATCH_N(s->n1, (launch_tmpl_reg<NN>(s, nb, stream, s->rot_m, s->Gm)));
-  } else {
-    dim3 g1(ceil_div(s->h2, s->W1), s->t0, nb);
-    tmpl_zy_kernel<<<g1, kThreads, s->smem1, stream>>>(s->rot_t, s->t0, s->t1, s->t2, s->n1,
-                                                       s->n2, s->h2, s->W1, s->p1, s->tw1,
-                                                       s->tw2, s->G);
   }
   TM_TRY(check_launch("template pass"));
   tmr.end(TM_STAGE_TEMPLATE);
   tmr.begin();
-  if (flc) {
+  if (flc && gen_x(s)) {
+    TM_TRY(gen_xpass_flc(s->gen, s->G, s->Gm, s->ft_target, s->ft_target2, nb, s->t0, s->n1,
+                         s->h2, s->hp, s->gtw[0], hs, H, half, s->Hm, s->Hm2, hl, stream));
+  } else if (flc) {
     TM_DISPATCH_N(s->n0, (launch_xpass_flc_reg<NN, HT>(s, nb, hs, H, stream)));
+  } else if (gen_x(s)) {
+    TM_TRY(gen_xpass(s->gen, s->G, s->ft_target, nb, s->t0, s->n1, s->h2, s->hp, s->gtw[0], hs, H,
+                     half, hl, stream));
   } else if (s->xtc) {
     const bool s1 = y_stage1_tc(s);
     TM_TRY(xcorr_tc_run(s->xcfg, s->G, s->ctarget, nb, s->t0, s->n0, s->n1, s->h2, s->hp, hs,
                         H, std::is_same<HT, __half2>::value, s->tc_err, stream,
                         s->wait_iters, s1, s1 ? s->n1 / 16 : 0, half_g, x_inner(s)));
-  } else if (s->reg0) {
-    TM_DISPATCH_N(s->n0, (launch_xpass_reg<NN, HT>(s, nb, hs, H, stream)));
   } else {
-    dim3 g2(ceil_div(s->h2, s->W2), s->n1);
-    xpass_kernel<HT><<<g2, kThreads, s->smem2, stream>>>(s->G, s->ft_target, nb, s->t0, s->n0,
-                                                        s->n1, s->h2, s->W2, s->p0, s->tw0, hs, H,
-                                                        s->hp);
+    TM_DISPATCH_N(s->n0, (launch_xpass_reg<NN, HT>(s, nb, hs, H, stream)));
   }
   TM_TRY(check_launch("x pass"));
   tmr.end(TM_STAGE_XPASS);
@@ -1404,16 +1209,18 @@ static int launch_template_x_y(Scan* s, int nb, float hs, HT* H, StageTimer& tmr
     TM_TRY(ypass_tc_run(s->ycfg, H, nb, s->n0, s->hp, s->h2, s->ytable, s->wait_iters, s->tc_err,
                         stream, seg_layout(s), y_stage1_tc(s), x_inner(s) ? s->H2 : nullptr,
                         x_inner(s)));
-  } else if (s->reg1) {
+  } else if (gen_y(s)) {
+    TM_TRY(gen_ypass(s->gen, H, half, nb, s->n0, s->hp, s->gtw[1], hl, stream));
+    if (flc) {
+      TM_TRY(gen_ypass(s->gen, s->Hm, false, nb, s->n0, s->hp, s->gtw[1], hl, stream));
+      TM_TRY(gen_ypass(s->gen, s->Hm2, false, nb, s->n0, s->hp, s->gtw[1], hl, stream));
+    }
+  } else {
     TM_DISPATCH_N(s->n1, (launch_ypass_reg<NN, HT>(s, nb, H, stream, seg_layout(s))));
     if (flc) {
       TM_DISPATCH_N(s->n1, (launch_ypass_reg<NN, float2>(s, nb, s->Hm, stream)));
       TM_DISPATCH_N(s->n1, (launch_ypass_reg<NN, float2>(s, nb, s->Hm2, stream)));
     }
-  } else {
-    dim3 g3(ceil_div(s->h2, s->W3), s->n0, nb);
-    ypass_kernel<HT><<<g3, kThreads, s->smem3, stream>>>(H, s->n0, s->n1, s->h2, s->W3, s->p1,
-                                                        s->tw1, s->hp);
   }
   TM_TRY(check_launch("y pass"));
   tmr.end(TM_STAGE_YPASS);
@@ -1443,7 +1250,7 @@ int scan_destroy(Scan* s) {
   return TM_OK;
 }
 
-int scan_create(const tm_scan_desc* desc, Scan** out) {
+int scan_create(const tm_scan_desc* desc, Scan** out, bool any_length) {
   TM_REQUIRE(desc && out, "scan_create: null pointer");
   *out = nullptr;
   const tm_scan_desc& d = *desc;
@@ -1474,8 +1281,29 @@ int scan_create(const tm_scan_desc* desc, Scan** out) {
   s->fused = !d.plain;
   s->half = d.precision == TM_PREC_MIXED;
   s->B = s->fused ? d.batch : 1;
-  if (s->fused) {
-    bool ok = line_supported(s->n0) && line_supported(s->n1) && (s->n2 % 2 == 0) &&
+  if (s->fused && any_length) {
+    s->gen = gen_config(s->n0, s->n1, s->n2, s->t0, s->t1, s->t2, s->hp,
+                        d.score == TM_SCORE_FLC, s->half);
+    if (!s->gen.ok || s->half) {
+      set_error("scan_create: the FP32 fused path does not support shape (%d,%d,%d)", s->n0, s->n1,
+                s->n2);
+      delete s;
+      return TM_E_UNSUPPORTED;
+    }
+    // the launch group shrinks to what a plan may hold: 8 GiB of group buffers, and the
+    // limit of tm_set_device_memory_limit
+    const int64_t spectra = d.score == TM_SCORE_FLC ? 3 : 1, rows = d.score == TM_SCORE_FLC ? 2 : 1;
+    const int64_t per = spectra * s->SH * 8 + rows * s->t0 * s->n1 * (int64_t)s->h2 * 8 +
+                        8 * s->T + 8 * s->TS + (1 << 14);
+    int64_t room = 8LL << 30;
+    if (device_memory_limit() > 0)
+      room = std::min(room, device_memory_limit() - 8 * s->S * (spectra == 3 ? 2 : 1) - 4 * s->N -
+                                16 * s->T - 8 * s->TS - (1 << 20));
+    s->B = (int)std::max<int64_t>(1, std::min<int64_t>(s->B, room / per));
+  } else if (s->fused) {
+    s->gen = gen_config(s->n0, s->n1, s->n2, s->t0, s->t1, s->t2, s->hp,
+                        d.score == TM_SCORE_FLC, s->half);
+    bool ok = s->gen.ok && line_supported(s->n0) && line_supported(s->n1) && (s->n2 % 2 == 0) &&
               line_supported(s->n2 / 2) && s->n0 <= kTile && s->n1 <= kTile &&
               s->n2 <= kThreads * kMaxV &&
               (d.score != TM_SCORE_FLC || (reg_supported(s->n0) && reg_supported(s->n1)));
@@ -1506,7 +1334,7 @@ int scan_create(const tm_scan_desc* desc, Scan** out) {
   size_t o_st = take(stats_workspace_bytes(B));
   size_t o_ts = take(sizeof(float2) * s->TS * B);
   size_t o_arr = 0, o_arrm = 0, o_ccm = 0, o_ccm2 = 0, o_spec = 0, o_specm = 0, o_G = 0, o_H = 0;
-  size_t o_tw0 = 0, o_tw1 = 0, o_tw2 = 0, o_Gm = 0, o_Hm = 0, o_Hm2 = 0;
+  size_t o_gtw[3] = {}, o_tw0 = 0, o_tw1 = 0, o_tw2 = 0, o_Gm = 0, o_Hm = 0, o_Hm2 = 0;
   if (!s->fused) {
     o_arr = take(sizeof(float) * s->N);
     o_spec = take(sizeof(float2) * s->S);
@@ -1527,6 +1355,11 @@ int scan_create(const tm_scan_desc* desc, Scan** out) {
     o_tw0 = take(sizeof(float2) * s->n0);
     o_tw1 = take(sizeof(float2) * s->n1);
     o_tw2 = take(sizeof(float2) * s->n2);
+    {
+      o_gtw[0] = take(sizeof(float4) * s->gen.x.plan.pairs);
+      o_gtw[1] = take(sizeof(float4) * s->gen.y.plan.pairs);
+      o_gtw[2] = take(sizeof(float4) * s->gen.z.plan.pairs);
+    }
   }
   size_t o_ct = 0, o_err = 0, o_zt = 0, o_yt = 0;
   if (s->fused && d.score != TM_SCORE_FLC && s->half) {
@@ -1539,7 +1372,7 @@ int scan_create(const tm_scan_desc* desc, Scan** out) {
     s->ytc = s->ytc_avail;
     if (s->ytc_avail) o_yt = take(ypass_tc_table_bytes(s->ycfg));
   }
-  if (s->fused && d.score != TM_SCORE_FLC) {
+  if (s->fused && d.score != TM_SCORE_FLC && !any_length) {
     TM_TRY(xcorr_tc_config(s->n0, s->t0, B, &s->xcfg));
     s->xtc_avail = s->xcfg.ok || (s->half && s->xcfg.ws);
     // default: tensor cores for half-precision spectra (the FP16 Hankel kernels), FFTs
@@ -1623,40 +1456,27 @@ int scan_create(const tm_scan_desc* desc, Scan** out) {
     cudaMemcpy(s->tw1, t1v.data(), sizeof(float2) * s->n1, cudaMemcpyHostToDevice);
     e = cudaMemcpy(s->tw2, t2v.data(), sizeof(float2) * s->n2, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) { int st = cuda_status(e, "scan_create: twiddles"); destroy(s); return st; }
-    s->p0 = make_line_plan(s->n0);
-    s->p1 = make_line_plan(s->n1);
     s->pm = make_line_plan(s->n2 / 2);
-    s->W1 = std::max(1, std::min(s->h2, kTile / s->n1));
-    s->W2 = std::max(1, std::min(s->h2, kTile / s->n0));
-    s->W3 = s->W1;
-    s->R4 = std::max(1, std::min(kTile / std::max(1, s->n2 / 2), (kThreads * kMaxV) / s->n2));
     s->R4f = std::max(1, std::min(kTile / std::max(1, 3 * (s->n2 / 2)),
                                   (kThreads * kMaxV) / s->n2));
-    s->smem1 = sizeof(float2) * (s->n1 + s->n2 + (size_t)s->n1 * s->W1) + sizeof(float) * s->t1 * s->t2;
-    s->smem2 = sizeof(float2) * (s->n0 + (size_t)s->n0 * s->W2);
-    s->smem3 = sizeof(float2) * (s->n1 + (size_t)s->n1 * s->W3);
-    // twiddles (padded to 16 bytes), two raw row buffers, the c2r buffer
-    s->smem4 = sizeof(float2) * ((s->n2 + 1) / 2 * 2 + 2 * (size_t)s->R4 * s->hp +
-                                 (size_t)s->R4 * (s->n2 / 2));
+    // what the template pass may hold of a template plane
+    const size_t plane = sizeof(float2) * (s->n1 + s->n2 +
+                                           (size_t)s->n1 * std::max(1, std::min(s->h2, kTile / s->n1))) +
+                         sizeof(float) * s->t1 * s->t2;
     // FLC z pass: twiddles, two raw sets of three parts, the c2r buffer of 3 R4f lines
     s->smem4f = sizeof(float2) * ((s->n2 + 1) / 2 * 2 + 6 * (size_t)s->R4f * s->hp +
                                   3 * (size_t)s->R4f * (s->n2 / 2));
-    size_t mx = std::max(std::max(s->smem1, s->smem2), std::max(s->smem3, s->smem4));
-    if (d.score == TM_SCORE_FLC) mx = std::max(mx, s->smem4f);
-    if (mx > 200 * 1024) {
+    const size_t mx = std::max(plane, d.score == TM_SCORE_FLC ? s->smem4f : 0);
+    if (mx > 200 * 1024 && !any_length) {
       set_error("scan_create: shared-memory tile of %zu bytes exceeds the limit", mx);
       destroy(s);
       return TM_E_UNSUPPORTED;
     }
-    cudaFuncSetAttribute(tmpl_zy_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max());
-    cudaFuncSetAttribute(xpass_kernel<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max());
-    cudaFuncSetAttribute(xpass_kernel<__half2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max());
-    cudaFuncSetAttribute(ypass_kernel<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max());
-    cudaFuncSetAttribute(ypass_kernel<__half2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max());
-    set_zpass_attrs(s->n2 / 2, (int)s->smem4);
+    set_zpass_attrs(s->n2 / 2);
     set_zpass4_attrs(s->n2 / 2);
-    s->reg0 = reg_supported(s->n0) && !getenv("PYTME_B200_GENERIC_FFT");
-    s->reg1 = reg_supported(s->n1) && !getenv("PYTME_B200_GENERIC_FFT");
+    s->reg0 = reg_supported(s->n0) && !any_length;
+    s->reg1 = reg_supported(s->n1) && !any_length;
+    s->z4 = s->n2 % 2 == 0 && zpass4_supported(s->n2 / 2) && !any_length;
     size_t zy = 0;
     if (s->reg1) {
       TM_DISPATCH_N(s->n1, (zy = reg_smem_bytes<NN>(s->n2, s->t1, s->t2, true)));
@@ -1664,6 +1484,17 @@ int scan_create(const tm_scan_desc* desc, Scan** out) {
     }
     if (s->reg0) set_reg_attrs_n(s->n0, 0);
     if (s->reg1) set_reg_attrs_n(s->n1, zy);
+    {
+      const linefft::Plan* plans[3] = {&s->gen.x.plan, &s->gen.y.plan, &s->gen.z.plan};
+      for (int a = 0; a < 3; ++a) {
+        s->gtw[a] = reinterpret_cast<float4*>(b8 + o_gtw[a]);
+        const auto t = linefft::twiddle_rows(*plans[a]);
+        e = cudaMemcpy(s->gtw[a], t.data(), sizeof(float2) * t.size(), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) { int st = cuda_status(e, "scan_create: twiddles"); destroy(s); return st; }
+      }
+      const int st = gen_prepare(s->gen, d.score == TM_SCORE_FLC, s->half);
+      if (st != TM_OK) { destroy(s); return st; }
+    }
   }
   // ---- cuFFT plans: fast-shape r2c/c2r (setup and plain path), template-shape (filter)
   int r;
@@ -2013,7 +1844,6 @@ static int launch_group(Scan* s, int nb, double hs, float out_scale, int32_t fir
   TM_TRY(prepare_templates(s, nb, stream));
   tmr.end(TM_STAGE_PREPARE);
   const int64_t rows = (int64_t)s->n0 * s->n1;
-  dim3 g4(ceil_div(rows, s->R4));
   if (s->half) {
     __half2* H = static_cast<__half2*>(s->H);
     TM_TRY(launch_template_x_y<__half2>(s, nb, (float)hs, H, tmr, stream));
@@ -2021,7 +1851,7 @@ static int launch_group(Scan* s, int nb, double hs, float out_scale, int32_t fir
     if (s->d.score == TM_SCORE_FLC)
       launch_zpass_flc<__half2>(s, H, nb, rows, out_scale, first, state_max, state_rot, stream);
     else
-      launch_zpass<__half2>(s, g4, x_inner(s) ? static_cast<__half2*>(s->H2) : H, nb, rows,
+      launch_zpass<__half2>(s, x_inner(s) ? static_cast<__half2*>(s->H2) : H, nb, rows,
                             out_scale, first, state_max, state_rot, stream);
     TM_TRY(check_launch("z pass"));
     tmr.end(TM_STAGE_ZPASS);
@@ -2032,7 +1862,7 @@ static int launch_group(Scan* s, int nb, double hs, float out_scale, int32_t fir
     if (s->d.score == TM_SCORE_FLC)
       launch_zpass_flc<float2>(s, H, nb, rows, out_scale, first, state_max, state_rot, stream);
     else
-      launch_zpass<float2>(s, g4, H, nb, rows, out_scale, first, state_max, state_rot, stream);
+      launch_zpass<float2>(s, H, nb, rows, out_scale, first, state_max, state_rot, stream);
     TM_TRY(check_launch("z pass"));
     tmr.end(TM_STAGE_ZPASS);
   }
@@ -2151,44 +1981,6 @@ int scan_run(Scan* s, const float* matrices, int n, int32_t first_index, float* 
   if (n == 0) return TM_OK;
   return s->fused ? run_fused(s, n, first_index, state_max, state_rot, matrices, stream)
                   : run_plain(s, n, first_index, state_max, state_rot, matrices, stream);
-}
-
-// Line-FFT self test: y[l][:] = FFT_dir(x[l][:]) for `lines` lines of length n
-// (interleaved smem tile), used by the test-suite to check the device FFT code.
-__global__ void line_fft_test_kernel(const float2* x, float2* y, int n, int lines, LinePlan p,
-                                     const float2* tw_g, int dir) {
-  extern __shared__ float4 smem_raw[];
-  float2* tw = reinterpret_cast<float2*>(smem_raw);
-  float2* buf = tw + n;
-  for (int i = threadIdx.x; i < n; i += kThreads) tw[i] = tw_g[i];
-  for (int e = threadIdx.x; e < n * lines; e += kThreads) {
-    int i = e / lines, l = e % lines;
-    buf[e] = x[(int64_t)l * n + i];
-  }
-  __syncthreads();
-  if (dir < 0) fft::fft_lines<-1, kMaxE, true>(buf, p, lines, 1, lines, tw, n, threadIdx.x, kThreads);
-  else fft::fft_lines<1, kMaxE, true>(buf, p, lines, 1, lines, tw, n, threadIdx.x, kThreads);
-  for (int e = threadIdx.x; e < n * lines; e += kThreads) {
-    int i = e / lines, l = e % lines;
-    y[(int64_t)l * n + i] = buf[e];
-  }
-}
-
-int line_fft_test(const void* x, void* y, int n, int lines, int dir, cudaStream_t stream) {
-  TM_REQUIRE(line_supported(n), "line_fft_test: length %d not supported", n);
-  TM_REQUIRE(lines >= 1 && (int64_t)n * lines <= kTile, "line_fft_test: tile too large");
-  LinePlan p = make_line_plan(n);
-  auto tv = twiddle_table(n);
-  float2* tw = nullptr;
-  TM_TRY(cuda_status(cudaMalloc(&tw, sizeof(float2) * n), "line_fft_test: alloc"));
-  cudaMemcpy(tw, tv.data(), sizeof(float2) * n, cudaMemcpyHostToDevice);
-  size_t smem = sizeof(float2) * (n + (size_t)n * lines);
-  cudaFuncSetAttribute(line_fft_test_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max());
-  line_fft_test_kernel<<<1, kThreads, smem, stream>>>((const float2*)x, (float2*)y, n, lines, p, tw, dir);
-  int st = check_launch("line_fft_test_kernel");
-  cudaStreamSynchronize(stream);
-  cudaFree(tw);
-  return st;
 }
 
 }  // namespace tmb

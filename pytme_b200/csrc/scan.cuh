@@ -12,7 +12,8 @@ namespace tmb {
 struct Scan;
 
 fft::LinePlan make_line_plan(int n);
-int scan_create(const tm_scan_desc* desc, Scan** out);
+// any_length: FP32 plans whose axes or score the fused path of tm_scan_create refuses
+int scan_create(const tm_scan_desc* desc, Scan** out, bool any_length = false);
 int scan_destroy(Scan* s);
 int64_t scan_device_bytes(const Scan* s);
 int scan_set_template(Scan* s, const float* tmpl, const float* mask, const float* filt,

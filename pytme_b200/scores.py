@@ -81,11 +81,15 @@ class ScanPlan:
         _device()
         st = N.lib.tm_scan_create(N.ctypes.byref(desc), N.ctypes.byref(handle))
         if st == N.TM_E_UNSUPPORTED and not plain:
-            # shapes outside the fused kernels' range run on the plain path
-            desc.plain = 1
+            # axes without fused kernels of their own: the FP32 passes over any smooth
+            # length, and the plain path where those do not fit either
             desc.precision = N.TM_PREC_FP32
-            self.plain, self.precision = True, "fp32"
-            st = N.lib.tm_scan_create(N.ctypes.byref(desc), N.ctypes.byref(handle))
+            self.precision = "fp32"
+            st = N.lib.tm_scan_create_any_length(N.ctypes.byref(desc), N.ctypes.byref(handle))
+            if st in (N.TM_E_UNSUPPORTED, N.TM_E_OOM):
+                desc.plain = 1
+                self.plain = True
+                st = N.lib.tm_scan_create(N.ctypes.byref(desc), N.ctypes.byref(handle))
         N.check(st, "tm_scan_create")
         self._h = handle
         self._keep = []

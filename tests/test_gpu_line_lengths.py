@@ -1,0 +1,101 @@
+"""Scans whose axes have lengths without a kernel of their own: every radix (2 to 16, primes
+7, 11 and 13), two to five stages, odd z lengths, tiles of fewer lines and a partial launch
+group, against the FP64 oracle.
+
+Tolerance: the transforms round in FP32, about 2e-7 of the map's size per transform and at
+most a few of them in a row, so 1e-5 of the largest score holds with room to spare."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from oracle import tm_oracle as O
+
+TOL = 1e-5
+
+SHAPES = [
+    (60, 50, 40), (77, 91, 39), (66, 49, 45), (61, 47, 37), (126, 63, 52), (112, 130, 27),
+    (625, 16, 18), (1050, 24, 26), (24, 1100, 22), (16, 18, 1250), (2048, 16, 15),
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("score,order", [("FLCSphericalMask", 1), ("FLC", 3), ("CC", 1)])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_any_length_matches_oracle(shape, score, order):
+    import pytme_b200 as P
+    from pytme_b200 import synthetic as syn
+
+    rng = np.random.default_rng(sum(shape))
+    tmpl = syn.blob_template(9, rng, radius=2.5, sigma=1.0)
+    mask = None if score == "CC" else syn.dilated_threshold_mask(tmpl, 0.1, 1) \
+        if score == "FLC" else syn.spherical_mask((9,) * 3, 4.5, center=(4.0,) * 3)
+    target, _, _ = syn.make_tomogram(shape, tmpl, 3, rng, scale=0.5)
+    rots = syn.random_rotation_matrices(5, rng)
+    P.backend.change_backend("b200", precision="fp32", rotation_batch=3)
+    md = P.MatchingData(target, tmpl, template_mask=mask, rotations=rots)
+    setup, scoring = P.MATCHING_EXHAUSTIVE_REGISTER[score]
+    res = P.scan_subsets(md, matching_score=scoring, matching_setup=setup,
+                         callback_class=P.MaxScoreOverRotations,
+                         callback_class_args={"score_threshold": 0}, interpolation_order=order)
+    one = [O.scan(target, tmpl, rots[i:i + 1], score, template_mask=mask, dtype=np.float64,
+                  score_threshold=-np.inf, interpolation_order=order)["scores"]
+           for i in range(len(rots))]
+    best = np.maximum(np.max(one, axis=0), 0.0)
+    tol = TOL * max(1.0, float(np.abs(one).max()))
+    assert np.abs(res[0] - best).max() <= tol
+    picked = np.take_along_axis(np.stack(one), np.maximum(res[2], 0)[None], 0)[0]
+    assert np.all(best - np.where(res[2] < 0, 0.0, picked) <= 2 * tol)
+
+
+@pytest.mark.gpu
+def test_any_length_plan_fits_a_memory_limit():
+    """A plan of any length takes smaller launch groups under a device memory limit; the
+    scores stay."""
+    from pytme_b200 import _native as N
+    from pytme_b200 import synthetic as syn
+    from pytme_b200.matching import rigid_transform_matrices
+    from pytme_b200.scores import ScanPlan
+    import torch
+
+    rng = np.random.default_rng(3)
+    shape, t = (66, 70, 39), 10
+    tmpl = syn.blob_template(t, rng, radius=2.5, sigma=1.0)
+    mask = syn.spherical_mask((t,) * 3, t / 2, center=((t - 1) / 2,) * 3)
+    target, _, _ = syn.make_tomogram(shape, tmpl, 3, rng, scale=0.5)
+    mats = torch.as_tensor(rigid_transform_matrices(
+        syn.random_rotation_matrices(9, rng), (np.asarray(tmpl.shape) - 1) / 2), device="cuda")
+    maps, sizes = [], []
+    try:
+        for limit in (0, 12 << 20, 5 << 20):
+            N.lib.tm_set_device_memory_limit(limit)
+            plan = ScanPlan("FLCSphericalMask", shape, tmpl.shape, batch=32)
+            assert limit == 0 or plan.device_bytes <= limit
+            plan.set_template(tmpl[::-1, ::-1, ::-1], mask[::-1, ::-1, ::-1])
+            plan.set_target(target)
+            smax = torch.zeros(shape, device="cuda")
+            plan.run(mats, 0, smax, torch.full(shape, -1, dtype=torch.int32, device="cuda"))
+            maps.append(smax.cpu().numpy())
+            sizes.append(plan.device_bytes)
+            assert not plan.plain
+            plan.close()
+    finally:
+        N.lib.tm_set_device_memory_limit(0)
+    assert sizes[0] > sizes[1] > sizes[2]
+    assert np.abs(maps[1] - maps[0]).max() <= TOL and np.abs(maps[2] - maps[0]).max() <= TOL
+
+
+def test_any_length_plan_arguments():
+    """What the any-length plan refuses, it refuses before touching a device."""
+    from pytme_b200 import _native as N
+
+    desc, h = N.ScanDesc(), ctypes.c_void_p()
+    desc.score, desc.batch = N.TM_SCORE_FLC, 2
+    for precision, shape, status in ((N.TM_PREC_MIXED, (64, 64, 63), N.TM_E_UNSUPPORTED),
+                                     (N.TM_PREC_FP32, (64, 17, 64), N.TM_E_UNSUPPORTED),
+                                     (N.TM_PREC_FP32, (64, 64, 4), N.TM_E_INVALID)):
+        desc.precision = precision
+        for i in range(3):
+            desc.fast_shape[i], desc.template_shape[i] = shape[i], 8
+        assert N.lib.tm_scan_create_any_length(ctypes.byref(desc), ctypes.byref(h)) == status
+        assert not h
