@@ -9,21 +9,21 @@ size_t smem_template(const Plan& p, int w, int t1, int t2) {
   return 16 * p.pairs + sizeof(float2) * (size_t)w * (p.rows + t1 + t2) +
          sizeof(float) * (size_t)t1 * (t2 | 1);
 }
-// the tile, the target's column and two buffers of t0 inputs; for FLC three tiles
-size_t smem_x(const Plan& p, int w, int t0, bool flc) {
-  return 16 * p.pairs + sizeof(float2) * (size_t)w * (flc ? 3 * p.rows : 2 * (p.rows + t0));
+// the tile, the target's column and two buffers of t0 inputs
+size_t smem_x(const Plan& p, int w, int t0) {
+  return 16 * p.pairs + sizeof(float2) * (size_t)w * 2 * (p.rows + t0);
 }
 size_t even_tile(const Plan& p, int w, int tiles) {
   return 16 * p.pairs + sizeof(float2) * (((size_t)w * p.rows * tiles + 1) & ~(size_t)1);
 }
-size_t smem_y(const Plan& p, int w, size_t elem) { return even_tile(p, w, 1) + elem * w * p.n; }
-// z pass: tiles, the staged rows, and per voxel of 2 w rows the maximum, its rotation and (not
+size_t smem_y(const Plan& p, int w) { return even_tile(p, w, 1) + sizeof(float2) * w * p.n; }
+// z pass: tiles, the staged rows (not for FLC tiles of fewer lines), and per voxel of 2 w rows the maximum, its rotation and (not
 // for FLC) the inverse denominator
 size_t smem_z(const Plan& p, int w, int hp, bool flc, bool half) {
   const size_t wide = sizeof(float2) * staged_pitch<float2>(hp);
   const size_t own = half ? sizeof(__half2) * staged_pitch<__half2>(hp) : wide;
-  return even_tile(p, w, flc ? 3 : 1) + 2 * w * ((flc ? 2 * wide : 0) + own) +
-         2 * (size_t)w * z_pitch(p.n) * (flc ? 6 : 10);
+  const size_t rows = flc ? (w == 8 ? 2 * wide + own : 0) : own;
+  return even_tile(p, w, flc ? 3 : 1) + 2 * w * rows + 2 * (size_t)w * z_pitch(p.n) * (flc ? 6 : 10);
 }
 
 }  // namespace
@@ -45,23 +45,21 @@ GenConfig gen_config(int n0, int n1, int n2, int t0, int t1, int t2, int hp, boo
     return false;
   };
   c.ok = pick(c.t, n1, 80, [&](const Plan& p, int w) { return smem_template(p, w, t1, t2); }) &&
-         pick(c.x, n0, flc ? 128 : 80,
-              [&](const Plan& p, int w) { return smem_x(p, w, t0, flc); }) &&
-         pick(c.y, n1, 80, [&](const Plan& p, int w) { return smem_y(p, w, 8); }) &&
+         pick(c.x, n0, 80, [&](const Plan& p, int w) { return smem_x(p, w, t0); }) &&
+         pick(c.y, n1, 80, smem_y) &&
          pick(c.z, n2, 80, [&](const Plan& p, int w) { return smem_z(p, w, hp, flc, half); });
-  if (c.ok) c.smem_y_half = smem_y(c.y.plan, c.y.plan.w, 4);
+  if (flc) c.ok = c.ok && pick(c.xs, n0, 128, [](const Plan& p, int w) { return even_tile(p, w, 2); });
   return c;
 }
 
-int gen_prepare_cols(const GenConfig& c, bool half);
-int gen_prepare_x(const GenConfig& c, bool half);
-int gen_prepare_xflc(const GenConfig& c, bool half);
+int gen_prepare_cols(const GenConfig& c);
+int gen_prepare_x(const GenConfig& c, bool flc);
 int gen_prepare_z(const GenConfig& c, bool half);
 int gen_prepare_zflc(const GenConfig& c, bool half);
 
 int gen_prepare(const GenConfig& c, bool flc, bool half) {
-  TM_TRY(gen_prepare_cols(c, half));
-  TM_TRY(flc ? gen_prepare_xflc(c, half) : gen_prepare_x(c, half));
+  TM_TRY(gen_prepare_cols(c));
+  TM_TRY(gen_prepare_x(c, flc));
   return flc ? gen_prepare_zflc(c, half) : gen_prepare_z(c, half);
 }
 

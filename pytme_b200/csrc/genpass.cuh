@@ -11,7 +11,8 @@ namespace tmb {
 // Element strides of the intermediate spectra H: value (b, x', k1 or y', k2) sits at
 // b * sb + x' * sx + k1 * sr + k2. Between passes of this family H is k1-outer,
 // [b][k1][x'][k2]: the rows (x', y') of neighbouring x', which the z pass takes together, are
-// neighbours in memory; the tensor-core and power-of-two passes use row-major [b][x'][k1][k2].
+// neighbours in memory; the passes of mixed-precision plans and the four-step z pass use
+// row-major [b][x'][k1][k2].
 struct HLayout {
   int64_t sb = 0, sx = 0, sr = 0;
 };
@@ -30,9 +31,8 @@ struct GenTile {
 };
 
 struct GenConfig {
-  bool ok = false;        // every axis and tile fits
-  GenTile t, x, y, z;     // template, x, y and z pass
-  size_t smem_y_half = 0;  // the y pass over half2
+  bool ok = false;         // every axis and tile fits
+  GenTile t, x, xs, y, z;  // template, x, FLC statistics' x, y and z pass
 };
 
 // Plans and tiles of a scan over (n0, n1, n2) with a (t0, t1, t2) template.
@@ -46,14 +46,15 @@ int gen_template(const GenConfig& c, const float* tmpl, int nb, int t0, int t1, 
                  int n2, int h2, int hp, const float4* tw1, const float2* tw2, float2* G,
                  cudaStream_t st);
 int gen_xpass(const GenConfig& c, const float2* G, const float2* Ft, int nb, int t0, int n1,
-              int h2, int hp, const float4* tw0, float scale, void* H, bool half,
+              int h2, int hp, const float4* tw0, float scale, float2* H, const HLayout& hl,
+              cudaStream_t st);
+// FLC: CC(f, m) and CC(f^2, m) of the rotated masks
+int gen_xstat(const GenConfig& c, const float2* Gm, const float2* Ft, const float2* Ft2, int nb,
+              int t0, int n1, int h2, int hp, const float4* tw0, float scale, float2* Hm,
+              float2* Hm2, const HLayout& hl, cudaStream_t st);
+int gen_ypass(const GenConfig& c, float2* H, int nb, int n0, int hp, const float4* tw1,
               const HLayout& hl, cudaStream_t st);
-int gen_xpass_flc(const GenConfig& c, const float2* Gt, const float2* Gm, const float2* Ft,
-                  const float2* Ft2, int nb, int t0, int n1, int h2, int hp, const float4* tw0,
-                  float scale, void* Ht, bool half, float2* Hm, float2* Hm2, const HLayout& hl,
-                  cudaStream_t st);
-int gen_ypass(const GenConfig& c, void* H, bool half, int nb, int n0, int hp,
-              const float4* tw1, const HLayout& hl, cudaStream_t st);
+// The z passes read complex64 or half2 rows.
 int gen_zpass(const GenConfig& c, const void* H, bool half, int nb, int n0, int n1, int n2,
               int hp, const float4* tw2, float scale, const float* inv_den, int32_t first,
               const int32_t* first_dev, float* state_max, int32_t* state_rot, const HLayout& hl,
@@ -62,6 +63,6 @@ int gen_zpass_flc(const GenConfig& c, const void* Ht, bool half, const float2* H
                   const float2* Hm2, int nb, int n0, int n1, int n2, int hp, const float4* tw2,
                   float scale_t, float scale_m, const double* stats, double eps, int32_t first,
                   const int32_t* first_dev, float* state_max, int32_t* state_rot,
-                  const HLayout& hl, cudaStream_t st);
+                  const HLayout& ht, const HLayout& hl, cudaStream_t st);
 
 }  // namespace tmb

@@ -7,11 +7,11 @@ namespace tmb {
 namespace {
 
 // ------------------------------------------------------------------ template pass
-// grid (hp / w, ceil(t0 / kXPlanes), nb). Direct real DFT along z of the t1 x t2 plane for
+// grid (hp / w, ceil(t0 / planes), nb). Direct real DFT along z of the t1 x t2 plane for
 // the tile's w columns (t2 of n2 inputs are non-zero), then the zero-padded FFT along y.
 template <int W>
 __global__ void __launch_bounds__(kMaxThreads, 2)
-gen_template_kernel(const float* __restrict__ tmpl, int t0, int t1, int t2, int n2, int h2,
+gen_template_kernel(const float* __restrict__ tmpl, int planes, int t0, int t1, int t2, int n2, int h2,
                     const Plan p, const float4* __restrict__ tw1_g,
                     const float2* __restrict__ tw2_g, float2* __restrict__ G) {
   extern __shared__ float4 smem_raw[];
@@ -26,10 +26,10 @@ gen_template_kernel(const float* __restrict__ tmpl, int t0, int t1, int t2, int 
   for (int i = tid; i < p.pairs; i += nt) tw[i] = tw1_g[i];
   for (int i = tid; i < t2 * w; i += nt) {
     const int z = i / w, c = k2_0 + i % w;
-    twz[i] = c < h2 ? tw2_g[(int)(((int64_t)z * c) % n2)] : make_float2(0.f, 0.f);
+    twz[i] = c < h2 ? tw2_g[(unsigned)(z * c) % (unsigned)n2] : make_float2(0.f, 0.f);
   }
-  const int x1 = min(t0, (int)(blockIdx.y + 1) * kXPlanes);
-  for (int x = blockIdx.y * kXPlanes; x < x1; ++x) {
+  const int x1 = min(t0, (int)(blockIdx.y + 1) * planes);
+  for (int x = blockIdx.y * planes; x < x1; ++x) {
     const float* src = tmpl + ((int64_t)b * t0 + x) * t1 * t2;
     for (int y = slot; y < t1; y += p.slots)
       for (int z = l; z < t2; z += w) plane[y * pt + z] = src[y * t2 + z];
@@ -110,27 +110,27 @@ line_fft_test_kernel(const float2* x, float2* y, const Plan p, const float4* tw_
 }
 
 // ------------------------------------------------------------------ y pass
-// grid (hp / w, ceil(n0 / kYPlanes), nb): inverse FFT along y, in place. The next plane's
+// grid (hp / w, ceil(n0 / planes), nb): inverse FFT along y, in place. The next plane's
 // columns are copied to shared memory (16 bytes at a time) while the later stages of the
 // current one run.
-template <int W, typename HT>
+template <int W>
 __global__ void __launch_bounds__(kMaxThreads, 2)
-gen_ypass_kernel(HT* __restrict__ H, int n0, const Plan p, const float4* __restrict__ tw_g,
+gen_ypass_kernel(float2* __restrict__ H, int planes, int n0, const Plan p, const float4* __restrict__ tw_g,
                  const HLayout hl) {
   extern __shared__ float4 smem_raw[];
   const int w = lines<W>(p), tid = threadIdx.x, nt = blockDim.x, l = tid % w, slot = tid / w;
   float4* tw = smem_raw;
   float2* sm = reinterpret_cast<float2*>(tw + p.pairs);
-  HT* stage = reinterpret_cast<HT*>(sm + ((p.rows * w + 1) & ~1));  // n x w
+  float2* stage = reinterpret_cast<float2*>(sm + ((p.rows * w + 1) & ~1));  // n x w
   const int k2 = blockIdx.x * w;
-  const int x0 = blockIdx.y * kYPlanes, x1 = min(n0, x0 + kYPlanes);
-  HT* base = H + blockIdx.z * hl.sb + k2;
-  auto fetch = [&](const HT* src) {
+  const int x0 = blockIdx.y * planes, x1 = min(n0, x0 + planes);
+  float2* base = H + blockIdx.z * hl.sb + k2;
+  auto fetch = [&](const float2* src) {
     if constexpr (W == 8) {
-      constexpr int PER = 16 / sizeof(HT), PIECES = 8 / PER;
-      const int piece = tid % PIECES * PER;
+      constexpr int PIECES = 4;
+      const int piece = tid % PIECES * 2;
       const int64_t step = nt / PIECES * hl.sr;
-      const HT* s = src + tid / PIECES * hl.sr + piece;
+      const float2* s = src + tid / PIECES * hl.sr + piece;
       for (int row = tid / PIECES; row < p.n; row += nt / PIECES, s += step)
         async_copy16(stage + row * 8 + piece, s);
     } else {
@@ -141,48 +141,56 @@ gen_ypass_kernel(HT* __restrict__ H, int n0, const Plan p, const float4* __restr
   fetch(base + x0 * hl.sx);
   for (int i = tid; i < p.pairs; i += nt) tw[i] = tw_g[i];
   for (int x = x0; x < x1; ++x) {
-    HT* col = base + x * hl.sx;
+    float2* col = base + x * hl.sx;
     async_wait_all();
     __syncthreads();  // plane x is in; the plane before has left the tile
     TM_RADIX(p.r[0], (first_stage<W, RR, 1, false>(p, sm, tw, l, slot, 0, [&](int q) {
-      return [a = stage + q * w + l, step = p.lr[0] * w](int r) { return load_c<HT>(a + r * step); };
+      return [a = stage + q * w + l, step = p.lr[0] * w](int r) { return a[r * step]; };
     })));
     __syncthreads();
     if (x + 1 < x1) fetch(col + hl.sx);
     mid_stages<W, 1>(p, sm, tw, l, slot);
     TM_RADIX(p.rl, (last_stage<W, RR, 1>(p, sm, l, slot,
                                          [&](int q, const float2(&v)[RR], float2*) {
-      HT* d = col + out_base(p, q) * hl.sr + l;
+      float2* d = col + out_base(p, q) * hl.sr + l;
       const int64_t step = (p.n / RR) * hl.sr;
       _Pragma("unroll")
-      for (int r = 0; r < RR; ++r) store_c(d + r * step, v[r]);
+      for (int r = 0; r < RR; ++r) d[r * step] = v[r];
     })));
   }
 }
 
 }  // namespace
 
-int gen_prepare_cols(const GenConfig& c, bool half) {
+int gen_prepare_cols(const GenConfig& c) {
   TM_LINES(c.t.plan, TM_TRY(raise(gen_template_kernel<WW>)));
-  TM_LINES(c.y.plan, TM_TRY((raise(gen_ypass_kernel<WW, float2>))));
-  if (half) TM_LINES(c.y.plan, TM_TRY((raise(gen_ypass_kernel<WW, __half2>))));
+  TM_LINES(c.y.plan, TM_TRY(raise(gen_ypass_kernel<WW>)));
   return TM_OK;
+}
+
+// Planes a CTA walks: the tables are loaded once for them, so as many as leave the chip eight
+// CTAs an SM (64^3, 8 rotations: template pass 24 us with four planes, ypass 18 with eight).
+static int planes_per_cta(int64_t columns, int n, int most) {
+  while (most > 1 && columns * ceil_div(n, most) < 148 * 8) most /= 2;
+  return most;
 }
 
 int gen_template(const GenConfig& c, const float* tmpl, int nb, int t0, int t1, int t2, int n1,
                  int n2, int h2, int hp, const float4* tw1, const float2* tw2, float2* G,
                  cudaStream_t st) {
-  const dim3 g(hp / c.t.plan.w, (unsigned)ceil_div(t0, kXPlanes), nb);
+  const int planes = planes_per_cta((int64_t)hp / c.t.plan.w * nb, t0, 4);
+  const dim3 g(hp / c.t.plan.w, (unsigned)ceil_div(t0, planes), nb);
   TM_LINES(c.t.plan, (gen_template_kernel<WW><<<g, c.t.threads(), c.t.smem, st>>>(
-                     tmpl, t0, t1, t2, n2, h2, c.t.plan, tw1, tw2, G)));
+                         tmpl, planes, t0, t1, t2, n2, h2, c.t.plan, tw1, tw2, G)));
   return check_launch("gen_template_kernel");
 }
 
-int gen_ypass(const GenConfig& c, void* H, bool half, int nb, int n0, int hp,
-              const float4* tw1, const HLayout& hl, cudaStream_t st) {
-  const dim3 g(hp / c.y.plan.w, (unsigned)ceil_div(n0, kYPlanes), nb);
-  TM_STORE(half, TM_LINES(c.y.plan, (gen_ypass_kernel<WW, HT><<<g, c.y.threads(), half ? c.smem_y_half : c.y.smem, st>>>(
-                                    static_cast<HT*>(H), n0, c.y.plan, tw1, hl))));
+int gen_ypass(const GenConfig& c, float2* H, int nb, int n0, int hp, const float4* tw1,
+              const HLayout& hl, cudaStream_t st) {
+  const int planes = planes_per_cta((int64_t)hp / c.y.plan.w * nb, n0, 8);
+  const dim3 g(hp / c.y.plan.w, (unsigned)ceil_div(n0, planes), nb);
+  TM_LINES(c.y.plan, (gen_ypass_kernel<WW><<<g, c.y.threads(), c.y.smem, st>>>(
+                         H, planes, n0, c.y.plan, tw1, hl)));
   return check_launch("gen_ypass_kernel");
 }
 

@@ -1,6 +1,6 @@
 // What the kernels of the fused scan passes over axes of any length share. The passes of
 // scan.cu's scheme live in genpass_cols.cu (template rows, y pass), genpass_x.cu,
-// genpass_xflc.cu, genpass_z.cu and genpass_zflc.cu, one file each because every kernel
+// genpass_z.cu and genpass_zflc.cu, several files because every kernel
 // holds all radices; genpass.cu chooses plans and tiles.
 //
 // Every pass moves tiles of W = 8 neighbouring k2 columns (one 64-byte segment of complex64,
@@ -22,8 +22,6 @@ using namespace linefft;
 namespace {
 
 constexpr int kMaxThreads = 8 * kMaxSlots;
-constexpr int kXPlanes = 4;  // x planes per CTA of the template pass
-constexpr int kYPlanes = 8;  // x' planes per CTA of the y pass
 constexpr size_t kSmemMax = 220 * 1024;
 
 template <typename T>
@@ -32,8 +30,6 @@ template <>
 __device__ __forceinline__ float2 load_c<float2>(const float2* p) { return *p; }
 template <>
 __device__ __forceinline__ float2 load_c<__half2>(const __half2* p) { return __half22float2(*p); }
-__device__ __forceinline__ void store_c(float2* p, float2 v) { *p = v; }
-__device__ __forceinline__ void store_c(__half2* p, float2 v) { *p = __float22half2_rn(v); }
 
 // asynchronous copies global -> shared
 __device__ __forceinline__ void async_copy8(void* smem, const void* gmem) {
@@ -91,7 +87,7 @@ inline int z_pitch(int n2) { return (n2 + 27) / 32 * 32 + 4; }
 // Rotations are split over more CTAs where the columns alone leave the chip idle: the
 // target's column is then read once per chunk, from the L2.
 inline int rotations_per_cta(int64_t columns, int nb) {
-  const int64_t want = 148 * 6;
+  const int64_t want = 148 * 16;
   const int64_t chunks = std::min<int64_t>(nb, std::max<int64_t>(1, want / columns));
   return (int)ceil_div(nb, chunks);
 }

@@ -1,4 +1,4 @@
-// The x pass of the scan over axes of any length (see genpass_dev.cuh).
+// The x pass of the scan over axes of any length, and the FLC statistics' (see genpass_dev.cuh).
 #include "genpass_dev.cuh"
 
 namespace tmb {
@@ -9,11 +9,11 @@ namespace {
 // with the target spectrum, inverse FFT, H written. The column of the target, times the scale
 // of H, stays in shared memory for all rotations, in the order of the tile: the product reads
 // it at constant offsets. The next rotation's few input rows are copied in meanwhile.
-template <int W, typename HT>
+template <int W>
 __global__ void __launch_bounds__(kMaxThreads, 2)
 gen_xpass_kernel(const float2* __restrict__ G, const float2* __restrict__ Ft, int B, int per,
                  int t0, int n1, int h2, const Plan p, const float4* __restrict__ tw_g,
-                 float scale, HT* __restrict__ H, const HLayout hl) {
+                 float scale, float2* __restrict__ H, const HLayout hl) {
   extern __shared__ float4 smem_raw[];
   const int w = lines<W>(p), tid = threadIdx.x, nt = blockDim.x, l = tid % w, slot = tid / w;
   float4* tw = smem_raw;
@@ -66,32 +66,103 @@ gen_xpass_kernel(const float2* __restrict__ G, const float2* __restrict__ Ft, in
     async_wait_all();  // the next inputs, for every thread after the barrier
     __syncthreads();
     mid_adjoints<W>(p, sm, tw, l, slot);
-    HT* h = H + b * hl.sb + k1 * hl.sr + k2;
+    float2* h = H + b * hl.sb + k1 * hl.sr + k2;
     // the next rotation's first stage writes the rows this thread reads here
     TM_RADIX(p.r[0], (first_adjoint<W, RR>(p, sm, tw, l, slot, [&](int q) {
       return [a = h + q * hl.sx, step = p.lr[0] * hl.sx](int r, float2 v) {
-        store_c(a + r * step, v);
+        a[r * step] = v;
       };
     })));
   }
 }
 
+// FLC statistics: the rotated mask's spectrum times the spectra of f and f^2, two inverse
+// transforms of one forward transform.
+template <int W>
+__global__ void __launch_bounds__(kMaxThreads, 1)
+gen_xstat_kernel(const float2* __restrict__ Gm, const float2* __restrict__ Ft,
+                 const float2* __restrict__ Ft2, int B, int per, int t0, int n1, int h2,
+                 const Plan p, const float4* __restrict__ tw_g, float scale,
+                 float2* __restrict__ Hm, float2* __restrict__ Hm2, const HLayout hl) {
+  extern __shared__ float4 smem_raw[];
+  const int w = lines<W>(p), tid = threadIdx.x, nt = blockDim.x, l = tid % w, slot = tid / w;
+  float4* tw = smem_raw;
+  float2* sm = reinterpret_cast<float2*>(tw + p.pairs);
+  const int tile = p.rows * w;  // tiles: mask, then CC(f, m); CC(f^2, m)
+  const int k2 = blockIdx.x * w + l, k1 = blockIdx.y;
+  const bool valid = k2 < h2;  // the row padding is transformed as zeros
+  for (int i = tid; i < p.pairs; i += nt) tw[i] = tw_g[i];
+  __syncthreads();
+  const int64_t row_s = (int64_t)n1 * h2, col = (int64_t)k1 * h2 + min(k2, h2 - 1);
+  const int b1 = min(B, (int)(blockIdx.z + 1) * per);
+  for (int b = blockIdx.z * per; b < b1; ++b) {
+    const float2* g = Gm + (int64_t)b * t0 * row_s + col;
+    TM_RADIX(p.r[0], (first_stage<W, RR, -1, true>(p, sm, tw, l, slot, t0, [&](int q) {
+      // the scale of H goes in with the few inputs
+      return [&, a = g + q * row_s, step = p.lr[0] * row_s](int r) {
+        if (!valid) return make_float2(0.f, 0.f);
+        const float2 c = __ldg(a + r * step);
+        return make_float2(c.x * scale, c.y * scale);
+      };
+    })));
+    __syncthreads();
+    mid_stages<W, -1>(p, sm, tw, l, slot);
+    TM_RADIX(p.rl, (last_stage<W, RR, -1>(p, sm, l, slot, [&](int q, float2(&v)[RR], float2* d) {
+      const int64_t at = col + out_base(p, q) * row_s, step = (p.n / RR) * row_s;
+      float2 u[RR];
+      _Pragma("unroll")
+      for (int r = 0; r < RR; ++r) u[r] = fft::cmul(v[r], __ldg(Ft2 + at + r * step));
+      fft::dft_small<RR, 1>(u);
+      _Pragma("unroll")
+      for (int r = 0; r < RR; ++r) d[tile + r * w] = u[r];
+      _Pragma("unroll")
+      for (int r = 0; r < RR; ++r) v[r] = fft::cmul(v[r], __ldg(Ft + at + r * step));
+      fft::dft_small<RR, 1>(v);
+      _Pragma("unroll")
+      for (int r = 0; r < RR; ++r) d[r * w] = v[r];
+    })));
+    __syncthreads();
+    for (int s = p.ns - 2; s >= 1; --s) {
+      for (int i = 0; i < 2; ++i)
+        TM_RADIX(p.r[s], (mid_adjoint<W, RR>(p, s, sm + i * tile, tw, l, slot)));
+      __syncthreads();
+    }
+    const int64_t h0 = b * hl.sb + k1 * hl.sr + k2;
+    for (int i = 0; i < 2; ++i) {
+      float2* h = (i ? Hm2 : Hm) + h0;
+      TM_RADIX(p.r[0], (first_adjoint<W, RR>(p, sm + i * tile, tw, l, slot, [&](int q) {
+        return [a = h + q * hl.sx, step = p.lr[0] * hl.sx](int r, float2 v) { a[r * step] = v; };
+      })));
+    }
+  }
+}
+
 }  // namespace
 
-int gen_prepare_x(const GenConfig& c, bool half) {
-  TM_STORE(half, TM_LINES(c.x.plan, TM_TRY((raise(gen_xpass_kernel<WW, HT>)))));
+int gen_prepare_x(const GenConfig& c, bool flc) {
+  TM_LINES(c.x.plan, TM_TRY(raise(gen_xpass_kernel<WW>)));
+  if (flc) TM_LINES(c.xs.plan, TM_TRY(raise(gen_xstat_kernel<WW>)));
   return TM_OK;
 }
 
 int gen_xpass(const GenConfig& c, const float2* G, const float2* Ft, int nb, int t0, int n1,
-              int h2, int hp, const float4* tw0, float scale, void* H, bool half,
-              const HLayout& hl, cudaStream_t st) {
+              int h2, int hp, const float4* tw0, float scale, float2* H, const HLayout& hl,
+              cudaStream_t st) {
   const int per = rotations_per_cta((int64_t)(hp / c.x.plan.w) * n1, nb);
   const dim3 g(hp / c.x.plan.w, n1, (unsigned)ceil_div(nb, per));
-  TM_STORE(half, TM_LINES(c.x.plan, (gen_xpass_kernel<WW, HT><<<g, c.x.threads(), c.x.smem, st>>>(
-                                    G, Ft, nb, per, t0, n1, h2, c.x.plan, tw0, scale,
-                                    static_cast<HT*>(H), hl))));
+  TM_LINES(c.x.plan, (gen_xpass_kernel<WW><<<g, c.x.threads(), c.x.smem, st>>>(
+                         G, Ft, nb, per, t0, n1, h2, c.x.plan, tw0, scale, H, hl)));
   return check_launch("gen_xpass_kernel");
+}
+
+int gen_xstat(const GenConfig& c, const float2* Gm, const float2* Ft, const float2* Ft2, int nb,
+              int t0, int n1, int h2, int hp, const float4* tw0, float scale, float2* Hm,
+              float2* Hm2, const HLayout& hl, cudaStream_t st) {
+  const int per = rotations_per_cta((int64_t)(hp / c.xs.plan.w) * n1, nb);
+  const dim3 g(hp / c.xs.plan.w, n1, (unsigned)ceil_div(nb, per));
+  TM_LINES(c.xs.plan, (gen_xstat_kernel<WW><<<g, c.xs.threads(), c.xs.smem, st>>>(
+                          Gm, Ft, Ft2, nb, per, t0, n1, h2, c.xs.plan, tw0, scale, Hm, Hm2, hl)));
+  return check_launch("gen_xstat_kernel");
 }
 
 }  // namespace tmb

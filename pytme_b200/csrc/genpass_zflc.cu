@@ -19,7 +19,7 @@ gen_zpass_flc_kernel(const HT* __restrict__ Ht, const float2* __restrict__ Hm,
                      const Plan p, const float4* __restrict__ tw_g, float scale_t, float scale_m,
                      const double* __restrict__ stats, double eps, int32_t first,
                      const int32_t* __restrict__ first_dev, float* __restrict__ state_max,
-                     int32_t* __restrict__ state_rot, const HLayout hl, int zp) {
+                     int32_t* __restrict__ state_rot, const HLayout ht, const HLayout hl, int zp) {
   if (first_dev) first = *first_dev;
   extern __shared__ float4 smem_raw[];
   const int w = lines<W>(p), tid = threadIdx.x, nt = blockDim.x, l = tid % w, slot = tid / w;
@@ -29,48 +29,56 @@ gen_zpass_flc_kernel(const HT* __restrict__ Ht, const float2* __restrict__ Hm,
   float2* sm = reinterpret_cast<float2*>(tw + p.pairs);
   const int tile = p.rows * w;
   const int pm = staged_pitch<float2>(hp), pt = staged_pitch<HT>(hp);
-  float2* rm = sm + ((3 * tile + 1) & ~1);  // staged rows of Hm, of Hm2, of Ht
+  // staged rows of Hm, of Hm2, of Ht; long lines (W = 0) are read from global memory instead
+  float2* rm = sm + ((3 * tile + 1) & ~1);
   float2* rm2 = rm + rows2 * pm;
   HT* rt = reinterpret_cast<HT*>(rm2 + rows2 * pm);
-  float* best = reinterpret_cast<float*>(rt + rows2 * pt);
+  float* best = reinterpret_cast<float*>(W ? rt + rows2 * pt : reinterpret_cast<HT*>(rm));
   uint16_t* arg = reinterpret_cast<uint16_t*>(best + rows2 * zp);
   const int y = blockIdx.x, x0 = blockIdx.y * rows2, nrows = min(rows2, n0 - x0);
-  const int64_t off = x0 * hl.sx + y * hl.sr;
+  const int64_t off = x0 * hl.sx + y * hl.sr, offt = x0 * ht.sx + y * ht.sr;
   auto stage = [&](int b) {
     const int64_t o = off + b * hl.sb;
     stage_rows<float2>(rm, Hm + o, nrows, hp, hl.sx, l, w, slot, p.slots);
     stage_rows<float2>(rm2, Hm2 + o, nrows, hp, hl.sx, l, w, slot, p.slots);
-    stage_rows<HT>(rt, Ht + o, nrows, hp, hl.sx, l, w, slot, p.slots);
+    stage_rows<HT>(rt, Ht + offt + b * ht.sb, nrows, hp, ht.sx, l, w, slot, p.slots);
     async_commit();
   };
-  stage(0);
+  if constexpr (W) stage(0);
   // rows past the edge repeat the last one; their voxels are not stored
   const int ra = min(l, nrows - 1), rb = min(l + w, nrows - 1);
   for (int i = tid; i < p.pairs; i += nt) tw[i] = tw_g[i];
   for (int i = tid; i < rows2 * zp; i += nt) best[i] = -INFINITY;
   const double eps2 = eps * eps;
   for (int b = 0; b < B; ++b) {
-    async_wait_all();
+    if constexpr (W) async_wait_all();
     __syncthreads();  // rotation b's rows are in; the tiles are free
+    const int64_t o = off + b * hl.sb;
+    const float2 *ma = W ? rm + ra * pm : Hm + o + ra * hl.sx;
+    const float2 *mb = W ? rm + rb * pm : Hm + o + rb * hl.sx;
+    const float2 *sa = W ? rm2 + ra * pm : Hm2 + o + ra * hl.sx;
+    const float2 *sb = W ? rm2 + rb * pm : Hm2 + o + rb * hl.sx;
+    const HT *ta = W ? rt + ra * pt : Ht + offt + b * ht.sb + ra * ht.sx;
+    const HT *tb = W ? rt + rb * pt : Ht + offt + b * ht.sb + rb * ht.sx;
     TM_RADIX(p.r[0], ({
       first_stage<W, RR, 1, false>(p, sm, tw, l, slot, 0, [&](int q) {
         return [=, lr = p.lr[0]](int r) {
-          return pair_input<RR>(rm + ra * pm, rm2 + ra * pm, q, r, lr, n2);
+          return pair_input<RR>(ma, sa, q, r, lr, n2);
         };
       });
       first_stage<W, RR, 1, false>(p, sm + tile, tw, l, slot, 0, [&](int q) {
         return [=, lr = p.lr[0]](int r) {
-          return pair_input<RR>(rm + rb * pm, rm2 + rb * pm, q, r, lr, n2);
+          return pair_input<RR>(mb, sb, q, r, lr, n2);
         };
       });
       first_stage<W, RR, 1, false>(p, sm + 2 * tile, tw, l, slot, 0, [&](int q) {
         return [=, lr = p.lr[0]](int r) {
-          return pair_input<RR>(rt + ra * pt, rt + rb * pt, q, r, lr, n2);
+          return pair_input<RR>(ta, tb, q, r, lr, n2);
         };
       });
     }));
     __syncthreads();
-    if (b + 1 < B) stage(b + 1);
+    if (W && b + 1 < B) stage(b + 1);
     for (int s = 1; s < p.ns - 1; ++s) {
       TM_RADIX(p.r[s], ({
         for (int i = 0; i < 3; ++i) mid_stage<W, RR, 1>(p, s, sm + i * tile, tw, l, slot);
@@ -128,12 +136,12 @@ int gen_zpass_flc(const GenConfig& c, const void* Ht, bool half, const float2* H
                   const float2* Hm2, int nb, int n0, int n1, int n2, int hp, const float4* tw2,
                   float scale_t, float scale_m, const double* stats, double eps, int32_t first,
                   const int32_t* first_dev, float* state_max, int32_t* state_rot,
-                  const HLayout& hl, cudaStream_t st) {
+                  const HLayout& ht, const HLayout& hl, cudaStream_t st) {
   const dim3 g(n1, (unsigned)ceil_div(n0, 2 * c.z.plan.w));
   TM_STORE(half, TM_LINES(c.z.plan, (gen_zpass_flc_kernel<WW, HT><<<g, c.z.threads(), c.z.smem, st>>>(
                                     static_cast<const HT*>(Ht), Hm, Hm2, nb, n0, n1, n2, hp,
                                     c.z.plan, tw2, scale_t, scale_m, stats, eps,
-                                    first, first_dev, state_max, state_rot, hl, z_pitch(n2)))));
+                                    first, first_dev, state_max, state_rot, ht, hl, z_pitch(n2)))));
   return check_launch("gen_zpass_flc_kernel");
 }
 

@@ -1,0 +1,32 @@
+// Template rows, x pass and y pass of mixed-precision plans (halfpass.cu).
+#pragma once
+
+#include <cuda_runtime.h>
+#include <cstdint>
+
+#include "fft_smem.cuh"
+
+namespace tmb {
+
+struct HalfConfig {
+  bool reg0 = false, reg1 = false;  // register-resident columns along x / y
+  fft::LinePlan p0{}, p1{};
+  int w0 = 1, w1 = 1;               // lines of a tile of the other lengths
+  size_t smt = 0, smx = 0, smy = 0;  // their shared memory
+};
+
+HalfConfig half_config(int n0, int n1, int n2, int h2, int t1, int t2);
+int half_prepare(const HalfConfig& c, int n0, int n1);
+// G[b][x][k1][h2] as complex64 or (register-resident y columns) half2.
+int half_template(const HalfConfig& c, const float* tmpl, int nb, int t0, int t1, int t2, int n1,
+                  int n2, int h2, const float2* tw1, const float2* tw2, void* G, bool half_g,
+                  cudaStream_t st);
+// Row-major half2 H; flc: the numerators of an FLC plan (register-resident columns).
+int half_xpass(const HalfConfig& c, const float2* G, const float2* Ft, int nb, int t0, int n0,
+               int n1, int h2, int hp, const float2* tw0, float scale, void* H, bool flc,
+               cudaStream_t st);
+// In place; seg: rows as 32-byte segments [Re x 8 | Im x 8] (register-resident columns only).
+int half_ypass(const HalfConfig& c, void* H, int nb, int n0, int n1, int h2, int hp,
+               const float2* tw1, bool seg, cudaStream_t st);
+
+}  // namespace tmb

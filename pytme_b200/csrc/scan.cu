@@ -27,10 +27,10 @@
 // Target-side quantities (target spectra and the FLCSphericalMask denominator)
 // are computed once by set_target; the denominator and the target mean are
 // evaluated in double precision.
-#include "colfft.cuh"
 #include "common.cuh"
 #include "fft_smem.cuh"
 #include "genpass.cuh"
+#include "halfpass.cuh"
 #include "ops.cuh"
 #include "scan.cuh"
 #include "tc_common.cuh"
@@ -45,12 +45,9 @@
 
 #include <algorithm>
 #include <cmath>
-#include <cstdlib>
 #include <vector>
 
 namespace tmb {
-
-using fft::LinePlan;
 
 static int cufft_status(cufftResult r, const char* what) {
   if (r == CUFFT_SUCCESS) return TM_OK;
@@ -58,28 +55,19 @@ static int cufft_status(cufftResult r, const char* what) {
   return r == CUFFT_ALLOC_FAILED ? TM_E_OOM : TM_E_CUFFT;
 }
 
-LinePlan make_line_plan(int n) {
-  LinePlan p{};
-  p.n = n;
-  int m = n, e2 = 0;
-  while (m % 2 == 0) { m /= 2; ++e2; }
-  int k = 0;
-  int eights = e2 / 3, rem = e2 % 3;
-  if (rem == 1 && eights > 0) { eights -= 1; p.radix[k++] = 4; p.radix[k++] = 4; }
-  else if (rem == 1) { p.radix[k++] = 2; }
-  else if (rem == 2) { p.radix[k++] = 4; }
-  for (int i = 0; i < eights; ++i) p.radix[k++] = 8;
-  for (int q : {3, 5, 7, 11, 13}) {
-    while (m % q == 0) { m /= q; p.radix[k++] = q; }
-  }
-  p.npass = (m == 1) ? k : -1;
-  return p;
+constexpr int kMaxLine = 4096;
+
+// Axis lengths of tm_scan_create's fused plans: 5-smooth, 2 to 4096.
+static bool line_supported(int n) {
+  if (n < 2 || n > kMaxLine) return false;
+  for (int q : {2, 3, 5})
+    while (n % q == 0) n /= q;
+  return n == 1;
 }
 
-static bool line_supported(int n) {
-  if (n < 2 || n > 4096) return false;
-  LinePlan p = make_line_plan(n);
-  return p.npass > 0 && p.npass <= fft::kMaxPasses && fft::supported_radices(p);
+// x and y lengths of its FLC plans.
+static bool flc_supported(int n) {
+  return n == 64 || n == 128 || n == 256 || n == 512 || n == 1024;
 }
 
 static std::vector<float2> twiddle_table(int n) {
@@ -119,495 +107,7 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(PENDING));
 }
 
-constexpr int kThreads = 512;
-constexpr int kMaxE = 8;             // complex elements per thread in a line-FFT tile
-constexpr int kTile = kThreads * kMaxE;  // elements per tile (4096)
-
-// ------------------------------------------------------------------ register-resident passes
-// Power-of-two axis lengths use the column codelet of colfft.cuh: T = N/8 threads
-// per column, W columns per CTA (thread id = t*W + l, so a warp spans W columns and
-// each global row segment of W elements is one contiguous access).
-
-// Stage 0 of the forward DIF when only rows [0, nz) of the column are non-zero and
-// nz <= T: the radix-8 DFT of a single non-zero input is that input, so output j is
-// x[t] * W_N^(j*t).
-template <int N>
-__device__ __forceinline__ void stage0_single(float2 (&v)[8], int t, const float2* tw) {
-  const float2 w1 = tw[t];
-  float2 x = v[0];
-  v[0] = x;
-#pragma unroll
-  for (int j = 1; j < 8; ++j) {
-    x = fft::cmul(x, w1);
-    v[j] = x;
-  }
-}
-
-template <int N, int W, int DIR>
-__device__ __forceinline__ void dif_rest(float2 (&v)[8], float2* sm, const float2* tw, int l,
-                                         int t) {
-  constexpr int NS = colfft::num_stages(N);
-  colfft::store_stage<N, W, 0>(v, sm, l, t);
-  __syncthreads();
-  if constexpr (NS > 1) {
-    colfft::load_stage<N, W, 1>(v, sm, l, t);
-    colfft::dif_stage_regs<N, 1, DIR>(v, t, tw);
-  }
-  if constexpr (NS > 2) {
-    colfft::store_stage<N, W, 1>(v, sm, l, t);
-    __syncthreads();
-    colfft::load_stage<N, W, 2>(v, sm, l, t);
-    colfft::dif_stage_regs<N, 2, DIR>(v, t, tw);
-  }
-  if constexpr (NS > 3) {
-    colfft::store_stage<N, W, 2>(v, sm, l, t);
-    __syncthreads();
-    colfft::load_stage<N, W, 3>(v, sm, l, t);
-    colfft::dif_stage_regs<N, 3, DIR>(v, t, tw);
-  }
-}
-
-// K1': template rows -> G. grid (ceil(h2/W), t0, B); N = n1.
-template <int N, int W, typename GT = float2>
-__global__ void __launch_bounds__(N / 8 * W, 1)
-tmpl_zy_reg_kernel(const float* __restrict__ tmpl, int t0, int t1, int t2, int n2, int h2,
-                   const float2* __restrict__ tw1_g, const float2* __restrict__ tw2_g,
-                   GT* __restrict__ G) {
-  constexpr int T = N / 8;
-  constexpr int NT = T * W;
-  extern __shared__ float4 smem_raw[];
-  float2* tw1 = reinterpret_cast<float2*>(smem_raw);
-  float2* sm = tw1 + N;
-  float2* tw2 = sm + colfft::smem_elems<N>(W);
-  float* plane = reinterpret_cast<float*>(tw2 + n2);
-  const int tid = threadIdx.x, l = tid % W, t = tid / W;
-  const int k2 = blockIdx.x * W + l;
-  const int x = blockIdx.y, b = blockIdx.z;
-  for (int i = tid; i < N; i += NT) tw1[i] = tw1_g[i];
-  for (int i = tid; i < n2; i += NT) tw2[i] = tw2_g[i];
-  const float* src = tmpl + ((int64_t)b * t0 + x) * t1 * t2;
-  for (int i = tid; i < t1 * t2; i += NT) plane[i] = src[i];
-  __syncthreads();
-  float2 v[8];
-#pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    const int y = t + T * r;
-    float2 acc = make_float2(0.f, 0.f);
-    if (y < t1 && k2 < h2) {
-      const float* row = plane + y * t2;
-      int idx = 0;
-      for (int z = 0; z < t2; ++z) {
-        const float a = row[z];
-        const float2 w = tw2[idx];
-        acc.x += a * w.x;
-        acc.y += a * w.y;
-        idx += k2;
-        if (idx >= n2) idx -= n2;
-      }
-    }
-    v[r] = acc;
-  }
-  if (t1 <= T) stage0_single<N>(v, t, tw1);
-  else colfft::dif_stage_regs<N, 0, -1>(v, t, tw1);
-  dif_rest<N, W, -1>(v, sm, tw1, l, t);
-  if (k2 < h2) {
-    GT* dst = G + ((int64_t)b * t0 + x) * N * h2;
-    constexpr int R = colfft::stage_radix(N, colfft::num_stages(N) - 1);
-#pragma unroll
-    for (int i = 0; i < 8 / R; ++i)
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int k1 = colfft::out_index<N>(t, i, r);
-        Store<GT>::store(dst + (int64_t)k1 * h2 + k2, v[i * R + r]);
-      }
-  }
-}
-
-// K2': x pass. grid (ceil(h2/W), n1); N = n0; loops over the rotations of the group.
-template <int N, int W, typename HT>
-__global__ void __launch_bounds__(N / 8 * W, 1024 / (N / 8 * W))
-xpass_reg_kernel(const float2* __restrict__ G, const float2* __restrict__ Ft, int B, int t0,
-                 int n1, int h2, const float2* __restrict__ tw0_g, float scale,
-                 HT* __restrict__ H, int hp) {
-  constexpr int T = N / 8;
-  constexpr int NT = T * W;
-  constexpr int R = colfft::stage_radix(N, colfft::num_stages(N) - 1);
-  extern __shared__ float4 smem_raw[];
-  float2* tw = reinterpret_cast<float2*>(smem_raw);
-  float2* sm = tw + N;
-  const int tid = threadIdx.x, l = tid % W, t = tid / W;
-  const int k2 = blockIdx.x * W + l;
-  const int k1 = blockIdx.y;
-  const bool valid = k2 < h2;
-  for (int i = tid; i < N; i += NT) tw[i] = tw0_g[i];
-  // offsets of the target-spectrum values this thread multiplies (through L1, reused
-  // by every rotation of the group)
-  const int64_t col = (int64_t)k1 * h2 + k2;
-  const int64_t row = (int64_t)n1 * h2;
-  const float2* fb = Ft + (int64_t)colfft::out_index<N>(t, 0, 0) * row + col;
-  __syncthreads();
-  const int64_t SH = (int64_t)N * n1 * hp, rowH = (int64_t)n1 * hp;
-  const int64_t colH = (int64_t)k1 * hp + k2;
-  for (int b = 0; b < B; ++b) {
-    const float2* g = G + (int64_t)b * t0 * row + col;
-    float2 v[8];
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      const int x = t + T * r;
-      v[r] = (valid && x < t0) ? g[(int64_t)x * row] : make_float2(0.f, 0.f);
-    }
-    if (t0 <= T) stage0_single<N>(v, t, tw);
-    else colfft::dif_stage_regs<N, 0, -1>(v, t, tw);
-    dif_rest<N, W, -1>(v, sm, tw, l, t);
-#pragma unroll
-    for (int i = 0; i < 8 / R; ++i)
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        // out_index(t, i, r) = out_index(t, i, 0) + r * N/R; out_index(t, i, 0) - out_index(t, 0, 0)
-        // depends on i only through compile-time digits
-        const int dk = colfft::out_index<N>(t, i, r) - colfft::out_index<N>(t, 0, 0);
-        const float2 f = valid ? __ldg(fb + (int64_t)dk * row) : make_float2(0.f, 0.f);
-        v[i * R + r] = fft::cmul(v[i * R + r], make_float2(f.x * scale, f.y * scale));
-      }
-    colfft::dif_adjoint<N, W>(v, sm, tw, l, t);
-    if (valid) {
-      HT* h = H + (int64_t)b * SH + colH;
-#pragma unroll
-      for (int r = 0; r < 8; ++r) Store<HT>::store(h + (int64_t)(t + T * r) * rowH, v[r]);
-    }
-  }
-}
-
-// K3': y pass (inverse FFT along axis 1, in place). grid (ceil(h2/W), ceil(n0/XP), B);
-// each CTA walks XP consecutive x planes; the next plane's columns are staged in shared
-// memory with cp.async while the current plane is transformed (each thread stages and
-// later reads only its own elements, so a stage is reused without a barrier). The pass
-// is bound by instruction issue and shared-memory traffic, not by loads in flight:
-// three or four staged planes measured slower than two. N = n1.
-constexpr int kYPlanes = 8;
-constexpr int kYStages = 2;
-
-template <int N, int W, typename HT>
-__global__ void __launch_bounds__(N / 8 * W, 1024 / (N / 8 * W))
-ypass_reg_kernel(HT* __restrict__ H, int n0, int h2, const float2* __restrict__ tw1_g, int hp,
-                 int seg) {
-  constexpr int T = N / 8;
-  constexpr int NT = T * W;
-  constexpr int R = colfft::stage_radix(N, colfft::num_stages(N) - 1);
-  extern __shared__ float4 smem_raw[];
-  float2* tw = reinterpret_cast<float2*>(smem_raw);
-  float2* sm = tw + N;
-  HT* stage = reinterpret_cast<HT*>(sm + colfft::smem_elems<N>(W));  // kYStages x N*W staging
-  const int tid = threadIdx.x, l = tid % W, t = tid / W;
-  const int k2 = blockIdx.x * W + l;
-  const int x0 = blockIdx.y * kYPlanes, b = blockIdx.z;
-  const int nx = min(kYPlanes, n0 - x0);
-  const bool valid = k2 < h2;
-  for (int i = tid; i < N; i += NT) tw[i] = tw1_g[i];
-  HT* base = H + ((int64_t)b * n0 + x0) * N * hp + k2;
-  const int64_t plane = (int64_t)N * hp;
-  auto fetch = [&](int xi) {
-    if (valid && xi < nx) {
-      HT* dst = stage + (xi % kYStages) * N * W;
-      const HT* src = base + (int64_t)xi * plane;
-#pragma unroll
-      for (int r = 0; r < 8; ++r)
-        cp_async<sizeof(HT)>(dst + (t + T * r) * W + l, src + (int64_t)(t + T * r) * hp);
-    }
-    cp_async_commit();  // one group per plane, empty past the last
-  };
-#pragma unroll
-  for (int xi = 0; xi < kYStages - 1; ++xi) fetch(xi);
-  __syncthreads();  // twiddles
-  for (int xi = 0; xi < nx; ++xi) {
-    HT* cur = stage + (xi % kYStages) * N * W;
-    fetch(xi + kYStages - 1);
-    cp_async_wait<kYStages - 1>();  // plane xi landed
-    float2 v[8];
-#pragma unroll
-    for (int r = 0; r < 8; ++r)
-      v[r] = valid ? Store<HT>::load(cur + (t + T * r) * W + l) : make_float2(0.f, 0.f);
-    colfft::dif_stage_regs<N, 0, 1>(v, t, tw);
-    dif_rest<N, W, 1>(v, sm, tw, l, t);
-    if constexpr (std::is_same<HT, __half2>::value) {
-      if (seg) {
-        // 32-byte segments [Re x 8 | Im x 8] of 8 consecutive k2 (the even/odd tensor-core
-        // z pass's input): the 8 lanes holding one row's segment exchange values so each
-        // stores one word, (Re, Re) of columns 2q, 2q+1 for q < 4, (Im, Im) after that
-        const int q = l & 7, lane = threadIdx.x & 31;
-        const int srcA = (lane & ~7) | ((2 * q) & 7);
-        const uint32_t sel = q < 4 ? 0x5410u : 0x7632u;
-        HT* h = base + (int64_t)xi * plane;
-#pragma unroll
-        for (int i = 0; i < 8 / R; ++i)
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            const int y = colfft::out_index<N>(t, i, r);
-            const __half2 hv = __float22half2_rn(v[i * R + r]);
-            uint32_t w = *reinterpret_cast<const uint32_t*>(&hv);
-            const uint32_t a = __shfl_sync(0xffffffffu, w, srcA);
-            const uint32_t b = __shfl_sync(0xffffffffu, w, srcA + 1);
-            w = __byte_perm(a, b, sel);
-            if (k2 < hp) *reinterpret_cast<uint32_t*>(h + (int64_t)y * hp) = w;
-          }
-        __syncthreads();  // the next plane's stage-0 stores reuse the exchange buffer
-        continue;
-      }
-    }
-    if (valid) {
-      HT* h = base + (int64_t)xi * plane;
-#pragma unroll
-      for (int i = 0; i < 8 / R; ++i)
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int y = colfft::out_index<N>(t, i, r);
-          Store<HT>::store(h + (int64_t)y * hp, v[i * R + r]);
-        }
-    }
-    __syncthreads();  // the next plane's stage-0 stores reuse the exchange buffer
-  }
-}
-
-// K2'' (FLC): x pass with three outputs per rotation. The rotated mask's spectrum is
-// transformed once and multiplied by the spectra of f and f^2 (the local mean and
-// mean square under the mask, CC(f, m) and CC(f^2, m)); the normalised template's
-// spectrum is multiplied by the spectrum of f (the numerator). The two statistics
-// outputs are always complex64.
-template <int N, int W, typename HT>
-__global__ void __launch_bounds__(N / 8 * W, 1)
-xpass_flc_reg_kernel(const float2* __restrict__ Gt, const float2* __restrict__ Gm,
-                     const float2* __restrict__ Ft, const float2* __restrict__ Ft2, int B, int t0,
-                     int n1, int h2, const float2* __restrict__ tw0_g, float scale,
-                     HT* __restrict__ Ht, float2* __restrict__ Hm, float2* __restrict__ Hm2,
-                     int hp) {
-  constexpr int T = N / 8;
-  constexpr int NT = T * W;
-  constexpr int R = colfft::stage_radix(N, colfft::num_stages(N) - 1);
-  extern __shared__ float4 smem_raw[];
-  float2* tw = reinterpret_cast<float2*>(smem_raw);
-  float2* sm = tw + N;
-  const int tid = threadIdx.x, l = tid % W, t = tid / W;
-  const int k2 = blockIdx.x * W + l;
-  const int k1 = blockIdx.y;
-  const bool valid = k2 < h2;
-  for (int i = tid; i < N; i += NT) tw[i] = tw0_g[i];
-  int64_t foff[8];
-#pragma unroll
-  for (int i = 0; i < 8 / R; ++i)
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int k0 = colfft::out_index<N>(t, i, r);
-      foff[i * R + r] = ((int64_t)k0 * n1 + k1) * h2 + k2;
-    }
-  __syncthreads();
-  const int64_t row = (int64_t)n1 * h2;
-  const int64_t col = (int64_t)k1 * h2 + k2;
-  const int64_t S = (int64_t)N * n1 * hp, rowH = (int64_t)n1 * hp;
-  const int64_t colH = (int64_t)k1 * hp + k2;
-  for (int b = 0; b < B; ++b) {
-    // mask spectrum along axis 0
-    float2 vm[8], v[8];
-    const float2* gm = Gm + (int64_t)b * t0 * row + col;
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      const int x = t + T * r;
-      vm[r] = (valid && x < t0) ? gm[(int64_t)x * row] : make_float2(0.f, 0.f);
-    }
-    if (t0 <= T) stage0_single<N>(vm, t, tw);
-    else colfft::dif_stage_regs<N, 0, -1>(vm, t, tw);
-    dif_rest<N, W, -1>(vm, sm, tw, l, t);
-    // CC(f, m)
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      float2 f = valid ? __ldg(Ft + foff[e]) : make_float2(0.f, 0.f);
-      v[e] = fft::cmul(vm[e], make_float2(f.x * scale, f.y * scale));
-    }
-    colfft::dif_adjoint<N, W>(v, sm, tw, l, t);
-    if (valid) {
-      float2* h = Hm + (int64_t)b * S + colH;
-#pragma unroll
-      for (int r = 0; r < 8; ++r) h[(int64_t)(t + T * r) * rowH] = v[r];
-    }
-    __syncthreads();
-    // CC(f^2, m)
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      float2 f = valid ? __ldg(Ft2 + foff[e]) : make_float2(0.f, 0.f);
-      v[e] = fft::cmul(vm[e], make_float2(f.x * scale, f.y * scale));
-    }
-    colfft::dif_adjoint<N, W>(v, sm, tw, l, t);
-    if (valid) {
-      float2* h = Hm2 + (int64_t)b * S + colH;
-#pragma unroll
-      for (int r = 0; r < 8; ++r) h[(int64_t)(t + T * r) * rowH] = v[r];
-    }
-    __syncthreads();
-    // numerator CC(f, t)
-    const float2* gt = Gt + (int64_t)b * t0 * row + col;
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      const int x = t + T * r;
-      v[r] = (valid && x < t0) ? gt[(int64_t)x * row] : make_float2(0.f, 0.f);
-    }
-    if (t0 <= T) stage0_single<N>(v, t, tw);
-    else colfft::dif_stage_regs<N, 0, -1>(v, t, tw);
-    dif_rest<N, W, -1>(v, sm, tw, l, t);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      float2 f = valid ? __ldg(Ft + foff[e]) : make_float2(0.f, 0.f);
-      v[e] = fft::cmul(v[e], make_float2(f.x * scale, f.y * scale));
-    }
-    colfft::dif_adjoint<N, W>(v, sm, tw, l, t);
-    if (valid) {
-      HT* h = Ht + (int64_t)b * S + colH;
-#pragma unroll
-      for (int r = 0; r < 8; ++r) Store<HT>::store(h + (int64_t)(t + T * r) * rowH, v[r]);
-    }
-    __syncthreads();
-  }
-}
-
-template <int N>
-constexpr int reg_lines() { return N >= 512 ? 8 : 16; }
-
-template <int N>
-size_t reg_smem_bytes(int n2, int t1, int t2, bool with_plane) {
-  size_t b = sizeof(float2) * (N + colfft::smem_elems<N>(reg_lines<N>()));
-  if (with_plane) b += sizeof(float2) * n2 + sizeof(float) * t1 * t2;
-  return b;
-}
-
-template <int N, typename HT>
-size_t ypass_smem_bytes() {
-  return reg_smem_bytes<N>(0, 0, 0, false) + kYStages * sizeof(HT) * N * reg_lines<N>();
-}
-
-static bool reg_supported(int n) {
-  return n == 64 || n == 128 || n == 256 || n == 512 || n == 1024;
-}
-
-// ------------------------------------------------------------------ K4: z pass + epilogue
-// grid (ceil(n0*n1/R)); each CTA owns R consecutive (x', y') rows = R*n2 output voxels.
-// c2r of length n2 (even) via a complex inverse FFT of length m = n2/2:
-//   E[k] = X[k] + conj(X[m-k]),  O[k] = (X[k] - conj(X[m-k])) * exp(+2 pi i k / n2),
-//   z = IDFT_m(E + i O)  ->  x[2j] = Re z[j], x[2j+1] = Im z[j]
-// with the imaginary parts of X[0] and X[m] dropped, as numpy/pocketfft's c2r does.
-constexpr int kMaxV = 8;   // output voxels per thread
-
-// K4'' (FLC): c2r of the numerator and both statistics rows, then
-// norm_scores (tme/backends/npfftw_backend.py:537-587) in double precision with the
-// rotation's own n_obs = sum(rotated mask), and the strict-> update.
-// The FLC z pass transforms, for every rotation, the local mean (Hm), the local mean
-// square (Hm2) and the numerator (H) of a block of R rows as one batch of 3 R lines (one
-// set of barriers per rotation). The next rotation's rows are copied (cp.async, 16-byte
-// pieces of three contiguous ranges) into the second of two raw buffer sets while the
-// current rotation is transformed.
-template <typename HT, int M = 0>
-__global__ void __launch_bounds__(kThreads, 1)
-zpass_flc_kernel(const HT* __restrict__ Ht, const float2* __restrict__ Hm,
-                 const float2* __restrict__ Hm2, int B, int64_t rows, int n2, int hp, int R,
-                 LinePlan pm, const float2* __restrict__ tw2_g, float scale_t, float scale_m,
-                 const double* __restrict__ stats, double eps, int32_t first_index,
-                 float* __restrict__ state_max, int32_t* __restrict__ state_rot, int64_t S,
-                 const int32_t* __restrict__ first_dev) {
-  if (first_dev) first_index = *first_dev;
-  extern __shared__ float4 smem_raw[];
-  const int m = n2 / 2;
-  float2* tw2 = reinterpret_cast<float2*>(smem_raw);
-  // raw set q, part k (0 Hm, 1 Hm2, 2 H): R rows of hp values (float2 room for each)
-  float2* raw0 = tw2 + (n2 + 1) / 2 * 2;  // 16-byte aligned
-  const int64_t part = (int64_t)R * hp;
-  float2* buf = raw0 + 6 * part;
-  const int tid = threadIdx.x;
-  const int64_t row0 = (int64_t)blockIdx.x * R;
-  const int nrows = (int)min((int64_t)R, rows - row0);
-  for (int i = tid; i < n2; i += kThreads) tw2[i] = tw2_g[i];
-  const int nout = nrows * n2;
-  const int64_t vox0 = row0 * n2;
-  const int set = R * n2;  // floats between the three parts' outputs in buf
-  float best[kMaxV];
-  int32_t arg[kMaxV];
-#pragma unroll
-  for (int c = 0; c < kMaxV; ++c) { best[c] = -INFINITY; arg[c] = -1; }
-  const float* outv = reinterpret_cast<const float*>(buf);
-  auto issue = [&](int b) {
-    if (b < B) {
-      const uint32_t dst0 = (uint32_t)__cvta_generic_to_shared(raw0 + (b & 1) * 3 * part);
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const char* src = k == 0   ? reinterpret_cast<const char*>(Hm + (int64_t)b * S + row0 * hp)
-                          : k == 1 ? reinterpret_cast<const char*>(Hm2 + (int64_t)b * S + row0 * hp)
-                                   : reinterpret_cast<const char*>(Ht + (int64_t)b * S + row0 * hp);
-        const int nbytes = nrows * hp * (k == 2 ? (int)sizeof(HT) : (int)sizeof(float2));
-        const uint32_t dst = dst0 + (uint32_t)(k * part * (int64_t)sizeof(float2));
-        for (int o = tid * 16; o < nbytes; o += kThreads * 16)
-          tc::cp_async16(dst + (uint32_t)o, src + o, 16u);
-      }
-    }
-    cp_async_commit();
-  };
-  // line l = k R + r of buf: the even/odd-combined half spectrum of part k, row r
-  auto build = [&](const float2* src_f, const HT* src_h, int k) {
-    for (int e = tid; e < nrows * m; e += kThreads) {
-      const int r = e / m, j = e - r * m;
-      float2 a, c;
-      if (k == 2) {
-        const HT* xr = src_h + (int64_t)r * hp;
-        a = Store<HT>::load(xr + j);
-        c = Store<HT>::load(xr + (m - j));
-      } else {
-        const float2* xr = src_f + (int64_t)r * hp;
-        a = xr[j];
-        c = xr[m - j];
-      }
-      if (j == 0) { a.y = 0.f; c.y = 0.f; }
-      const float2 cc = fft::cconj(c);
-      const float2 E = fft::cadd(a, cc);
-      const float2 O = fft::cmul(fft::csub(a, cc), fft::cconj(tw2[j]));
-      buf[(int64_t)(k * R + r) * m + j] = make_float2(E.x - O.y, E.y + O.x);
-    }
-  };
-  issue(0);
-  for (int b = 0; b < B; ++b) {
-    // the other buffer set was last read by rotation b - 1, which ended with a barrier
-    issue(b + 1);
-    cp_async_wait<1>();
-    __syncthreads();  // rotation b's rows landed for every thread
-    const float2* rs = raw0 + (b & 1) * 3 * part;
-    build(rs, nullptr, 0);
-    build(rs + part, nullptr, 1);
-    build(nullptr, reinterpret_cast<const HT*>(rs + 2 * part), 2);
-    __syncthreads();
-    if constexpr (M > 0)
-      fft::fft_lines_ct<M, 1, kMaxE, false>(buf, 3 * R, M, 1, tw2, 2 * M, tid, kThreads);
-    else
-      fft::fft_lines<1, kMaxE, false>(buf, pm, 3 * R, m, 1, tw2, n2, tid, kThreads);
-    const double nobs = stats[b * 4 + 2];
-#pragma unroll
-    for (int c = 0; c < kMaxV; ++c) {
-      const int v = tid + c * kThreads;
-      if (v < nout) {
-        const double e1 = (double)outv[v] * (double)scale_m / nobs;
-        const double e2 = (double)outv[set + v] * (double)scale_m / nobs;
-        const double var = e2 - e1 * e1;
-        double sd = sqrt(var > 0 ? var : 0.0);
-        if (sd < eps) sd = 1.0;
-        const float sc = (float)((double)outv[2 * set + v] * (double)scale_t / (sd * nobs));
-        if (sc > best[c]) { best[c] = sc; arg[c] = first_index + b; }
-      }
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int c = 0; c < kMaxV; ++c) {
-    int v = tid + c * kThreads;
-    if (v < nout && arg[c] >= 0) {
-      int64_t g = vox0 + v;
-      if (best[c] > state_max[g]) { state_max[g] = best[c]; state_rot[g] = arg[c]; }
-    }
-  }
-}
-
+// ------------------------------------------------------------------ K4: z pass, four steps
 // K4' (four-step): c2r along axis 2 for m = n2/2 = M1*M2 (M2 a multiple of M1).
 // Thread (row, j) of a row's M1 threads builds Z[k] = E + iO for k = j + M1*k2 straight
 // from global memory (the half-length c2r pre-twiddle), runs an inverse DFT of size M2
@@ -903,13 +403,10 @@ struct Scan {
   float2* tw0 = nullptr;
   float2* tw1 = nullptr;
   float2* tw2 = nullptr;
-  LinePlan pm{};
-  bool reg0 = false, reg1 = false;  // register-resident column kernels for n0 / n1
   bool z4 = false;                  // four-step z pass for n2 / 2
-  GenConfig gen{};                  // passes over axes of any other length
+  GenConfig gen{};                  // line-FFT passes
+  HalfConfig hc{};                  // template, x and y passes over half2 spectra
   float4* gtw[3] = {};              // their twiddle tables
-  int R4f = 1;  // rows per block of the FLC z pass (three parts per row)
-  size_t smem4f = 0;
   cufftHandle fwd = 0, inv = 0, tfwd = 0, tinv = 0;
   bool have_fwd = false, have_tfwd = false;
   // CUDA-graph replay of a full launch group (see scan_set_graph)
@@ -935,7 +432,7 @@ struct Scan {
 // shared-memory y pass for lengths without a register kernel writes interleaved values,
 // so it is paired with them only.)
 static bool seg_layout(const Scan* s) {
-  return s->half && s->ztc && s->zcfg.eo && (s->ytc || s->reg1);
+  return s->half && s->ztc && s->zcfg.eo && (s->ytc || s->hc.reg1);
 }
 
 // Whether the warp-specialised tensor-core x pass runs every launch group: it can then read
@@ -956,23 +453,12 @@ static bool x_inner(const Scan* s) {
   return s->H2 && s->ytc && !s->yinplace && !y_stage1_tc(s) && x_writes_stage1(s);
 }
 
-// Which passes run over axes of any length (genpass.cuh): those without tensor cores whose
-// length has no kernel of its own. FLC takes the power-of-two kernels for both x and y or
-// for neither.
-static bool flc_reg(const Scan* s) { return s->reg0 && s->reg1; }
-static bool gen_x(const Scan* s) {
-  return s->d.score == TM_SCORE_FLC ? !flc_reg(s) : !s->xtc && !s->reg0;
-}
-static bool gen_y(const Scan* s) {
-  return s->d.score == TM_SCORE_FLC ? !flc_reg(s) : !s->ytc && !s->reg1;
-}
-static bool gen_z(const Scan* s) {
-  return s->d.score == TM_SCORE_FLC ? !flc_reg(s) : !(s->ztc && s->half) && !s->z4;
-}
-// H is k1-outer where all three run so, row-major otherwise.
+// H is k1-outer where the line-FFT passes run along all three axes, row-major otherwise; the
+// FLC statistics always are.
+static HLayout stat_layout(const Scan* s) { return h_k1_outer(s->n0, s->n1, s->hp); }
 static HLayout h_layout(const Scan* s) {
-  return gen_x(s) && gen_y(s) && gen_z(s) ? h_k1_outer(s->n0, s->n1, s->hp)
-                                          : h_row_major(s->n0, s->n1, s->hp);
+  const bool line_z = s->d.score == TM_SCORE_FLC || !s->z4;
+  return !s->half && !s->xtc && line_z ? stat_layout(s) : h_row_major(s->n0, s->n1, s->hp);
 }
 
 // Stage timing: record an event before a stage and accumulate after it.
@@ -992,42 +478,15 @@ struct StageTimer {
   }
 };
 
-// ---- z pass dispatch: compile-time half-lengths for the common sizes
-#define TM_DISPATCH_M(m, CALL)                                   \
-  switch (m) {                                                   \
-    case 32: { constexpr int MM = 32; CALL; } break;             \
-    case 50: { constexpr int MM = 50; CALL; } break;             \
-    case 64: { constexpr int MM = 64; CALL; } break;             \
-    case 80: { constexpr int MM = 80; CALL; } break;             \
-    case 100: { constexpr int MM = 100; CALL; } break;           \
-    case 128: { constexpr int MM = 128; CALL; } break;           \
-    case 160: { constexpr int MM = 160; CALL; } break;           \
-    default: { constexpr int MM = 0; CALL; } break;              \
-  }
-
+// ---- z pass dispatch
 template <typename HT>
-static void launch_zpass_flc(Scan* s, HT* H, int nb, int64_t rows, float out_scale,
-                             int32_t first, float* state_max, int32_t* state_rot,
-                             cudaStream_t st) {
+static int launch_zpass_flc(Scan* s, HT* H, int nb, float out_scale, int32_t first,
+                            float* state_max, int32_t* state_rot, cudaStream_t st) {
   const double* stats = s->stats_ws + (int64_t)nb * kStatChunks * 3;
-  if (gen_z(s)) {
-    gen_zpass_flc(s->gen, H, std::is_same<HT, __half2>::value, s->Hm, s->Hm2, nb, s->n0, s->n1,
-                  s->n2, s->hp, s->gtw[2], out_scale, out_scale, stats, 1.1920928955078125e-07,
-                  first, s->graph_first, state_max, state_rot, h_layout(s), st);
-    return;
-  }
-  dim3 g4f(ceil_div(rows, s->R4f));
-  TM_DISPATCH_M(s->n2 / 2, (zpass_flc_kernel<HT, MM><<<g4f, kThreads, s->smem4f, st>>>(
-                               H, s->Hm, s->Hm2, nb, rows, s->n2, s->hp, s->R4f, s->pm, s->tw2,
-                               out_scale, out_scale, stats, 1.1920928955078125e-07, first,
-                               state_max, state_rot, s->SH, s->graph_first)));
-}
-
-static void set_zpass_attrs(int m) {
-  TM_DISPATCH_M(m, (cudaFuncSetAttribute(zpass_flc_kernel<float2, MM>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max()),
-                    cudaFuncSetAttribute(zpass_flc_kernel<__half2, MM>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max())));
+  return gen_zpass_flc(s->gen, H, std::is_same<HT, __half2>::value, s->Hm, s->Hm2, nb, s->n0,
+                       s->n1, s->n2, s->hp, s->gtw[2], out_scale, out_scale, stats,
+                       1.1920928955078125e-07, first, s->graph_first, state_max, state_rot,
+                       h_layout(s), stat_layout(s), st);
 }
 
 #define TM_DISPATCH_4STEP(m, CALL)                                  \
@@ -1086,141 +545,58 @@ static void launch_zpass(Scan* s, HT* H, int nb, int64_t rows, float out_scale,
             h_layout(s), st);
 }
 
-// ---- launch helpers for the register-resident kernels
-template <int N>
-static void set_reg_attrs(size_t zy_smem) {
-  constexpr int W = reg_lines<N>();
-  const int sm = (int)reg_smem_bytes<N>(0, 0, 0, false);
-  cudaFuncSetAttribute(xpass_reg_kernel<N, W, float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max());
-  cudaFuncSetAttribute(xpass_reg_kernel<N, W, __half2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max());
-  cudaFuncSetAttribute(ypass_reg_kernel<N, W, float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max());
-  cudaFuncSetAttribute(ypass_reg_kernel<N, W, __half2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max());
-  cudaFuncSetAttribute(tmpl_zy_reg_kernel<N, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max());
-  cudaFuncSetAttribute(tmpl_zy_reg_kernel<N, W, __half2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max());
-  cudaFuncSetAttribute(xpass_flc_reg_kernel<N, W, float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max());
-  cudaFuncSetAttribute(xpass_flc_reg_kernel<N, W, __half2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin_max());
-}
-
-static void set_reg_attrs_n(int n, size_t zy_smem) {
-  switch (n) {
-    case 64: set_reg_attrs<64>(zy_smem); break;
-    case 128: set_reg_attrs<128>(zy_smem); break;
-    case 256: set_reg_attrs<256>(zy_smem); break;
-    case 512: set_reg_attrs<512>(zy_smem); break;
-    case 1024: set_reg_attrs<1024>(zy_smem); break;
-    default: break;
-  }
-}
-
-template <int N>
-static void launch_tmpl_reg(Scan* s, int nb, cudaStream_t st, const float* in = nullptr,
-                            float2* out = nullptr, bool half_g = false) {
-  constexpr int W = reg_lines<N>();
-  dim3 g(ceil_div(s->h2, W), s->t0, nb);
-  size_t smem = reg_smem_bytes<N>(s->n2, s->t1, s->t2, true);
-  if (half_g)
-    tmpl_zy_reg_kernel<N, W, __half2><<<g, N / 8 * W, smem, st>>>(
-        in ? in : s->rot_t, s->t0, s->t1, s->t2, s->n2, s->h2, s->tw1, s->tw2,
-        reinterpret_cast<__half2*>(out ? out : s->G));
-  else
-    tmpl_zy_reg_kernel<N, W><<<g, N / 8 * W, smem, st>>>(in ? in : s->rot_t, s->t0, s->t1, s->t2,
-                                                         s->n2, s->h2, s->tw1, s->tw2,
-                                                         out ? out : s->G);
-}
-
-template <int N, typename HT>
-static void launch_xpass_flc_reg(Scan* s, int nb, float hs, HT* H, cudaStream_t st) {
-  constexpr int W = reg_lines<N>();
-  dim3 g(ceil_div(s->h2, W), s->n1);
-  xpass_flc_reg_kernel<N, W, HT><<<g, N / 8 * W, reg_smem_bytes<N>(0, 0, 0, false), st>>>(
-      s->G, s->Gm, s->ft_target, s->ft_target2, nb, s->t0, s->n1, s->h2, s->tw0, hs, H, s->Hm,
-      s->Hm2, s->hp);
-}
-
-template <int N, typename HT>
-static void launch_xpass_reg(Scan* s, int nb, float hs, HT* H, cudaStream_t st) {
-  constexpr int W = reg_lines<N>();
-  dim3 g(ceil_div(s->h2, W), s->n1);
-  xpass_reg_kernel<N, W, HT><<<g, N / 8 * W, reg_smem_bytes<N>(0, 0, 0, false), st>>>(
-      s->G, s->ft_target, nb, s->t0, s->n1, s->h2, s->tw0, hs, H, s->hp);
-}
-
-template <int N, typename HT>
-static void launch_ypass_reg(Scan* s, int nb, HT* H, cudaStream_t st, bool seg = false) {
-  constexpr int W = reg_lines<N>();
-  dim3 g(ceil_div(s->h2, W), ceil_div(s->n0, kYPlanes), nb);
-  ypass_reg_kernel<N, W, HT><<<g, N / 8 * W, ypass_smem_bytes<N, HT>(), st>>>(
-      H, s->n0, s->h2, s->tw1, s->hp, seg ? 1 : 0);
-}
-
-#define TM_DISPATCH_N(n, CALL)      \
-  switch (n) {                      \
-    case 64: { constexpr int NN = 64; CALL; } break;    \
-    case 128: { constexpr int NN = 128; CALL; } break;  \
-    case 256: { constexpr int NN = 256; CALL; } break;  \
-    case 512: { constexpr int NN = 512; CALL; } break;  \
-    case 1024: { constexpr int NN = 1024; CALL; } break; \
-    default: break;                 \
-  }
-
 template <typename HT>
 static int launch_template_x_y(Scan* s, int nb, float hs, HT* H, StageTimer& tmr,
                                cudaStream_t stream) {
   const bool flc = s->d.score == TM_SCORE_FLC;
   // the warp-specialised tensor-core x pass reads the template spectra G as FP16 (it
   // rounds them to FP16 for its MMAs anyway), so the template pass writes them so
-  const bool half_g = s->reg1 && x_writes_stage1(s);
+  const bool half_g = s->half && s->hc.reg1 && x_writes_stage1(s);
+  const HLayout hl = h_layout(s), sl = stat_layout(s);
+  constexpr bool half = std::is_same<HT, __half2>::value;
   tmr.begin();
-  const HLayout hl = h_layout(s);
-  const bool half = std::is_same<HT, __half2>::value;
-  if (gen_y(s) && !half_g) {
+  if constexpr (half)
+    TM_TRY(half_template(s->hc, s->rot_t, nb, s->t0, s->t1, s->t2, s->n1, s->n2, s->h2, s->tw1,
+                         s->tw2, s->G, half_g, stream));
+  else
     TM_TRY(gen_template(s->gen, s->rot_t, nb, s->t0, s->t1, s->t2, s->n1, s->n2, s->h2, s->hp,
                         s->gtw[1], s->tw2, s->G, stream));
-    if (flc)
-      TM_TRY(gen_template(s->gen, s->rot_m, nb, s->t0, s->t1, s->t2, s->n1, s->n2, s->h2, s->hp,
-                          s->gtw[1], s->tw2, s->Gm, stream));
-  } else {
-    TM_DISPATCH_N(s->n1, (launch_tmpl_reg<NN>(s, nb, stream, nullptr, nullptr, half_g)));
-    if (flc) TM_DISPATCH_N(s->n1, (launch_tmpl_reg<NN>(s, nb, stream, s->rot_m, s->Gm)));
-  }
-  TM_TRY(check_launch("template pass"));
+  if (flc)
+    TM_TRY(gen_template(s->gen, s->rot_m, nb, s->t0, s->t1, s->t2, s->n1, s->n2, s->h2, s->hp,
+                        s->gtw[1], s->tw2, s->Gm, stream));
   tmr.end(TM_STAGE_TEMPLATE);
   tmr.begin();
-  if (flc && gen_x(s)) {
-    TM_TRY(gen_xpass_flc(s->gen, s->G, s->Gm, s->ft_target, s->ft_target2, nb, s->t0, s->n1,
-                         s->h2, s->hp, s->gtw[0], hs, H, half, s->Hm, s->Hm2, hl, stream));
-  } else if (flc) {
-    TM_DISPATCH_N(s->n0, (launch_xpass_flc_reg<NN, HT>(s, nb, hs, H, stream)));
-  } else if (gen_x(s)) {
-    TM_TRY(gen_xpass(s->gen, s->G, s->ft_target, nb, s->t0, s->n1, s->h2, s->hp, s->gtw[0], hs, H,
-                     half, hl, stream));
-  } else if (s->xtc) {
+  if (flc)
+    TM_TRY(gen_xstat(s->gen, s->Gm, s->ft_target, s->ft_target2, nb, s->t0, s->n1, s->h2, s->hp,
+                     s->gtw[0], hs, s->Hm, s->Hm2, sl, stream));
+  if (s->xtc) {
     const bool s1 = y_stage1_tc(s);
     TM_TRY(xcorr_tc_run(s->xcfg, s->G, s->ctarget, nb, s->t0, s->n0, s->n1, s->h2, s->hp, hs,
-                        H, std::is_same<HT, __half2>::value, s->tc_err, stream,
-                        s->wait_iters, s1, s1 ? s->n1 / 16 : 0, half_g, x_inner(s)));
+                        H, half, s->tc_err, stream, s->wait_iters, s1, s1 ? s->n1 / 16 : 0,
+                        half_g, x_inner(s)));
+  } else if constexpr (half) {
+    TM_TRY(half_xpass(s->hc, s->G, s->ft_target, nb, s->t0, s->n0, s->n1, s->h2, s->hp, s->tw0,
+                      hs, H, flc, stream));
   } else {
-    TM_DISPATCH_N(s->n0, (launch_xpass_reg<NN, HT>(s, nb, hs, H, stream)));
+    TM_TRY(gen_xpass(s->gen, s->G, s->ft_target, nb, s->t0, s->n1, s->h2, s->hp, s->gtw[0], hs, H,
+                     hl, stream));
   }
   TM_TRY(check_launch("x pass"));
   tmr.end(TM_STAGE_XPASS);
   tmr.begin();
-  if (s->ytc && std::is_same<HT, __half2>::value) {
-    TM_TRY(ypass_tc_run(s->ycfg, H, nb, s->n0, s->hp, s->h2, s->ytable, s->wait_iters, s->tc_err,
-                        stream, seg_layout(s), y_stage1_tc(s), x_inner(s) ? s->H2 : nullptr,
-                        x_inner(s)));
-  } else if (gen_y(s)) {
-    TM_TRY(gen_ypass(s->gen, H, half, nb, s->n0, s->hp, s->gtw[1], hl, stream));
-    if (flc) {
-      TM_TRY(gen_ypass(s->gen, s->Hm, false, nb, s->n0, s->hp, s->gtw[1], hl, stream));
-      TM_TRY(gen_ypass(s->gen, s->Hm2, false, nb, s->n0, s->hp, s->gtw[1], hl, stream));
-    }
+  if (flc) {
+    TM_TRY(gen_ypass(s->gen, s->Hm, nb, s->n0, s->hp, s->gtw[1], sl, stream));
+    TM_TRY(gen_ypass(s->gen, s->Hm2, nb, s->n0, s->hp, s->gtw[1], sl, stream));
+  }
+  if constexpr (half) {
+    if (s->ytc)
+      TM_TRY(ypass_tc_run(s->ycfg, H, nb, s->n0, s->hp, s->h2, s->ytable, s->wait_iters, s->tc_err,
+                          stream, seg_layout(s), y_stage1_tc(s), x_inner(s) ? s->H2 : nullptr,
+                          x_inner(s)));
+    else
+      TM_TRY(half_ypass(s->hc, H, nb, s->n0, s->n1, s->h2, s->hp, s->tw1, seg_layout(s), stream));
   } else {
-    TM_DISPATCH_N(s->n1, (launch_ypass_reg<NN, HT>(s, nb, H, stream, seg_layout(s))));
-    if (flc) {
-      TM_DISPATCH_N(s->n1, (launch_ypass_reg<NN, float2>(s, nb, s->Hm, stream)));
-      TM_DISPATCH_N(s->n1, (launch_ypass_reg<NN, float2>(s, nb, s->Hm2, stream)));
-    }
+    TM_TRY(gen_ypass(s->gen, H, nb, s->n0, s->hp, s->gtw[1], hl, stream));
   }
   TM_TRY(check_launch("y pass"));
   tmr.end(TM_STAGE_YPASS);
@@ -1304,9 +680,8 @@ int scan_create(const tm_scan_desc* desc, Scan** out, bool any_length) {
     s->gen = gen_config(s->n0, s->n1, s->n2, s->t0, s->t1, s->t2, s->hp,
                         d.score == TM_SCORE_FLC, s->half);
     bool ok = s->gen.ok && line_supported(s->n0) && line_supported(s->n1) && (s->n2 % 2 == 0) &&
-              line_supported(s->n2 / 2) && s->n0 <= kTile && s->n1 <= kTile &&
-              s->n2 <= kThreads * kMaxV &&
-              (d.score != TM_SCORE_FLC || (reg_supported(s->n0) && reg_supported(s->n1)));
+              line_supported(s->n2 / 2) && s->n2 <= kMaxLine &&
+              (d.score != TM_SCORE_FLC || (flc_supported(s->n0) && flc_supported(s->n1)));
     if (!ok) {
       set_error("scan_create: fused path does not support shape (%d,%d,%d) / score %d",
                 s->n0, s->n1, s->n2, d.score);
@@ -1456,34 +831,17 @@ int scan_create(const tm_scan_desc* desc, Scan** out, bool any_length) {
     cudaMemcpy(s->tw1, t1v.data(), sizeof(float2) * s->n1, cudaMemcpyHostToDevice);
     e = cudaMemcpy(s->tw2, t2v.data(), sizeof(float2) * s->n2, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) { int st = cuda_status(e, "scan_create: twiddles"); destroy(s); return st; }
-    s->pm = make_line_plan(s->n2 / 2);
-    s->R4f = std::max(1, std::min(kTile / std::max(1, 3 * (s->n2 / 2)),
-                                  (kThreads * kMaxV) / s->n2));
     // what the template pass may hold of a template plane
     const size_t plane = sizeof(float2) * (s->n1 + s->n2 +
-                                           (size_t)s->n1 * std::max(1, std::min(s->h2, kTile / s->n1))) +
+                                           (size_t)s->n1 * std::max(1, std::min(s->h2, kMaxLine / s->n1))) +
                          sizeof(float) * s->t1 * s->t2;
-    // FLC z pass: twiddles, two raw sets of three parts, the c2r buffer of 3 R4f lines
-    s->smem4f = sizeof(float2) * ((s->n2 + 1) / 2 * 2 + 6 * (size_t)s->R4f * s->hp +
-                                  3 * (size_t)s->R4f * (s->n2 / 2));
-    const size_t mx = std::max(plane, d.score == TM_SCORE_FLC ? s->smem4f : 0);
-    if (mx > 200 * 1024 && !any_length) {
-      set_error("scan_create: shared-memory tile of %zu bytes exceeds the limit", mx);
+    if (plane > 200 * 1024 && !any_length) {
+      set_error("scan_create: shared-memory tile of %zu bytes exceeds the limit", plane);
       destroy(s);
       return TM_E_UNSUPPORTED;
     }
-    set_zpass_attrs(s->n2 / 2);
     set_zpass4_attrs(s->n2 / 2);
-    s->reg0 = reg_supported(s->n0) && !any_length;
-    s->reg1 = reg_supported(s->n1) && !any_length;
     s->z4 = s->n2 % 2 == 0 && zpass4_supported(s->n2 / 2) && !any_length;
-    size_t zy = 0;
-    if (s->reg1) {
-      TM_DISPATCH_N(s->n1, (zy = reg_smem_bytes<NN>(s->n2, s->t1, s->t2, true)));
-      if (zy > 200 * 1024) s->reg1 = false;
-    }
-    if (s->reg0) set_reg_attrs_n(s->n0, 0);
-    if (s->reg1) set_reg_attrs_n(s->n1, zy);
     {
       const linefft::Plan* plans[3] = {&s->gen.x.plan, &s->gen.y.plan, &s->gen.z.plan};
       for (int a = 0; a < 3; ++a) {
@@ -1492,7 +850,11 @@ int scan_create(const tm_scan_desc* desc, Scan** out, bool any_length) {
         e = cudaMemcpy(s->gtw[a], t.data(), sizeof(float2) * t.size(), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) { int st = cuda_status(e, "scan_create: twiddles"); destroy(s); return st; }
       }
-      const int st = gen_prepare(s->gen, d.score == TM_SCORE_FLC, s->half);
+      int st = gen_prepare(s->gen, d.score == TM_SCORE_FLC, s->half);
+      if (st == TM_OK && s->half) {
+        s->hc = half_config(s->n0, s->n1, s->n2, s->h2, s->t1, s->t2);
+        st = half_prepare(s->hc, s->n0, s->n1);
+      }
       if (st != TM_OK) { destroy(s); return st; }
     }
   }
@@ -1849,7 +1211,7 @@ static int launch_group(Scan* s, int nb, double hs, float out_scale, int32_t fir
     TM_TRY(launch_template_x_y<__half2>(s, nb, (float)hs, H, tmr, stream));
     tmr.begin();
     if (s->d.score == TM_SCORE_FLC)
-      launch_zpass_flc<__half2>(s, H, nb, rows, out_scale, first, state_max, state_rot, stream);
+      TM_TRY(launch_zpass_flc<__half2>(s, H, nb, out_scale, first, state_max, state_rot, stream));
     else
       launch_zpass<__half2>(s, x_inner(s) ? static_cast<__half2*>(s->H2) : H, nb, rows,
                             out_scale, first, state_max, state_rot, stream);
@@ -1860,7 +1222,7 @@ static int launch_group(Scan* s, int nb, double hs, float out_scale, int32_t fir
     TM_TRY(launch_template_x_y<float2>(s, nb, (float)hs, H, tmr, stream));
     tmr.begin();
     if (s->d.score == TM_SCORE_FLC)
-      launch_zpass_flc<float2>(s, H, nb, rows, out_scale, first, state_max, state_rot, stream);
+      TM_TRY(launch_zpass_flc<float2>(s, H, nb, out_scale, first, state_max, state_rot, stream));
     else
       launch_zpass<float2>(s, H, nb, rows, out_scale, first, state_max, state_rot, stream);
     TM_TRY(check_launch("z pass"));

@@ -5,13 +5,11 @@
 #include <cstdint>
 
 #include "pytme_b200.h"
-#include "fft_smem.cuh"
 
 namespace tmb {
 
 struct Scan;
 
-fft::LinePlan make_line_plan(int n);
 // any_length: FP32 plans whose axes or score the fused path of tm_scan_create refuses
 int scan_create(const tm_scan_desc* desc, Scan** out, bool any_length = false);
 int scan_destroy(Scan* s);

@@ -14,7 +14,7 @@ from oracle import tm_oracle as O
 TOL = 1e-5
 
 SHAPES = [
-    (60, 50, 40), (77, 91, 39), (66, 49, 45), (61, 47, 37), (126, 63, 52), (112, 130, 27),
+    (64, 128, 64), (13, 16, 512), (60, 50, 40), (77, 91, 39), (66, 49, 45), (61, 47, 37), (126, 63, 52), (112, 130, 27),
     (625, 16, 18), (1050, 24, 26), (24, 1100, 22), (16, 18, 1250), (2048, 16, 15),
 ]
 
