@@ -3,6 +3,8 @@
 // scipy.ndimage.maximum_filter with mode="constant", cval=0) and the greedy
 // minimum-distance filter of find_candidate_indices
 // (tme/external/bindings.cpp:85-126).
+#include <algorithm>
+
 #include "common.cuh"
 #include "peaks.cuh"
 
@@ -40,10 +42,104 @@ __global__ void peak_mask_kernel(const float* __restrict__ f, const float* __res
     mask[v] = f[v] == s[v];
 }
 
-int max_filter_peaks(const float* scores, int n0, int n1, int n2, int size, float* tmp_a,
-                     float* tmp_b, uint8_t* mask, cudaStream_t stream) {
-  TM_REQUIRE(scores && tmp_a && tmp_b && mask, "max_filter_peaks: null pointer");
-  TM_REQUIRE(n0 > 0 && n1 > 0 && n2 > 0 && size >= 1, "max_filter_peaks: bad shape/size");
+// The same running maximum in a few comparisons an element, whatever the window: HBM traffic
+// bounds both kernels (512 x 512 x 200, size 24: the loop over the window took 0.68 ms an axis).
+// A padded axis (size / 2 zeros before, the rest of size - 1 after) has
+// out[i] = max padded[i .. i + size - 1].
+constexpr int kFilterThreads = 128;
+constexpr int kMaxWindow = 192;     // columns of the strided kernel kept in shared memory
+constexpr int kRowFloats = 12288;   // padded rows of the contiguous kernel
+
+// Contiguous axis: whole padded rows in shared memory, windows doubled until two of them cover
+// `size` (log2 size steps between two buffers). A window that runs into the next row is never
+// read, so the steps ignore rows.
+__global__ void __launch_bounds__(256)
+max_filter_rows_kernel(const float* __restrict__ in, float* __restrict__ out, int64_t rows, int n,
+                       int size, int per) {
+  extern __shared__ float buf[];
+  const int p = n + size - 1, lo = size / 2;
+  const int64_t row0 = (int64_t)blockIdx.x * per;
+  const int nr = (int)min((int64_t)per, rows - row0), total = nr * p;
+  float *a = buf, *b = buf + per * p;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int r = warp; r < nr; r += 8) {
+    const float* src = in + (row0 + r) * n;
+    for (int i = lane; i < p; i += 32)
+      a[r * p + i] = i >= lo && i < lo + n ? src[i - lo] : 0.f;
+  }
+  __syncthreads();
+  int have = 1;
+  for (; 2 * have <= size; have *= 2) {
+    for (int i = threadIdx.x; i < total; i += 256)
+      b[i] = i + have < total ? fmaxf(a[i], a[i + have]) : a[i];
+    __syncthreads();
+    float* t = a;
+    a = b;
+    b = t;
+  }
+  for (int r = warp; r < nr; r += 8) {
+    float* dst = out + (row0 + r) * n;
+    const float* m = a + r * p;
+    for (int i = lane; i < n; i += 32) dst[i] = fmaxf(m[i], m[i + size - have]);
+  }
+}
+
+// Strided axis: a thread walks one column in blocks of `size` padded values; out of the suffix
+// maxima of a block (kept in shared memory) and the running prefix maximum of the next it has
+// every window (van Herk, "A fast algorithm for local minimum and maximum filters", Pattern
+// Recognition Letters 13, 1992). MASK: compare with the scores instead of storing the maxima.
+template <bool MASK>
+__global__ void __launch_bounds__(kFilterThreads)
+max_filter_columns_kernel(const float* __restrict__ in, float* __restrict__ out,
+                          const float* __restrict__ scores, uint8_t* __restrict__ mask,
+                          int64_t columns, int len, int64_t stride, int size) {
+  extern __shared__ float buf[];
+  float* s = buf + threadIdx.x;  // s[j * kFilterThreads]
+  const int64_t c = (int64_t)blockIdx.x * kFilterThreads + threadIdx.x;
+  if (c >= columns) return;
+  const int64_t base = c / stride * stride * len + c % stride;
+  const float* src = in + base;
+  const int lo = size / 2;
+  auto value = [&](int i) {  // padded value i
+    const int x = i - lo;
+    return x >= 0 && x < len ? __ldg(src + x * stride) : 0.f;
+  };
+  for (int j = 0; j < size; ++j) s[j * kFilterThreads] = value(j);
+  for (int i0 = 0; i0 < len; i0 += size) {
+    float m = s[(size - 1) * kFilterThreads];
+    for (int j = size - 2; j >= 0; --j) {
+      m = fmaxf(m, s[j * kFilterThreads]);
+      s[j * kFilterThreads] = m;
+    }
+    float pre = -INFINITY;
+    for (int j0 = 0; j0 < size; j0 += 8) {
+      float x[8], f[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int j = j0 + k;
+        x[k] = j < size ? value(i0 + size + j) : 0.f;
+        if (MASK) f[k] = j < size && i0 + j < len ? __ldg(scores + base + (i0 + j) * stride) : 0.f;
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int j = j0 + k;
+        if (j < size) {
+          const float o = fmaxf(s[j * kFilterThreads], pre);
+          if (i0 + j < len) {
+            if (MASK) mask[base + (i0 + j) * stride] = o == f[k];
+            else out[base + (i0 + j) * stride] = o;
+          }
+          s[j * kFilterThreads] = x[k];
+          pre = fmaxf(pre, x[k]);
+        }
+      }
+    }
+  }
+}
+
+// Windows and rows beyond the shared memory of the fast kernels: one loop per voxel.
+static int max_filter_peaks_long(const float* scores, int n0, int n1, int n2, int size,
+                                 float* tmp_a, float* tmp_b, uint8_t* mask, cudaStream_t stream) {
   const int64_t n = (int64_t)n0 * n1 * n2;
   int64_t blocks = ceil_div(n, 256);
   if (blocks > 148 * 32) blocks = 148 * 32;
@@ -54,63 +150,167 @@ int max_filter_peaks(const float* scores, int n0, int n1, int n2, int size, floa
   return check_launch("max_filter_peaks");
 }
 
-// Greedy filter: point 0 is kept; point i is kept when, for every kept point j,
-// floor(sqrt(|c_i - c_j|^2)) > min_distance — the integer arithmetic of the int64
-// overload the reference's peak callers reach. One CTA walks the points in order;
-// the kept coordinates live in `kept` (shared memory when they fit, else the
-// caller's workspace), and every thread tests a strided share of them.
-constexpr int kNmsThreads = 1024;
+int max_filter_peaks(const float* scores, int n0, int n1, int n2, int size, float* tmp_a,
+                     float* tmp_b, uint8_t* mask, cudaStream_t stream) {
+  TM_REQUIRE(scores && tmp_a && tmp_b && mask, "max_filter_peaks: null pointer");
+  TM_REQUIRE(n0 > 0 && n1 > 0 && n2 > 0 && size >= 1, "max_filter_peaks: bad shape/size");
+  if (size > kMaxWindow || n2 > kRowFloats - size)
+    return max_filter_peaks_long(scores, n0, n1, n2, size, tmp_a, tmp_b, mask, stream);
+  const int p = n2 + size - 1;
+  const int per = std::max(1, 3072 / p);
+  const int64_t rows = (int64_t)n0 * n1;
+  const size_t smem_r = 2 * sizeof(float) * (size_t)per * p;
+  const size_t smem_c = sizeof(float) * (size_t)size * kFilterThreads;
+  const int most = 2 * sizeof(float) * kRowFloats;
+  TM_TRY(cuda_status(cudaFuncSetAttribute(max_filter_rows_kernel,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, most),
+                     "max_filter_peaks: shared memory"));
+  TM_TRY(cuda_status(cudaFuncSetAttribute(max_filter_columns_kernel<false>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, most),
+                     "max_filter_peaks: shared memory"));
+  TM_TRY(cuda_status(cudaFuncSetAttribute(max_filter_columns_kernel<true>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, most),
+                     "max_filter_peaks: shared memory"));
+  max_filter_rows_kernel<<<(unsigned)ceil_div(rows, per), 256, smem_r, stream>>>(
+      scores, tmp_a, rows, n2, size, per);
+  const int64_t cy = (int64_t)n0 * n2, cx = (int64_t)n1 * n2;
+  max_filter_columns_kernel<false><<<(unsigned)ceil_div(cy, kFilterThreads), kFilterThreads,
+                                     smem_c, stream>>>(tmp_a, tmp_b, nullptr, nullptr, cy, n1, n2,
+                                                       size);
+  max_filter_columns_kernel<true><<<(unsigned)ceil_div(cx, kFilterThreads), kFilterThreads,
+                                    smem_c, stream>>>(tmp_b, nullptr, scores, mask, cx, n0, cx,
+                                                      size);
+  return check_launch("max_filter_peaks");
+}
 
-__device__ __forceinline__ bool too_close(int64_t dx, int64_t dy, int64_t dz, int64_t md) {
-  // floor(sqrt(d2)) <= md is never true for md < 0 (every point is kept) and always
-  // true once (md + 1)^2 exceeds any squared distance of 32-bit coordinates
-  if (md < 0) return false;
-  if (md >= (int64_t)3037000499LL) return true;
-  int64_t d2 = dx * dx + dy * dy + dz * dz;
-  // floor(sqrt(d2)) <= md  <=>  d2 < (md + 1)^2 for non-negative integers
-  return d2 < (md + 1) * (md + 1);
+// Greedy filter: point 0 is kept; point i is kept when, for every kept point j,
+// floor(sqrt(|c_i - c_j|^2)) > min_distance, the integer arithmetic of the int64
+// overload the reference's peak callers reach. One CTA takes the points in order, 64 at a
+// time: all threads test the 64 against the points kept so far and against each other, then
+// one warp settles the 64 among themselves (a point falls when an earlier kept one is too
+// close, and stands when all such are settled and fell). A pass a point took 1.7 ms for 3000
+// points. The kept coordinates live in `kept` (shared memory when they fit, else the caller's
+// workspace), as 32-bit values when all coordinates are below 2^30 in size.
+constexpr int kNmsThreads = 1024;
+constexpr int kNmsChunk = 64;
+
+struct FarTest {
+  int64_t md, lim;  // floor(sqrt(d2)) <= md  <=>  d2 < (md + 1)^2 = lim
+  int md32;
+  bool all, none;   // every / no pair is too close
+  __device__ explicit FarTest(int64_t m)
+      : md(m), lim((m + 1) * (m + 1)), md32((int)min(m, (int64_t)0x7fffffff)),
+        all(m >= (int64_t)3037000499LL), none(m < 0) {}
+  __device__ __forceinline__ bool close(int4 a, int4 b) const {
+    const int dx = abs(a.x - b.x), dy = abs(a.y - b.y), dz = abs(a.z - b.z);
+    if (max(max(dx, dy), dz) > md32) return false;
+    return (int64_t)dx * dx + (int64_t)dy * dy + (int64_t)dz * dz < lim;
+  }
+  __device__ __forceinline__ bool close(const int64_t* a, const int64_t* b) const {
+    const int64_t dx = a[0] - b[0], dy = a[1] - b[1], dz = a[2] - b[2];
+    return dx * dx + dy * dy + dz * dz < lim;
+  }
+};
+
+template <typename T>
+struct KeptPoint;
+template <>
+struct KeptPoint<int4> {
+  static __device__ __forceinline__ const int4& at(const void* p, int j) {
+    return static_cast<const int4*>(p)[j];
+  }
+  static __device__ __forceinline__ void load(const int64_t* c, void* p, int j) {
+    static_cast<int4*>(p)[j] = make_int4((int)c[0], (int)c[1], (int)c[2], 0);
+  }
+};
+template <>
+struct KeptPoint<int64_t> {
+  static __device__ __forceinline__ const int64_t* at(const void* p, int j) {
+    return static_cast<const int64_t*>(p) + 3 * (int64_t)j;
+  }
+  static __device__ __forceinline__ void load(const int64_t* c, void* p, int j) {
+    int64_t* d = static_cast<int64_t*>(p) + 3 * (int64_t)j;
+    d[0] = c[0];
+    d[1] = c[1];
+    d[2] = c[2];
+  }
+};
+
+template <typename T>
+__device__ __forceinline__ void greedy_chunks(const int64_t* __restrict__ coords, int n,
+                                              const FarTest& far, int32_t* __restrict__ out_idx,
+                                              int32_t* __restrict__ out_count, void* kept,
+                                              void* chunk, unsigned long long* conf, int* count) {
+  using K = KeptPoint<T>;
+  __shared__ unsigned fell[2];
+  const int tid = threadIdx.x, pt = tid % kNmsChunk, group = tid / kNmsChunk;
+  constexpr int GROUPS = kNmsThreads / kNmsChunk;
+  for (int base = 0; base < n; base += kNmsChunk) {
+    const int m = min(kNmsChunk, n - base);
+    if (tid < m) K::load(coords + 3 * (int64_t)(base + tid), chunk, tid);
+    if (tid < kNmsChunk) conf[tid] = 0ull;
+    if (tid < 2) fell[tid] = 0u;
+    __syncthreads();
+    if (pt < m && !far.none) {
+      const int c = *count;
+      bool hit = far.all && c > 0;
+      for (int j = group; j < c && !hit; j += GROUPS)
+        hit = far.close(K::at(chunk, pt), K::at(kept, j));
+      if (hit) atomicOr(&fell[pt / 32], 1u << (pt % 32));
+      unsigned long long bits = 0ull;
+      for (int q = group; q < pt; q += GROUPS)
+        if (far.all || far.close(K::at(chunk, pt), K::at(chunk, q))) bits |= 1ull << q;
+      if (bits) atomicOr(&conf[pt], bits);
+    }
+    __syncthreads();
+    if (tid < 32) {
+      const unsigned long long live = m == 64 ? ~0ull : (1ull << m) - 1ull;
+      unsigned long long out = ((unsigned long long)fell[1] << 32 | fell[0]) | ~live, in = 0ull;
+      const unsigned long long c0 = conf[tid], c1 = conf[tid + 32];
+      while ((in | out) != ~0ull) {
+        const bool u0 = !((in | out) >> tid & 1), u1 = !((in | out) >> (tid + 32) & 1);
+        const bool f0 = u0 && (c0 & in), f1 = u1 && (c1 & in);
+        const bool k0 = u0 && !(c0 & ~out), k1 = u1 && !(c1 & ~out);
+        out |= (unsigned long long)__ballot_sync(0xffffffffu, f1) << 32 |
+               __ballot_sync(0xffffffffu, f0);
+        in |= (unsigned long long)__ballot_sync(0xffffffffu, k1) << 32 |
+              __ballot_sync(0xffffffffu, k0);
+      }
+      const int c = *count;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int q = tid + 32 * h;
+        if (in >> q & 1) {
+          const int at = c + __popcll(in & ((1ull << q) - 1ull));
+          K::load(coords + 3 * (int64_t)(base + q), kept, at);
+          out_idx[at] = base + q;
+        }
+      }
+      __syncwarp();
+      if (tid == 0) *count = c + __popcll(in);
+    }
+    __syncthreads();
+  }
+  if (tid == 0) *out_count = *count;
 }
 
 __global__ void __launch_bounds__(kNmsThreads)
 greedy_nms_kernel(const int64_t* __restrict__ coords, int n, int64_t min_distance,
                   int32_t* __restrict__ out_idx, int32_t* __restrict__ out_count,
                   int64_t* __restrict__ kept_global, int smem_cap) {
-  extern __shared__ int64_t kept_smem[];
-  int64_t* kept = (n <= smem_cap) ? kept_smem : kept_global;
+  extern __shared__ __align__(16) int64_t kept_smem[];
+  void* kept = (n <= smem_cap) ? kept_smem : kept_global;
+  __shared__ __align__(16) int64_t chunk[3 * kNmsChunk];
+  __shared__ unsigned long long conf[kNmsChunk];
   __shared__ int count;
-  if (threadIdx.x == 0) {
-    count = 0;
-    if (n > 0) {
-      kept[0] = coords[0];
-      kept[1] = coords[1];
-      kept[2] = coords[2];
-      out_idx[0] = 0;
-      count = 1;
-    }
-  }
-  __syncthreads();
-  for (int i = 1; i < n; ++i) {
-    const int64_t x = coords[3 * (int64_t)i], y = coords[3 * (int64_t)i + 1],
-                  z = coords[3 * (int64_t)i + 2];
-    const int c = count;
-    int reject = 0;
-    for (int j = threadIdx.x; j < c; j += blockDim.x) {
-      if (too_close(x - kept[3 * j], y - kept[3 * j + 1], z - kept[3 * j + 2], min_distance)) {
-        reject = 1;
-        break;
-      }
-    }
-    reject = __syncthreads_or(reject);
-    if (!reject && threadIdx.x == 0) {
-      kept[3 * c] = x;
-      kept[3 * c + 1] = y;
-      kept[3 * c + 2] = z;
-      out_idx[c] = i;
-      count = c + 1;
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *out_count = count;
+  if (threadIdx.x == 0) count = 0;
+  bool wide = reinterpret_cast<uintptr_t>(kept) % 16 != 0;
+  for (int64_t i = threadIdx.x; i < 3 * (int64_t)n; i += kNmsThreads)
+    wide |= coords[i] >= (1LL << 30) || coords[i] <= -(1LL << 30);
+  wide = __syncthreads_or(wide);
+  const FarTest far(min_distance);
+  if (wide) greedy_chunks<int64_t>(coords, n, far, out_idx, out_count, kept, chunk, conf, &count);
+  else greedy_chunks<int4>(coords, n, far, out_idx, out_count, kept, chunk, conf, &count);
 }
 
 int64_t nms_workspace_bytes(int n) { return (int64_t)(n > 0 ? n : 1) * 3 * sizeof(int64_t); }
@@ -125,6 +325,9 @@ int greedy_nms(const int64_t* coords, int n, int64_t min_distance, int32_t* out_
              "greedy_nms: %d points need a workspace of %lld bytes", n,
              (long long)nms_workspace_bytes(n));
   const size_t smem = (size_t)(n <= smem_cap ? (n > 0 ? n : 1) : 1) * 3 * sizeof(int64_t);
+  TM_TRY(cuda_status(cudaFuncSetAttribute(greedy_nms_kernel,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024),
+                     "greedy_nms: shared memory"));
   greedy_nms_kernel<<<1, kNmsThreads, smem, stream>>>(coords, n, min_distance, out_idx,
                                                      out_count,
                                                      static_cast<int64_t*>(workspace), smem_cap);

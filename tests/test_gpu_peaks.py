@@ -1,0 +1,68 @@
+"""Box maximum filter and greedy distance filter at the edges of their kernels: window sizes
+around powers of two, windows larger than an axis, the sizes where the long-window loop takes
+over; chunks of 64 points, points beyond shared memory and beyond 32-bit coordinates. Both are
+exact."""
+import numpy as np
+import pytest
+
+from oracle import tm_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("shape,size", [
+    ((40, 33, 50), 1), ((40, 33, 50), 2), ((41, 30, 37), 3), ((64, 64, 64), 8), ((70, 45, 61), 24),
+    ((30, 90, 64), 31), ((20, 21, 300), 33), ((5, 6, 7), 16), ((1, 9, 2), 5), ((24, 18, 11), 192),
+    ((24, 18, 11), 193), ((3, 2, 12200), 100)])
+def test_max_filter_peaks_match_scipy(shape, size):
+    from scipy.ndimage import maximum_filter
+
+    from pytme_b200.peaks import max_filter_candidates, max_filter_coordinates
+
+    rng = np.random.default_rng(size + sum(shape))
+    for s in (rng.normal(size=shape), rng.integers(-3, 4, shape), -1.0 - rng.random(shape),
+              np.where(rng.random(shape) < 0.5, -np.inf, rng.normal(size=shape))):
+        s = s.astype(np.float32)
+        want = np.argwhere(maximum_filter(s, size=size, mode="constant") == s)
+        assert np.array_equal(max_filter_coordinates(s, size), want)
+        coords, vals = max_filter_candidates(s, size)
+        assert np.array_equal(coords, want) and np.array_equal(vals, s[tuple(want.T)])
+
+
+def test_max_filter_peaks_skip_nan():
+    """A NaN is no peak and hides none."""
+    from scipy.ndimage import maximum_filter
+
+    from pytme_b200.peaks import max_filter_coordinates
+
+    rng = np.random.default_rng(4)
+    s = rng.normal(size=(30, 28, 40)).astype(np.float32)
+    hole = rng.random(s.shape) < 0.05
+    low = np.where(hole, -np.inf, s).astype(np.float32)
+    want = (maximum_filter(low, size=7, mode="constant") == low) & ~hole
+    got = max_filter_coordinates(np.where(hole, np.nan, s).astype(np.float32), 7)
+    assert np.array_equal(got, np.argwhere(want))
+
+
+@pytest.mark.parametrize("n", [1, 2, 63, 64, 65, 129, 2048, 2049, 4000])
+@pytest.mark.parametrize("span,md", [(60, 7), (400, 30), (8, 3), (10 ** 5, 2 * 10 ** 4), (50, 0)])
+def test_greedy_filter_matches_oracle(n, span, md):
+    from pytme_b200.peaks import find_candidate_indices
+
+    c = np.random.default_rng(n + span).integers(-span, span, (n, 3)).astype(np.int64)
+    assert np.array_equal(find_candidate_indices(c, md), O.find_candidate_indices(c, md))
+    far = c + np.array([1 << 31, -(1 << 33), 5])  # coordinates beyond 32 bits
+    assert np.array_equal(find_candidate_indices(far, md), O.find_candidate_indices(c, md))
+
+
+def test_greedy_filter_settles_long_chains():
+    """Points a step apart, each too close to its neighbours: every second one is kept, in
+    whatever order they come."""
+    from pytme_b200.peaks import find_candidate_indices
+
+    c = np.zeros((500, 3), np.int64)
+    c[:, 1] = np.arange(500)
+    assert np.array_equal(find_candidate_indices(c, 1), np.arange(0, 500, 2))
+    p = np.random.default_rng(0).permutation(500)
+    assert np.array_equal(find_candidate_indices(c[p], 1), O.find_candidate_indices(c[p], 1))
+    assert np.array_equal(find_candidate_indices(c, 1 << 40), [0])
