@@ -9,6 +9,7 @@ distance filter running on the GPU (``pytme_b200.peaks``).
 """
 from __future__ import annotations
 
+import threading
 from typing import Dict, List, Tuple
 
 import numpy as np
@@ -20,20 +21,31 @@ from .matching import apply_convolution_mode
 _NUMPY_DTYPES = {torch.float32: np.float32, torch.int32: np.int32, torch.float64: np.float64,
                  torch.int64: np.int64}
 _CHUNK = 16 << 20
+_PINNED_MIN = 1 << 20
 _staging: Dict[str, torch.Tensor] = {}
+_staging_lock = threading.Lock()
 
 
 def download(t: torch.Tensor) -> np.ndarray:
     """A device tensor as a new host array.
 
-    Large tensors go through two pinned 16 MiB chunks, kept for the life of the process:
-    the copy engine fills one while the host copies the other into the result. A plain
-    ``.cpu()`` stages through pageable memory and moved the 420 MB state of a
-    512x512x200 scan at about 2 GB/s."""
+    Tensors from 1 MiB on go through two pinned chunks of at most 16 MiB, kept for the life of
+    the process: the copy engine fills one while the host copies the other into the result. A
+    plain ``.cpu()`` stages through pageable memory and moved the 420 MB state of a 512x512x200
+    scan, and the 13 MB maps of a 160x160x128 one, at about 2 GB/s. A thread that finds the
+    chunks in use takes the plain way."""
     t = t.contiguous()
     nbytes = t.numel() * t.element_size()
-    if not t.is_cuda or nbytes < 2 * _CHUNK or t.dtype not in _NUMPY_DTYPES:
+    if not t.is_cuda or nbytes < _PINNED_MIN or t.dtype not in _NUMPY_DTYPES \
+            or not _staging_lock.acquire(blocking=False):
         return t.cpu().numpy()
+    try:
+        return _download_pinned(t, nbytes)
+    finally:
+        _staging_lock.release()
+
+
+def _download_pinned(t: torch.Tensor, nbytes: int) -> np.ndarray:
     stage = _staging.get("pinned")
     if stage is None:
         stage = torch.empty(2 * _CHUNK, dtype=torch.uint8, pin_memory=True)
@@ -43,9 +55,11 @@ def download(t: torch.Tensor) -> np.ndarray:
     dst = out.reshape(-1).view(np.uint8)
     stream = torch.cuda.current_stream(t.device)
     done = [torch.cuda.Event(), torch.cuda.Event()]
+    # at least four chunks, so that copies and host work overlap on small maps too
+    chunk = min(_CHUNK, max(1 << 18, -(-nbytes // 4)))
     pending = None
-    for i, off in enumerate(range(0, nbytes, _CHUNK)):
-        m = min(_CHUNK, nbytes - off)
+    for i, off in enumerate(range(0, nbytes, chunk)):
+        m = min(chunk, nbytes - off)
         # chunk i - 2 used this half and was copied out in the previous iteration
         stage[(i % 2) * _CHUNK:(i % 2) * _CHUNK + m].copy_(src[off:off + m], non_blocking=True)
         done[i % 2].record(stream)

@@ -23,6 +23,7 @@ from typing import Dict, List, Optional, Sequence, Tuple
 import numpy as np
 import torch
 
+from .analyzer import download
 from .matching import (TargetSpectrum, _evaluate_filter, apply_convolution_mode,
                        fourier_padding, rigid_transform_matrices)
 from .scores import ScanPlan, _prepare_target
@@ -223,7 +224,7 @@ def scan_batch(jobs: List[MatchJob], precision: str = "mixed", rotation_batch="a
             r = torch.roll(sarg, shifts=shift, dims=axis)
             s = apply_convolution_mode(s, "same", job.target.shape, tmpl.shape, conv)
             r = apply_convolution_mode(r, "same", job.target.shape, tmpl.shape, conv)
-            out.append((s.contiguous().cpu().numpy(), r.contiguous().cpu().numpy()))
+            out.append((download(s), download(r)))
     finally:
         for p in plans.values():
             p.close()

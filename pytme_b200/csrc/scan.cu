@@ -249,9 +249,10 @@ __global__ void sum_double_kernel(const float* __restrict__ x, int64_t n, double
   }
 }
 
+// out_c = x - mean in float; out_z = (v, v^2) of v = x - mean in double.
 __global__ void center_kernel(const float* __restrict__ x, const double* __restrict__ partial,
                               int nparts, int64_t n, float* __restrict__ out_c,
-                              double* __restrict__ out_d, double* __restrict__ out_d2) {
+                              double2* __restrict__ out_z) {
   __shared__ double mean;
   if (threadIdx.x == 0) {
     double s = 0.0;
@@ -263,8 +264,7 @@ __global__ void center_kernel(const float* __restrict__ x, const double* __restr
        i += (int64_t)gridDim.x * blockDim.x) {
     double v = (double)x[i] - mean;
     if (out_c) out_c[i] = (float)v;
-    if (out_d) out_d[i] = v;
-    if (out_d2) out_d2[i] = v * v;
+    if (out_z) out_z[i] = make_double2(v, v * v);
   }
 }
 
@@ -276,8 +276,8 @@ __global__ void square_kernel(const float* __restrict__ x, float* __restrict__ y
   }
 }
 
-__global__ void zmul_kernel(const double2* __restrict__ a, const double2* __restrict__ b,
-                            double2* __restrict__ out, int64_t n) {
+__global__ void zmul_kernel(const double2* a, const double2* __restrict__ b, double2* out,
+                            int64_t n) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     double2 x = a[i], y = b[i];
@@ -286,7 +286,7 @@ __global__ void zmul_kernel(const double2* __restrict__ a, const double2* __rest
 }
 
 __global__ void pad_double_kernel(const float* __restrict__ src, int t0, int t1, int t2,
-                                  double* __restrict__ dst, int n1, int n2) {
+                                  double2* __restrict__ dst, int n1, int n2) {
   const int64_t n = (int64_t)t0 * t1 * t2;
   for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n;
        v += (int64_t)gridDim.x * blockDim.x) {
@@ -294,18 +294,19 @@ __global__ void pad_double_kernel(const float* __restrict__ src, int t0, int t1,
     int64_t r = v / t2;
     int i1 = (int)(r % t1);
     int i0 = (int)(r / t1);
-    dst[((int64_t)i0 * n1 + i1) * n2 + i2] = (double)src[v];
+    dst[((int64_t)i0 * n1 + i1) * n2 + i2] = make_double2((double)src[v], 0.0);
   }
 }
 
-// inverse denominator 1 / (n_obs * sd) from unnormalised double inverse transforms
-__global__ void inv_den_kernel(const double* __restrict__ cc1, const double* __restrict__ cc2,
-                               double invN, double n_obs, double eps, float* __restrict__ out,
+// inverse denominator 1 / (n_obs * sd) from the unnormalised double inverse transform, whose
+// real and imaginary parts are CC(f, m) and CC(f^2, m)
+__global__ void inv_den_kernel(const double2* __restrict__ cc, double invN, double n_obs, double eps, float* __restrict__ out,
                                int64_t n) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
-    double e = cc1[i] * invN / n_obs;
-    double e2 = cc2[i] * invN / n_obs;
+    const double2 c = cc[i];
+    double e = c.x * invN / n_obs;
+    double e2 = c.y * invN / n_obs;
     double var = e2 - e * e;
     double sd = sqrt(var > 0 ? var : 0.0);
     if (sd < eps) sd = 1.0;
@@ -407,8 +408,13 @@ struct Scan {
   GenConfig gen{};                  // line-FFT passes
   HalfConfig hc{};                  // template, x and y passes over half2 spectra
   float4* gtw[3] = {};              // their twiddle tables
+  // cuFFT plans, made when first needed: fast shape r2c (target) and c2r (plain path),
+  // template shape (filter)
   cufftHandle fwd = 0, inv = 0, tfwd = 0, tinv = 0;
-  bool have_fwd = false, have_tfwd = false;
+  bool have_fwd = false, have_inv = false, have_tfwd = false;
+  // buffers of a launch group, idle while the target is set
+  char* group = nullptr;
+  size_t group_bytes = 0;
   // CUDA-graph replay of a full launch group (see scan_set_graph)
   bool use_graph = false;
   cudaGraphExec_t gexec = nullptr;
@@ -613,7 +619,8 @@ static void destroy(Scan* s) {
   if (s->gev_out) cudaEventDestroy(s->gev_out);
   if (s->have_events)
     for (auto& e : s->ev) cudaEventDestroy(e);
-  if (s->have_fwd) { cufftDestroy(s->fwd); cufftDestroy(s->inv); }
+  if (s->have_fwd) cufftDestroy(s->fwd);
+  if (s->have_inv) cufftDestroy(s->inv);
   if (s->have_tfwd) { cufftDestroy(s->tfwd); cufftDestroy(s->tinv); }
   if (s->base) cudaFree(s->base);
   if (s->coef) cudaFree(s->coef);
@@ -727,6 +734,7 @@ int scan_create(const tm_scan_desc* desc, Scan** out, bool any_length) {
       o_Hm = take(sizeof(float2) * (size_t)B * s->SH);
       o_Hm2 = take(sizeof(float2) * (size_t)B * s->SH);
     }
+    s->group_bytes = off - o_G;
     o_tw0 = take(sizeof(float2) * s->n0);
     o_tw1 = take(sizeof(float2) * s->n1);
     o_tw2 = take(sizeof(float2) * s->n2);
@@ -799,6 +807,7 @@ int scan_create(const tm_scan_desc* desc, Scan** out, bool any_length) {
     }
   } else {
     s->G = reinterpret_cast<float2*>(b8 + o_G);
+    s->group = b8 + o_G;
     s->H = b8 + o_H;
     if (h2_buf) s->H2 = b8 + o_H2;
     if (d.score == TM_SCORE_FLC) {
@@ -858,39 +867,86 @@ int scan_create(const tm_scan_desc* desc, Scan** out, bool any_length) {
       if (st != TM_OK) { destroy(s); return st; }
     }
   }
-  // ---- cuFFT plans: fast-shape r2c/c2r (setup and plain path), template-shape (filter)
-  int r;
-  r = cufftPlan3d(&s->fwd, s->n0, s->n1, s->n2, CUFFT_R2C);
-  if (r == CUFFT_SUCCESS) r = cufftPlan3d(&s->inv, s->n0, s->n1, s->n2, CUFFT_C2R);
-  if (r != CUFFT_SUCCESS) { int st = cufft_status((cufftResult)r, "scan_create: fast plans"); destroy(s); return st; }
-  s->have_fwd = true;
-  int ts[3] = {s->t0, s->t1, s->t2};
-  r = cufftPlanMany(&s->tfwd, 3, ts, nullptr, 1, 0, nullptr, 1, 0, CUFFT_R2C, B);
-  if (r == CUFFT_SUCCESS)
-    r = cufftPlanMany(&s->tinv, 3, ts, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2R, B);
-  if (r != CUFFT_SUCCESS) { int st = cufft_status((cufftResult)r, "scan_create: template plans"); destroy(s); return st; }
-  s->have_tfwd = true;
   *out = s;
   return TM_OK;
 }
 
 int64_t scan_device_bytes(const Scan* s) { return (int64_t)s->bytes; }
 
+static int need_fwd(Scan* s) {
+  if (s->have_fwd) return TM_OK;
+  TM_TRY(cufft_status(cufftPlan3d(&s->fwd, s->n0, s->n1, s->n2, CUFFT_R2C), "r2c plan"));
+  s->have_fwd = true;
+  return TM_OK;
+}
+
+static int need_inv(Scan* s) {
+  if (s->have_inv) return TM_OK;
+  TM_TRY(cufft_status(cufftPlan3d(&s->inv, s->n0, s->n1, s->n2, CUFFT_C2R), "c2r plan"));
+  s->have_inv = true;
+  return TM_OK;
+}
+
+static int need_template_plans(Scan* s) {
+  if (s->have_tfwd) return TM_OK;
+  int ts[3] = {s->t0, s->t1, s->t2};
+  TM_TRY(cufft_status(cufftPlanMany(&s->tfwd, 3, ts, nullptr, 1, 0, nullptr, 1, 0, CUFFT_R2C, s->B),
+                      "template r2c plan"));
+  const cufftResult r =
+      cufftPlanMany(&s->tinv, 3, ts, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2R, s->B);
+  if (r != CUFFT_SUCCESS) {
+    cufftDestroy(s->tfwd);
+    return cufft_status(r, "template c2r plan");
+  }
+  s->have_tfwd = true;
+  return TM_OK;
+}
+
+// Work buffers of scan_set_target: from the plan's idle group buffers while they last, else
+// from the stream's pool (which unmaps them again at the next synchronisation: that alone took
+// milliseconds a call). Freed, in stream order, when it goes out of scope.
+struct TargetWork {
+  Scan* s;
+  cudaStream_t st;
+  size_t used = 0;
+  std::vector<void*> owned;
+  TargetWork(Scan* s_, cudaStream_t st_) : s(s_), st(st_) {}
+  TargetWork(const TargetWork&) = delete;
+  TargetWork& operator=(const TargetWork&) = delete;
+  ~TargetWork() {
+    for (void* p : owned) cudaFreeAsync(p, st);
+  }
+  template <typename T>
+  int get(T** out, int64_t n) {
+    const size_t bytes = (sizeof(T) * (size_t)n + 255) & ~(size_t)255;
+    if (s->group && used + bytes <= s->group_bytes) {
+      *out = reinterpret_cast<T*>(s->group + used);
+      used += bytes;
+      return TM_OK;
+    }
+    void* p = nullptr;
+    TM_TRY(cuda_status(cudaMallocAsync(&p, bytes, st), "scan_set_target: alloc"));
+    owned.push_back(p);
+    *out = static_cast<T*>(p);
+    return TM_OK;
+  }
+};
+
 // target: fast-shaped (top-left padded, already filtered) float32 device array.
 int scan_set_target(Scan* s, const float* target, cudaStream_t stream) {
   TM_REQUIRE(s && target, "scan_set_target: null pointer");
   TM_TRY(cuda_status(cudaStreamSynchronize(stream), "scan_set_target: sync"));
+  TM_TRY(need_fwd(s));
   cufftSetStream(s->fwd, stream);
-  cufftSetStream(s->inv, stream);
-  const int64_t N = s->N, S = s->S;
+  const int64_t N = s->N;
+  TargetWork work(s, stream);
   if (s->d.score == TM_SCORE_CC) {
     // CC correlates the raw target (cc_setup, tme/matching_scores.py:153-189)
     float* tmp = nullptr;
-    TM_TRY(cuda_status(cudaMallocAsync((void**)&tmp, sizeof(float) * N, stream), "scan_set_target: alloc"));
+    TM_TRY(work.get(&tmp, N));
     cudaMemcpyAsync(tmp, target, sizeof(float) * N, cudaMemcpyDeviceToDevice, stream);
-    int r = cufftExecR2C(s->fwd, tmp, (cufftComplex*)s->ft_target);
-    cudaFreeAsync(tmp, stream);
-    TM_TRY(cufft_status((cufftResult)r, "scan_set_target: r2c"));
+    TM_TRY(cufft_status(cufftExecR2C(s->fwd, tmp, (cufftComplex*)s->ft_target),
+                        "scan_set_target: r2c"));
     if (s->xtc_avail)
       TM_TRY(xcorr_tc_prepare(s->ft_target, s->ctarget, s->n0, s->n1, s->h2, stream));
     s->target_ready = true;
@@ -902,10 +958,10 @@ int scan_set_target(Scan* s, const float* target, cudaStream_t stream) {
   const int nparts = 592;
   double* partial = nullptr;
   float* centred = nullptr;
-  TM_TRY(cuda_status(cudaMallocAsync((void**)&partial, sizeof(double) * nparts, stream), "alloc"));
-  TM_TRY(cuda_status(cudaMallocAsync((void**)&centred, sizeof(float) * N, stream), "alloc"));
+  TM_TRY(work.get(&partial, nparts));
+  TM_TRY(work.get(&centred, N));
   sum_double_kernel<<<nparts, 256, 0, stream>>>(target, N, partial);
-  center_kernel<<<grid_for(N), 256, 0, stream>>>(target, partial, nparts, N, centred, nullptr, nullptr);
+  center_kernel<<<grid_for(N), 256, 0, stream>>>(target, partial, nparts, N, centred, nullptr);
   TM_TRY(check_launch("scan_set_target: centre"));
   std::vector<double> hp(nparts);
   cudaMemcpyAsync(hp.data(), partial, sizeof(double) * nparts, cudaMemcpyDeviceToHost, stream);
@@ -913,60 +969,41 @@ int scan_set_target(Scan* s, const float* target, cudaStream_t stream) {
   double tot = 0.0;
   for (double v : hp) tot += v;
   s->target_mean = tot / (double)N;
-  int r;
   if (s->d.score == TM_SCORE_FLC) {
     // flc_setup (tme/matching_scores.py:357-387): spectra of f and f^2
     float* sq = nullptr;
-    TM_TRY(cuda_status(cudaMallocAsync((void**)&sq, sizeof(float) * N, stream), "alloc"));
+    TM_TRY(work.get(&sq, N));
     square_kernel<<<grid_for(N), 256, 0, stream>>>(centred, sq, N);
-    r = cufftExecR2C(s->fwd, centred, (cufftComplex*)s->ft_target);
+    cufftResult r = cufftExecR2C(s->fwd, centred, (cufftComplex*)s->ft_target);
     if (r == CUFFT_SUCCESS) r = cufftExecR2C(s->fwd, sq, (cufftComplex*)s->ft_target2);
-    cudaFreeAsync(sq, stream);
+    TM_TRY(cufft_status(r, "scan_set_target: transforms"));
   } else {
     // flcSphericalMask_setup (tme/matching_scores.py:390-450): the local-variance
-    // denominator from CC(f^2, m) and CC(f, m), here in double precision.
+    // denominator from CC(f, m) and CC(f^2, m) in double precision, as the two parts of one
+    // complex correlation of f + i f^2 with the mask: one complex plan for three transforms.
     TM_REQUIRE(s->template_ready, "scan_set_target: FLCSphericalMask needs the template mask first");
-    cufftHandle dfwd, dinv;
-    r = cufftPlan3d(&dfwd, s->n0, s->n1, s->n2, CUFFT_D2Z);
-    if (r != CUFFT_SUCCESS) { cudaFreeAsync(centred, stream); cudaFreeAsync(partial, stream); return cufft_status((cufftResult)r, "scan_set_target: D2Z plan"); }
-    r = cufftPlan3d(&dinv, s->n0, s->n1, s->n2, CUFFT_Z2D);
-    if (r != CUFFT_SUCCESS) { cufftDestroy(dfwd); cudaFreeAsync(centred, stream); cudaFreeAsync(partial, stream); return cufft_status((cufftResult)r, "scan_set_target: Z2D plan"); }
-    cufftSetStream(dfwd, stream);
-    cufftSetStream(dinv, stream);
-    double *f = nullptr, *f2 = nullptr;
-    double2 *Ff = nullptr, *Ff2 = nullptr, *Fm = nullptr;
-    cudaError_t e = cudaMallocAsync((void**)&f, sizeof(double) * N, stream);
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&f2, sizeof(double) * N, stream);
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&Ff, sizeof(double2) * S, stream);
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&Ff2, sizeof(double2) * S, stream);
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&Fm, sizeof(double2) * S, stream);
-    if (e != cudaSuccess) {
-      cufftDestroy(dfwd); cufftDestroy(dinv);
-      return cuda_status(e, "scan_set_target: FP64 buffers");
-    }
-    center_kernel<<<grid_for(N), 256, 0, stream>>>(target, partial, nparts, N, nullptr, f, f2);
-    r = cufftExecD2Z(dfwd, f, Ff);
-    if (r == CUFFT_SUCCESS) r = cufftExecD2Z(dfwd, f2, Ff2);
-    // mask: top-left padded into f (reused)
-    cudaMemsetAsync(f, 0, sizeof(double) * N, stream);
-    pad_double_kernel<<<grid_for(s->T), 256, 0, stream>>>(s->mask, s->t0, s->t1, s->t2, f, s->n1, s->n2);
-    if (r == CUFFT_SUCCESS) r = cufftExecD2Z(dfwd, f, Fm);
-    zmul_kernel<<<grid_for(S), 256, 0, stream>>>(Ff, Fm, Ff, S);
-    zmul_kernel<<<grid_for(S), 256, 0, stream>>>(Ff2, Fm, Ff2, S);
-    if (r == CUFFT_SUCCESS) r = cufftExecZ2D(dinv, Ff, f);
-    if (r == CUFFT_SUCCESS) r = cufftExecZ2D(dinv, Ff2, f2);
-    inv_den_kernel<<<grid_for(N), 256, 0, stream>>>(f, f2, 1.0 / (double)N, s->mask_sum,
+    double2 *f = nullptr, *m = nullptr;
+    TM_TRY(work.get(&f, N));
+    TM_TRY(work.get(&m, N));
+    cufftHandle z2z;
+    TM_TRY(cufft_status(cufftPlan3d(&z2z, s->n0, s->n1, s->n2, CUFFT_Z2Z),
+                        "scan_set_target: Z2Z plan"));
+    cufftSetStream(z2z, stream);
+    center_kernel<<<grid_for(N), 256, 0, stream>>>(target, partial, nparts, N, nullptr, f);
+    cudaMemsetAsync(m, 0, sizeof(double2) * N, stream);
+    pad_double_kernel<<<grid_for(s->T), 256, 0, stream>>>(s->mask, s->t0, s->t1, s->t2, m, s->n1,
+                                                         s->n2);
+    cufftResult r = cufftExecZ2Z(z2z, f, f, CUFFT_FORWARD);
+    if (r == CUFFT_SUCCESS) r = cufftExecZ2Z(z2z, m, m, CUFFT_FORWARD);
+    zmul_kernel<<<grid_for(N), 256, 0, stream>>>(f, m, f, N);
+    if (r == CUFFT_SUCCESS) r = cufftExecZ2Z(z2z, f, f, CUFFT_INVERSE);
+    inv_den_kernel<<<grid_for(N), 256, 0, stream>>>(f, 1.0 / (double)N, s->mask_sum,
                                                    (double)1.1920928955078125e-07, s->inv_den, N);
     if (r == CUFFT_SUCCESS) r = cufftExecR2C(s->fwd, centred, (cufftComplex*)s->ft_target);
-    cudaFreeAsync(f, stream); cudaFreeAsync(f2, stream);
-    cudaFreeAsync(Ff, stream); cudaFreeAsync(Ff2, stream); cudaFreeAsync(Fm, stream);
     cudaStreamSynchronize(stream);
-    cufftDestroy(dfwd);
-    cufftDestroy(dinv);
+    cufftDestroy(z2z);
+    TM_TRY(cufft_status(r, "scan_set_target: transforms"));
   }
-  cudaFreeAsync(centred, stream);
-  cudaFreeAsync(partial, stream);
-  TM_TRY(cufft_status((cufftResult)r, "scan_set_target: transforms"));
   if (s->xtc_avail)
     TM_TRY(xcorr_tc_prepare(s->ft_target, s->ctarget, s->n0, s->n1, s->h2, stream));
   s->target_ready = true;
@@ -1087,6 +1124,7 @@ int scan_set_template(Scan* s, const float* tmpl, const float* mask, const float
   TM_REQUIRE(s->d.score == TM_SCORE_CC || mask, "scan_set_template: this score needs a mask");
   cudaMemcpyAsync(s->tmpl, tmpl, sizeof(float) * s->T, cudaMemcpyDeviceToDevice, stream);
   if (mask) cudaMemcpyAsync(s->mask, mask, sizeof(float) * s->T, cudaMemcpyDeviceToDevice, stream);
+  if (filt) TM_TRY(need_template_plans(s));
   s->d.has_template_filter = filt != nullptr;
   if (filt) cudaMemcpyAsync(s->tfilter, filt, sizeof(float) * s->TS, cudaMemcpyDeviceToDevice, stream);
   if (mask) {
@@ -1168,6 +1206,8 @@ static int run_plain(Scan* s, int n, int32_t first_index, float* state_max, int3
   const float scale = (float)(1.0 / (double)N);
   const double eps = 1.1920928955078125e-07;
   const bool flc = s->d.score == TM_SCORE_FLC;
+  TM_TRY(need_fwd(s));
+  TM_TRY(need_inv(s));
   cufftSetStream(s->fwd, stream);
   cufftSetStream(s->inv, stream);
   for (int i = 0; i < n; ++i) {
