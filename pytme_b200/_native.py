@@ -43,7 +43,8 @@ EXPORTED = (
     "tm_find_candidate_indices_workspace", "tm_find_candidate_indices",
     "tm_find_candidate_indices_noalloc", "tm_fft_filter",
     "tm_euler_zyz", "tm_refine_rotate", "tm_refine_forward", "tm_refine_grad_filtered",
-    "tm_refine_backward", "tm_spline_prefilter", "tm_rigid_transform_cubic",
+    "tm_refine_backward", "tm_refine_backward_workspace", "tm_refine_backward_ws",
+    "tm_spline_prefilter", "tm_rigid_transform_cubic",
     "tm_scan_set_interpolation", "tm_build_filter", "tm_whitening_bins", "tm_whitening_filter",
     "tm_scan_set_xpass", "tm_scan_check", "tm_scan_xpass_mode", "tm_scan_set_zpass",
     "tm_scan_zpass_mode", "tm_scan_set_ypass", "tm_scan_ypass_mode", "tm_scan_set_wait_budget",
@@ -153,6 +154,9 @@ def _load():
         "tm_refine_rotate": (c_int, [POINTER(RefineDesc), f32p, vp]),
         "tm_refine_forward": (c_int, [POINTER(RefineDesc), f32p, vp, f32p, vp]),
         "tm_refine_grad_filtered": (c_int, [POINTER(RefineDesc), f32p, vp, f32p, f32p, vp]),
+        "tm_refine_backward_workspace": (c_int64, [POINTER(RefineDesc)]),
+        "tm_refine_backward_ws": (c_int, [POINTER(RefineDesc), f32p, f32p, vp, f32p, f32p, vp, vp,
+                                          vp, f32p, vp, vp]),
         "tm_refine_backward": (c_int, [POINTER(RefineDesc), f32p, f32p, vp, f32p, f32p, vp, vp,
                                        vp, f32p, vp]),
     }

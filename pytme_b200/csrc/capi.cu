@@ -364,8 +364,10 @@ int tm_fft_filter(tm_fft_plan* p, float* x, void* spectrum, const float* filter,
   TM_REQUIRE(p && x && spectrum && filter, "tm_fft_filter: null pointer");
   TM_REQUIRE(!p->dbl, "tm_fft_filter: single-precision plans only");
   TM_TRY(tm_fft_r2c(p, x, spectrum, stream));
-  TM_TRY(tmb::apply_real_filter(spectrum, filter, p->n_ft, p->batch, S(stream)));
-  return tm_fft_c2r(p, spectrum, x, 1.0 / (double)p->n_item, stream);
+  // the inverse transform's scale goes in with the filter
+  TM_TRY(tmb::apply_real_filter(spectrum, filter, p->n_ft, p->batch, S(stream),
+                                (float)(1.0 / (double)p->n_item)));
+  return tm_fft_c2r(p, spectrum, x, 1.0, stream);
 }
 
 // ------------------------------------------------------------------ refinement
@@ -415,7 +417,23 @@ int tm_refine_backward(const tm_refine_desc* d, const float* tmpl_filtered,
                        double* grad_angles, float* grad_tmpl, void* stream) {
   TM_REQUIRE(d, "tm_refine_backward: null descriptor");
   return tmb::refine_backward(refine_args(d), tmpl_filtered, grad_rotated, sums, grad_scores,
-                              drot, grad_rot, grad_shift, grad_angles, grad_tmpl, S(stream));
+                              drot, grad_rot, grad_shift, grad_angles, grad_tmpl, nullptr,
+                              S(stream));
+}
+
+int64_t tm_refine_backward_workspace(const tm_refine_desc* d) {
+  return d ? 16LL * d->template_shape[0] * d->template_shape[1] * d->template_shape[2] : 0;
+}
+
+int tm_refine_backward_ws(const tm_refine_desc* d, const float* tmpl_filtered,
+                          const float* grad_rotated, const double* sums,
+                          const float* grad_scores, const float* drot, double* grad_rot,
+                          double* grad_shift, double* grad_angles, float* grad_tmpl,
+                          void* workspace, void* stream) {
+  TM_REQUIRE(d, "tm_refine_backward_ws: null descriptor");
+  return tmb::refine_backward(refine_args(d), tmpl_filtered, grad_rotated, sums, grad_scores,
+                              drot, grad_rot, grad_shift, grad_angles, grad_tmpl, workspace,
+                              S(stream));
 }
 
 }  // extern "C"

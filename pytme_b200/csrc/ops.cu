@@ -528,23 +528,27 @@ int complex_multiply(const void* a, const void* b, void* out, int64_t n, cudaStr
   return check_launch("cmul_kernel");
 }
 
-// spectrum *= real filter, broadcast over a batch of spectra
-__global__ void filter_kernel(float2* __restrict__ x, const float* __restrict__ f, int64_t n,
-                              int batch) {
-  const int64_t total = n * batch;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
+// spectrum *= real filter (times a scale), broadcast over a batch of spectra; grid (n, batch)
+__global__ void filter_kernel(float2* __restrict__ x, const float* __restrict__ f, float scale,
+                              int64_t n, int batch) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
-    float w = f[i % n];
-    float2 v = x[i];
-    x[i] = make_float2(v.x * w, v.y * w);
+    const float w = f[i] * scale;
+    for (int b = blockIdx.y; b < batch; b += gridDim.y) {
+      float2 v = x[b * n + i];
+      x[b * n + i] = make_float2(v.x * w, v.y * w);
+    }
   }
 }
 
-int apply_real_filter(void* spectra, const float* filt, int64_t n, int batch, cudaStream_t stream) {
+int apply_real_filter(void* spectra, const float* filt, int64_t n, int batch, cudaStream_t stream,
+                      float scale) {
   if (n <= 0 || batch <= 0) return TM_OK;
-  int64_t blocks = ceil_div(n * batch, 256);
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  filter_kernel<<<(unsigned)blocks, 256, 0, stream>>>((float2*)spectra, filt, n, batch);
+  const int64_t bx = std::min<int64_t>(ceil_div(n, 256), 148 * 16);
+  // about sixteen CTAs an SM; a thread takes the same place of several spectra
+  const int64_t by = std::max<int64_t>(1, std::min<int64_t>(batch, 148 * 16 / bx));
+  filter_kernel<<<dim3((unsigned)bx, (unsigned)by), 256, 0, stream>>>((float2*)spectra, filt, scale,
+                                                                     n, batch);
   return check_launch("filter_kernel");
 }
 

@@ -52,7 +52,8 @@ int max_score_over_rotations(const float* scores, float* max_scores, int32_t* ro
                              int32_t index, int64_t n, cudaStream_t stream);
 
 int complex_multiply(const void* a, const void* b, void* out, int64_t n, cudaStream_t stream);
-int apply_real_filter(void* spectra, const float* filt, int64_t n, int batch, cudaStream_t stream);
+int apply_real_filter(void* spectra, const float* filt, int64_t n, int batch, cudaStream_t stream,
+                      float scale = 1.f);
 int scale_real(float* x, float s, int64_t n, cudaStream_t stream);
 int plain_epilogue(const float* x, const float* inv_den, const float* cc_m, const float* cc_m2,
                    const double* stats, double eps, float scale, float* mx, int32_t* rot,

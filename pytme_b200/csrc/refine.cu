@@ -23,7 +23,7 @@
 // pass); per voxel dS/dT_f = M_r (gB + 2 gC T_f + gD f) and
 // dS/dM_r = gA + gB T_f + gC T_f^2 + gD T_f f + gE f + gF f^2 are chained through the
 // trilinear weights into dS/du, then into dS/dR, dS/ds, dS/d(angles) and the template
-// density gradient (summed over peaks, in shared memory when t^3 floats fit).
+// density gradient (summed over peaks with 16-byte atomics, see refine_backward_kernel).
 #include "common.cuh"
 #include "refine.cuh"
 
@@ -35,8 +35,11 @@ namespace tmb {
 namespace {
 
 constexpr int kRefThreads = 256;
-constexpr int kRefBackSmemThreads = 512;       // one CTA per SM holds the gradient
-constexpr int kSmemGradMaxVoxels = 48 * 1024;  // 192 KiB of float template gradient
+// Voxels a thread of the per-voxel kernels takes: setting up its walk through the box (five
+// integer divisions), the pose and, for the gradient, the score's double-precision derivatives
+// cost more than a voxel (2048 peaks of 32^3, one voxel a thread: rotation 0.64 ms, gradient of
+// the filtered template 1.18 ms).
+constexpr int kRefVoxels = 16;
 
 struct Box {
   int t0, t1, t2;
@@ -312,31 +315,46 @@ refine_forward_kernel(const float* __restrict__ T, const float* __restrict__ M, 
     double acc[6] = {0, 0, 0, 0, 0, 0};
     Walker w;
     w.init(b, threadIdx.x, blockDim.x);
-    for (int v = threadIdx.x; v < b.nv; v += blockDim.x, w.next(b)) {
-      float d[3], u[3];
-      pose_coords(b, Rs, ss, w, d, u);
-      Stencil st;
-      if (!stencil(b, u, st)) continue;
-      float c[8];
-      corners8(M, st, c);
-      const float mr = lerp8(c, st);
-      if (mr == 0.f) continue;
-      float tr;
-      if (FILTERED) {
-        tr = __ldg(Tf + (int64_t)p * b.nv + v);
-      } else {
-        corners8(T, st, c);
-        tr = lerp8(c, st);
+    // Without the filter two voxels at a time, their mask corners in flight together (512 peaks
+    // of 48^3: 0.87 ms with one, 0.76 with two); with it the registers cost more than that gives
+    // (2048 peaks of 32^3: 0.53 and 0.69 ms).
+    constexpr int AHEAD = FILTERED ? 1 : 2;
+    for (int v = threadIdx.x; v < b.nv; v += AHEAD * blockDim.x) {
+      Stencil st[AHEAD];
+      float c[AHEAD][8];
+      Walker at[AHEAD];
+      bool in[AHEAD];
+#pragma unroll
+      for (int k = 0; k < AHEAD; ++k) {
+        at[k] = w;
+        float d[3], u[3];
+        pose_coords(b, Rs, ss, w, d, u);
+        in[k] = v + k * (int)blockDim.x < b.nv && stencil(b, u, st[k]);
+        if (in[k]) corners8(M, st[k], c[k]);
+        w.next(b);
       }
-      const double m = mr, tf = tr;
-      const double f = target_at(tg, n0, n1, n2, outside, ks, w);
-      const double mt = m * tf, mf = m * f;
-      acc[0] += m;
-      acc[1] += mt;
-      acc[2] += mt * tf;
-      acc[3] += mt * f;
-      acc[4] += mf;
-      acc[5] += mf * f;
+#pragma unroll
+      for (int k = 0; k < AHEAD; ++k) {
+        if (!in[k]) continue;
+        const float mr = lerp8(c[k], st[k]);
+        if (mr == 0.f) continue;
+        float tr;
+        if (FILTERED) {
+          tr = __ldg(Tf + (int64_t)p * b.nv + v + k * (int)blockDim.x);
+        } else {
+          corners8(T, st[k], c[k]);
+          tr = lerp8(c[k], st[k]);
+        }
+        const double m = mr, tf = tr;
+        const double f = target_at(tg, n0, n1, n2, outside, ks, at[k]);
+        const double mt = m * tf, mf = m * f;
+        acc[0] += m;
+        acc[1] += mt;
+        acc[2] += mt * tf;
+        acc[3] += mt * f;
+        acc[4] += mf;
+        acc[5] += mf * f;
+      }
     }
     block_sums<6>(acc, red);
     if (threadIdx.x == 0) {
@@ -358,9 +376,11 @@ refine_grad_filtered_kernel(const float* __restrict__ M, int t0, int t1, int t2,
   const int p = blockIdx.y;
   __shared__ float Rs[9], ss[3];
   __shared__ int ks[3];
+  __shared__ ScoreGrad shared_grad;
   load_pose(rot, shifts, corners, p, Rs, ss, ks);
+  if (threadIdx.x == 32) shared_grad = score_grad(sums + 6 * p, eps, (double)gout[p]);
   __syncthreads();
-  const ScoreGrad sg = score_grad(sums + 6 * p, eps, (double)gout[p]);
+  const ScoreGrad sg = shared_grad;
   const Box b = make_box(t0, t1, t2);
   const int start = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
   Walker w;
@@ -388,9 +408,13 @@ refine_grad_filtered_kernel(const float* __restrict__ M, int t0, int t1, int t2,
 
 // Chain through the interpolation into the pose and template gradients. FILTERED reads
 // T_f and dS/dT_r = L^T dS/dT_f from memory; otherwise both come from the in-place
-// interpolation. SMEM_GT accumulates the template gradient in shared memory.
-template <bool FILTERED, bool SMEM_GT, int THREADS>
-__global__ void __launch_bounds__(THREADS)
+// interpolation. The scatter of the template gradient sets the pace: a voxel adds to the eight
+// corners of its cell, which are taken as two float4 atomics into the cell's own slot of gQ
+// (its four corners of either x plane, summed per template voxel by cell_gradient_kernel).
+// 2048 peaks of 32^3, every voxel scattering: eight adds in shared memory (one CTA an SM) 2.6 ms,
+// four float2 adds in global memory 1.76 ms.
+template <bool FILTERED>
+__global__ void __launch_bounds__(kRefThreads)
 refine_backward_kernel(const float* __restrict__ T, const float* __restrict__ M, int t0, int t1,
                        int t2, const float* __restrict__ rot, const float* __restrict__ shifts,
                        const int32_t* __restrict__ corners, int P, const float* __restrict__ Tf,
@@ -398,15 +422,11 @@ refine_backward_kernel(const float* __restrict__ T, const float* __restrict__ M,
                        int n1, int n2, float outside, double eps, const double* __restrict__ sums,
                        const float* __restrict__ gout, const float* __restrict__ dR,
                        double* __restrict__ grad_rot, double* __restrict__ grad_shift,
-                       double* __restrict__ grad_angles, float* __restrict__ gT) {
-  extern __shared__ float gts[];
+                       double* __restrict__ grad_angles, float4* __restrict__ gQ) {
   __shared__ double red[32 * 12];
   __shared__ float Rs[9], ss[3];
   __shared__ int ks[3];
   const Box b = make_box(t0, t1, t2);
-  if (SMEM_GT) {
-    for (int v = threadIdx.x; v < b.nv; v += blockDim.x) gts[v] = 0.f;
-  }
   for (int p = blockIdx.x; p < P; p += gridDim.x) {
     __syncthreads();
     if (threadIdx.x < 9) Rs[threadIdx.x] = rot[p * 9 + threadIdx.x];
@@ -432,31 +452,43 @@ refine_backward_kernel(const float* __restrict__ T, const float* __restrict__ M,
         Stencil st;
         if (!stencil(b, u, st)) continue;
         float tq[8], mq[8];
-        corners8(T, st, tq);
         corners8(M, st, mq);
-        const float mr = lerp8(mq, st);
-        const float tf = FILTERED ? __ldg(Tf + (int64_t)p * b.nv + v) : lerp8(tq, st);
-        const float f = target_at(tg, n0, n1, n2, outside, ks, w);
-        const float gm = fmaf(tf, fmaf(gC, tf, fmaf(gD, f, gB)), fmaf(f, fmaf(gF, f, gE), gA));
-        const float gt = FILTERED ? __ldg(gTr_in + (int64_t)p * b.nv + v)
-                                  : mr * fmaf(2.f * gC, tf, fmaf(gD, f, gB));
+        // where the mask is zero at all corners it adds nothing: the template's gradient there
+        // comes from the filter alone
+        bool masked = true;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) masked = masked && mq[q] == 0.f;
+        if (!FILTERED && masked) continue;
+        float gt = 0.f;
+        if (FILTERED) {
+          gt = __ldg(gTr_in + (int64_t)p * b.nv + v);
+          if (masked && gt == 0.f) continue;
+        }
+        corners8(T, st, tq);
+        float gm = 0.f;
+        if (!masked) {
+          const float mr = lerp8(mq, st);
+          const float tf = FILTERED ? __ldg(Tf + (int64_t)p * b.nv + v) : lerp8(tq, st);
+          const float f = target_at(tg, n0, n1, n2, outside, ks, w);
+          gm = fmaf(tf, fmaf(gC, tf, fmaf(gD, f, gB)), fmaf(f, fmaf(gF, f, gE), gA));
+          if (!FILTERED) gt = mr * fmaf(2.f * gC, tf, fmaf(gD, f, gB));
+        }
         // dS/du through the trilinear weights of T and M
         float e[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) e[q] = fmaf(gt, tq[q], gm * mq[q]);
         float du[3];
         lerp8_grad(e, st, du);
-        if (gT != nullptr && gt != 0.f) {
-          const float wx[2] = {1.f - st.f0, st.f0}, wy[2] = {1.f - st.f1, st.f1};
-          const float wz[2] = {(1.f - st.f2) * gt, st.f2 * gt};
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const int i = st.base + ((q & 4) ? st.s0 : 0) + ((q & 2) ? st.s1 : 0) +
-                          ((q & 1) ? st.s2 : 0);
-            const float wq = wx[q >> 2] * wy[(q >> 1) & 1] * wz[q & 1];
-            if (SMEM_GT) atomicAdd(gts + i, wq);
-            else atomicAdd(gT + i, wq);
-          }
+        if (gQ != nullptr && gt != 0.f) {
+          // corners (y, z), (y, z + 1), (y + 1, z), (y + 1, z + 1) of planes x and x + 1; a step
+          // of 0 at the upper edge goes with a weight of 0
+          const float y0 = 1.f - st.f1, z0 = (1.f - st.f2) * gt, z1 = st.f2 * gt;
+          const float4 c = make_float4(y0 * z0, y0 * z1, st.f1 * z0, st.f1 * z1);
+          const float x0 = 1.f - st.f0, x1 = st.f0;
+          atomicAdd(gQ + st.base, make_float4(x0 * c.x, x0 * c.y, x0 * c.z, x0 * c.w));
+          if (x1 != 0.f)
+            atomicAdd(gQ + st.base + st.s0,
+                      make_float4(x1 * c.x, x1 * c.y, x1 * c.z, x1 * c.w));
         }
         // u_i = sum_j R[j][i] d_j + c_i: dS/dR[j][i] += du_i d_j; dS/ds_j = -sum_i R[j][i] du_i
 #pragma unroll
@@ -488,13 +520,19 @@ refine_backward_kernel(const float* __restrict__ T, const float* __restrict__ M,
         }
     }
   }
-  if (SMEM_GT && gT != nullptr) {
-    __syncthreads();
-    for (int v = threadIdx.x; v < b.nv; v += blockDim.x) {
-      const float g = gts[v];
-      if (g != 0.f) atomicAdd(gT + v, g);
-    }
-  }
+}
+
+// Template gradient from the cells' slots.
+__global__ void cell_gradient_kernel(const float4* __restrict__ q, int t1, int t2, int nv,
+                                     float* __restrict__ gT) {
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= nv) return;
+  const int z = v % t2, y = v / t2 % t1;
+  float g = q[v].x;
+  if (z > 0) g += q[v - 1].y;
+  if (y > 0) g += q[v - t2].z;
+  if (z > 0 && y > 0) g += q[v - t2 - 1].w;
+  gT[v] += g;
 }
 
 int resident_grid(const void* fn, int threads, size_t smem, int P) {
@@ -528,12 +566,20 @@ static int check_refine_args(const RefineArgs& a, const char* what) {
   return TM_OK;
 }
 
+// CTAs of the per-voxel kernels: kRefVoxels a thread, fewer where few peaks would leave the chip
+// idle.
+static dim3 voxel_grid(int nv, int P) {
+  int64_t blocks = ceil_div(nv, kRefThreads * kRefVoxels);
+  while (blocks * P < 148 * 16 && blocks * kRefThreads < nv) blocks *= 2;
+  return dim3((unsigned)std::min<int64_t>(blocks, 512), (unsigned)P);
+}
+
 int refine_rotate(const RefineArgs& a, float* Tr, cudaStream_t st) {
   TM_TRY(check_refine_args(a, "refine_rotate"));
   TM_REQUIRE(Tr, "refine_rotate: null output");
   TM_REQUIRE(a.P <= 65535, "refine_rotate: at most 65535 peaks per call");
   const int nv = a.t[0] * a.t[1] * a.t[2];
-  dim3 g((unsigned)std::min<int64_t>(ceil_div(nv, kRefThreads), 512), (unsigned)a.P);
+  const dim3 g = voxel_grid(nv, a.P);
   refine_rotate_kernel<<<g, kRefThreads, 0, st>>>(a.tmpl, a.t[0], a.t[1], a.t[2], a.rot,
                                                   a.shifts, Tr);
   return check_launch("refine_rotate_kernel");
@@ -563,55 +609,45 @@ int refine_grad_filtered(const RefineArgs& a, const float* Tf, const double* sum
   TM_REQUIRE(Tf && sums && grad_scores && gTf, "refine_grad_filtered: null pointer");
   TM_REQUIRE(a.P <= 65535, "refine_grad_filtered: at most 65535 peaks per call");
   const int nv = a.t[0] * a.t[1] * a.t[2];
-  dim3 g((unsigned)std::min<int64_t>(ceil_div(nv, kRefThreads), 512), (unsigned)a.P);
+  const dim3 g = voxel_grid(nv, a.P);
   refine_grad_filtered_kernel<<<g, kRefThreads, 0, st>>>(
       a.mask, a.t[0], a.t[1], a.t[2], a.rot, a.shifts, a.corners, Tf, a.target, a.n[0], a.n[1],
       a.n[2], a.outside, a.eps, sums, grad_scores, gTf);
   return check_launch("refine_grad_filtered_kernel");
 }
 
-template <bool FILTERED, bool SMEM>
-static int launch_backward(const RefineArgs& a, const float* Tf, const float* gTr,
-                           const double* sums, const float* gout, const float* dR, double* gRot,
-                           double* gShift, double* gAng, float* gT, cudaStream_t st) {
-  constexpr int kThreads = SMEM ? kRefBackSmemThreads : kRefThreads;
-  const int nv = a.t[0] * a.t[1] * a.t[2];
-  const size_t smem = SMEM ? (size_t)nv * sizeof(float) : 0;
-  auto fn = refine_backward_kernel<FILTERED, SMEM, kThreads>;
-  if (SMEM)
-    TM_TRY(cuda_status(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)smem),
-                       "refine_backward: shared memory attribute"));
-  const int g = resident_grid((const void*)fn, kThreads, smem, a.P);
-  fn<<<g, kThreads, smem, st>>>(a.tmpl, a.mask, a.t[0], a.t[1], a.t[2], a.rot, a.shifts,
-                                   a.corners, a.P, Tf, gTr, a.target, a.n[0], a.n[1], a.n[2],
-                                   a.outside, a.eps, sums, gout, dR, gRot, gShift, gAng, gT);
-  return check_launch("refine_backward_kernel");
-}
-
 int refine_backward(const RefineArgs& a, const float* Tf, const float* gTr, const double* sums,
                     const float* grad_scores, const float* dR, double* grad_rot,
-                    double* grad_shift, double* grad_angles, float* grad_tmpl,
+                    double* grad_shift, double* grad_angles, float* grad_tmpl, void* workspace,
                     cudaStream_t st) {
   TM_TRY(check_refine_args(a, "refine_backward"));
   TM_REQUIRE(sums && grad_scores, "refine_backward: null pointer");
   TM_REQUIRE((Tf == nullptr) == (gTr == nullptr),
              "refine_backward: the filtered template and its gradient go together");
   TM_REQUIRE(!grad_angles || dR, "refine_backward: angle gradients need dR");
+  TM_REQUIRE((uintptr_t)workspace % 16 == 0, "refine_backward: workspace must be 16-byte aligned");
   const int nv = a.t[0] * a.t[1] * a.t[2];
-  const bool smem = grad_tmpl != nullptr && nv <= kSmemGradMaxVoxels;
-  if (Tf) {
-    if (smem)
-      return launch_backward<true, true>(a, Tf, gTr, sums, grad_scores, dR, grad_rot, grad_shift,
-                                         grad_angles, grad_tmpl, st);
-    return launch_backward<true, false>(a, Tf, gTr, sums, grad_scores, dR, grad_rot, grad_shift,
-                                        grad_angles, grad_tmpl, st);
+  float4* q = nullptr;
+  if (grad_tmpl) {
+    q = static_cast<float4*>(workspace);
+    if (!q)
+      TM_TRY(cuda_status(cudaMallocAsync((void**)&q, sizeof(float4) * (size_t)nv, st),
+                         "refine_backward: workspace"));
+    cudaMemsetAsync(q, 0, sizeof(float4) * (size_t)nv, st);
   }
-  if (smem)
-    return launch_backward<false, true>(a, nullptr, nullptr, sums, grad_scores, dR, grad_rot,
-                                        grad_shift, grad_angles, grad_tmpl, st);
-  return launch_backward<false, false>(a, nullptr, nullptr, sums, grad_scores, dR, grad_rot,
-                                       grad_shift, grad_angles, grad_tmpl, st);
+  auto fn = Tf ? refine_backward_kernel<true> : refine_backward_kernel<false>;
+  const int g = resident_grid((const void*)fn, kRefThreads, 0, a.P);
+  fn<<<g, kRefThreads, 0, st>>>(a.tmpl, a.mask, a.t[0], a.t[1], a.t[2], a.rot, a.shifts, a.corners,
+                                a.P, Tf, gTr, a.target, a.n[0], a.n[1], a.n[2], a.outside, a.eps,
+                                sums, grad_scores, dR, grad_rot, grad_shift, grad_angles, q);
+  int rc = check_launch("refine_backward_kernel");
+  if (q && rc == TM_OK) {
+    cell_gradient_kernel<<<(unsigned)ceil_div(nv, 256), 256, 0, st>>>(q, a.t[1], a.t[2], nv,
+                                                                     grad_tmpl);
+    rc = check_launch("cell_gradient_kernel");
+  }
+  if (q && !workspace) cudaFreeAsync(q, st);
+  return rc;
 }
 
 }  // namespace tmb

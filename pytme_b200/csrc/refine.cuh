@@ -31,7 +31,7 @@ int refine_grad_filtered(const RefineArgs& a, const float* Tf, const double* sum
                          const float* grad_scores, float* gTf, cudaStream_t st);
 int refine_backward(const RefineArgs& a, const float* Tf, const float* gTr, const double* sums,
                     const float* grad_scores, const float* dR, double* grad_rot,
-                    double* grad_shift, double* grad_angles, float* grad_tmpl,
+                    double* grad_shift, double* grad_angles, float* grad_tmpl, void* workspace,
                     cudaStream_t st);
 
 }  // namespace tmb

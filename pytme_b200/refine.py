@@ -22,8 +22,10 @@ c = (t - 1)/2, the rotation centre of the scan. The particle centre in the targe
 ``corners + c + shifts``.
 
 The rotated templates are checkpointed: the forward pass keeps only six sums per peak
-and the backward pass recomputes the rotation (and the template filter) instead of
-reading stored copies.
+and the backward pass recomputes the rotation instead of reading stored copies. With a
+template filter, whose transforms cost more than the rotation, the filtered templates are
+kept for the backward pass when all peaks fit one chunk and a quarter of
+``max_work_bytes``; beyond that they are recomputed too.
 """
 from __future__ import annotations
 
@@ -180,6 +182,8 @@ class RefineProblem:
         n_ft = self.template_shape[0] * self.template_shape[1] * (self.template_shape[2] // 2 + 1)
         per_peak = (2 * nv * 4 + n_ft * 8) if self.template_filter is not None else 0
         self.chunk = max(1, int(max_work_bytes // per_peak)) if per_peak else 1 << 30
+        # filtered templates up to this size stay from the forward to the backward pass
+        self.keep_bytes = int(max_work_bytes) // 4
         self._plans: Dict[int, _FilterPlan] = {}
 
     @property
@@ -257,23 +261,27 @@ class FLCRefineFunction(torch.autograd.Function):
         N.check(N.lib.tm_euler_zyz(N.ptr(ang), P, N.ptr(rot), N.ptr(drot), st), "tm_euler_zyz")
         sums = torch.empty((P, 6), dtype=torch.float64, device=dev)
         scores = torch.empty((P,), dtype=torch.float32, device=dev)
+        kept = None
         for lo, hi in problem.chunks(P):
             d = problem.desc(tmpl, rot, sh, cor, lo, hi)
             tf = None
             if problem.filtered:
                 tf, spec = _work(problem, hi - lo, dev)
                 _filtered_templates(problem, d, hi - lo, tf, spec)
+                if hi - lo == P and tf.numel() * 4 <= problem.keep_bytes:
+                    kept = tf
             N.check(N.lib.tm_refine_forward(N.ctypes.byref(d), N.ptr(tf), N.ptr(sums[lo:hi]),
                                             N.ptr(scores[lo:hi]), st), "tm_refine_forward")
         ctx.problem = problem
-        ctx.save_for_backward(tmpl, sh, cor, rot, drot, sums)
+        ctx.save_for_backward(tmpl, sh, cor, rot, drot, sums,
+                              kept if any(ctx.needs_input_grad) else None)
         ctx.template_shape = tuple(template.shape)
         return scores
 
     @staticmethod
     def backward(ctx, grad_scores):
         problem: RefineProblem = ctx.problem
-        tmpl, sh, cor, rot, drot, sums = ctx.saved_tensors
+        tmpl, sh, cor, rot, drot, sums, kept = ctx.saved_tensors
         P = int(sums.shape[0])
         dev = sums.device
         g = grad_scores.detach().to(dtype=torch.float32).contiguous()
@@ -282,23 +290,27 @@ class FLCRefineFunction(torch.autograd.Function):
         g_t = torch.zeros(tmpl.shape, dtype=torch.float32, device=dev) \
             if ctx.needs_input_grad[0] else None
         st = N.stream_ptr()
+        work = None if g_t is None else torch.empty((tmpl.numel(), 4), dtype=torch.float32,
+                                                    device=dev)
         for lo, hi in problem.chunks(P):
             d = problem.desc(tmpl, rot, sh, cor, lo, hi)
             tf = gbuf = None
             if problem.filtered:
-                tf, spec = _work(problem, hi - lo, dev)
-                _filtered_templates(problem, d, hi - lo, tf, spec)
-                gbuf = torch.empty_like(tf)
+                gbuf, spec = _work(problem, hi - lo, dev)
+                tf = kept
+                if tf is None:
+                    tf = torch.empty_like(gbuf)
+                    _filtered_templates(problem, d, hi - lo, tf, spec)
                 N.check(N.lib.tm_refine_grad_filtered(N.ctypes.byref(d), N.ptr(tf),
                                                       N.ptr(sums[lo:hi]), N.ptr(g[lo:hi]),
                                                       N.ptr(gbuf), st),
                         "tm_refine_grad_filtered")
                 problem.plan(hi - lo).apply(gbuf, spec, problem.template_filter)
-            N.check(N.lib.tm_refine_backward(N.ctypes.byref(d), N.ptr(tf), N.ptr(gbuf),
-                                             N.ptr(sums[lo:hi]), N.ptr(g[lo:hi]),
-                                             N.ptr(drot[lo:hi]), None, N.ptr(g_sh[lo:hi]),
-                                             N.ptr(g_ang[lo:hi]), N.ptr(g_t), st),
-                    "tm_refine_backward")
+            N.check(N.lib.tm_refine_backward_ws(N.ctypes.byref(d), N.ptr(tf), N.ptr(gbuf),
+                                                N.ptr(sums[lo:hi]), N.ptr(g[lo:hi]),
+                                                N.ptr(drot[lo:hi]), None, N.ptr(g_sh[lo:hi]),
+                                                N.ptr(g_ang[lo:hi]), N.ptr(g_t), N.ptr(work),
+                                                st), "tm_refine_backward_ws")
         gt = None if g_t is None else g_t.reshape(ctx.template_shape)
         return gt, g_ang.to(torch.float32), g_sh.to(torch.float32), None, None
 
