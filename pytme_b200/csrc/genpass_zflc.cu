@@ -11,7 +11,9 @@ namespace {
 // The thread that ends with two rows' numerators also holds their statistics. Only values of
 // one rotation share a transform: a rotation whose template normalises to NaN (an empty
 // rotated mask) leaves the others alone. Variance and quotient in double, as norm_scores
-// takes them (tme/backends/npfftw_backend.py:537-587), the quotient by rsqrt.
+// takes them (tme/backends/npfftw_backend.py:537-587), the quotient by rsqrt, for the voxels
+// that an FP32 bound does not rule out: double precision for every voxel and rotation was a
+// third of the pass's instructions.
 template <int W, typename HT>
 __global__ void __launch_bounds__(kMaxThreads, 2)
 gen_zpass_flc_kernel(const HT* __restrict__ Ht, const float2* __restrict__ Hm,
@@ -20,6 +22,7 @@ gen_zpass_flc_kernel(const HT* __restrict__ Ht, const float2* __restrict__ Hm,
                      const double* __restrict__ stats, double eps, int32_t first,
                      const int32_t* __restrict__ first_dev, float* __restrict__ state_max,
                      int32_t* __restrict__ state_rot, const HLayout ht, const HLayout hl, int zp) {
+  constexpr int kNone = 0xffff;  // no rotation of the group: groups hold at most 4096
   if (first_dev) first = *first_dev;
   extern __shared__ float4 smem_raw[];
   const int w = lines<W>(p), tid = threadIdx.x, nt = blockDim.x, l = tid % w, slot = tid / w;
@@ -48,7 +51,13 @@ gen_zpass_flc_kernel(const HT* __restrict__ Ht, const float2* __restrict__ Hm,
   // rows past the edge repeat the last one; their voxels are not stored
   const int ra = min(l, nrows - 1), rb = min(l + w, nrows - 1);
   for (int i = tid; i < p.pairs; i += nt) tw[i] = tw_g[i];
-  for (int i = tid; i < rows2 * zp; i += nt) best[i] = -INFINITY;
+  // the maxima start from the caller's state, so that few voxels of a later group improve
+  for (int rho = slot; rho < rows2; rho += p.slots)
+    for (int z = l; z < n2; z += w) {
+      best[rho * zp + z] = rho < nrows
+          ? state_max[((int64_t)(x0 + rho) * n1 + y) * n2 + z] : 1e14f;
+      arg[rho * zp + z] = kNone;
+    }
   const double eps2 = eps * eps;
   for (int b = 0; b < B; ++b) {
     if constexpr (W) async_wait_all();
@@ -87,12 +96,15 @@ gen_zpass_flc_kernel(const HT* __restrict__ Ht, const float2* __restrict__ Hm,
     }
     const double nobs = stats[b * 4 + 2];
     const double sm_n = (double)scale_m / nobs, st_n = (double)scale_t / nobs;
-    // st = (CC(f, m), CC(f^2, m)), u the numerator
-    auto update = [&](int i, float2 st, float u) {
-      const double e1 = (double)st.x * sm_n, var = (double)st.y * sm_n - e1 * e1;
-      const double inv = var >= eps2 ? rsqrt(var) : 1.0;
-      const float s = (float)((double)u * st_n * inv);
-      if (s > best[i]) { best[i] = s; arg[i] = (uint16_t)b; }
+    const float fm = (float)sm_n, ft = (float)st_n;
+    // Whether a voxel may beat its running maximum, with a margin for FP32: its score squared,
+    // (u t)^2 / var, against best^2, var from below. st = (CC(f, m), CC(f^2, m)), u the numerator.
+    auto may_beat = [&](float2 st, float u, float best) {
+      const float e1 = st.x * fm, e2 = st.y * fm, ut = u * ft;
+      const float low = fmaf(-e1, e1, e2) - 1e-6f * fmaf(e1, e1, fabsf(e2));
+      const float u2 = ut * ut * (1.f + 4e-6f);
+      const bool below = ut <= 0.f || (u2 >= 1e-30f && u2 <= best * best * low);
+      return !(best >= 0.f && best < 1e15f && below);
     };
     TM_RADIX(p.rl, ({
       for (int i = 0; i < 2; ++i)
@@ -103,25 +115,38 @@ gen_zpass_flc_kernel(const HT* __restrict__ Ht, const float2* __restrict__ Hm,
         });
       last_stage<W, RR, 1>(p, sm + 2 * tile, l, slot,
                            [&](int q, const float2(&v)[RR], float2* d) {
-        const int at = l * zp + out_base(p, q);
+        const int at = l * zp + out_base(p, q), step = n2 / RR, half = w * zp;
+        uint32_t found = 0;  // bit r: row rho's voxel r may improve, bit 16 + r: row rho + w's
         _Pragma("unroll")
         for (int r = 0; r < RR; ++r) {
-          const int i = at + r * (n2 / RR);
-          update(i, d[r * w - 2 * tile], v[r].x);
-          update(i + w * zp, d[r * w - tile], v[r].y);
+          const int i = at + r * step;
+          if (may_beat(d[r * w - 2 * tile], v[r].x, best[i])) found |= 1u << r;
+          if (may_beat(d[r * w - tile], v[r].y, best[i + half])) found |= 0x10000u << r;
         }
+        if (!found) return;
+        _Pragma("unroll")
+        for (int r = 0; r < RR; ++r) d[r * w] = v[r];
+        do {
+          const int bit = __ffs(found) - 1, r = bit & 15, second = bit >> 4;
+          found &= found - 1;
+          const int i = at + r * step + second * half;
+          const float2 st = d[r * w - (2 - second) * tile], n = d[r * w];
+          const double e1 = (double)st.x * sm_n, var = (double)st.y * sm_n - e1 * e1;
+          const double inv = var >= eps2 ? rsqrt(var) : 1.0;
+          const float s = (float)((double)(second ? n.y : n.x) * st_n * inv);
+          if (s > best[i]) { best[i] = s; arg[i] = (uint16_t)b; }
+        } while (found);
       });
     }));
   }
   __syncthreads();
   for (int rho = slot; rho < nrows; rho += p.slots)
     for (int z = l; z < n2; z += w) {
+      const int k = arg[rho * zp + z];
+      if (k == kNone) continue;
       const int64_t v = ((int64_t)(x0 + rho) * n1 + y) * n2 + z;
-      const float s = best[rho * zp + z];
-      if (s > state_max[v]) {
-        state_max[v] = s;
-        state_rot[v] = first + (int32_t)arg[rho * zp + z];
-      }
+      state_max[v] = best[rho * zp + z];
+      state_rot[v] = first + k;
     }
 }
 
