@@ -17,12 +17,13 @@ size_t even_tile(const Plan& p, int w, int tiles) {
   return 16 * p.pairs + sizeof(float2) * (((size_t)w * p.rows * tiles + 1) & ~(size_t)1);
 }
 size_t smem_y(const Plan& p, int w) { return even_tile(p, w, 1) + sizeof(float2) * w * p.n; }
-// z pass: tiles, the staged rows (not for FLC tiles of fewer lines), and per voxel of 2 w rows the maximum, its rotation and (not
+// z pass: tiles, the staged rows (for FLC see flc_staged), and per voxel of 2 w rows the maximum, its rotation and (not
 // for FLC) the inverse denominator
 size_t smem_z(const Plan& p, int w, int hp, bool flc, bool half) {
   const size_t wide = sizeof(float2) * staged_pitch<float2>(hp);
   const size_t own = half ? sizeof(__half2) * staged_pitch<__half2>(hp) : wide;
-  const size_t rows = flc ? (w == 8 ? 2 * wide + own : 0) : own;
+  const bool staged = half ? flc_staged<__half2>(w == 8) : flc_staged<float2>(w == 8);
+  const size_t rows = flc ? (staged ? 2 * wide + own : 0) : own;
   return even_tile(p, w, flc ? 3 : 1) + 2 * w * rows + 2 * (size_t)w * z_pitch(p.n) * (flc ? 6 : 10);
 }
 

@@ -54,6 +54,15 @@ __host__ __device__ constexpr int staged_pitch(int hp) {
   return hp + 16 / (int)sizeof(HT);
 }
 
+// Whether the FLC z pass stages its rows in shared memory, which costs it CTAs an SM: for
+// complex64 numerators in eight-line tiles it does (240 x 240 x 120, 32 rotations: 1.92 ms
+// against 2.04), for half2 ones and long lines it reads them in place (256 x 256 x 128 mixed, 64
+// rotations: 4.02 against 4.82).
+template <typename HT>
+__host__ __device__ constexpr bool flc_staged(bool eight_lines) {
+  return eight_lines && sizeof(HT) == sizeof(float2);
+}
+
 // Stage `nrows` rows of hp values, sx apart, w lanes and `slots` rows at a time.
 template <typename HT>
 __device__ __forceinline__ void stage_rows(HT* dst, const HT* src, int nrows, int hp, int64_t sx,

@@ -22,6 +22,7 @@ gen_zpass_flc_kernel(const HT* __restrict__ Ht, const float2* __restrict__ Hm,
                      const double* __restrict__ stats, double eps, int32_t first,
                      const int32_t* __restrict__ first_dev, float* __restrict__ state_max,
                      int32_t* __restrict__ state_rot, const HLayout ht, const HLayout hl, int zp) {
+  constexpr bool STAGED = flc_staged<HT>(W == 8);
   constexpr int kNone = 0xffff;  // no rotation of the group: groups hold at most 4096
   if (first_dev) first = *first_dev;
   extern __shared__ float4 smem_raw[];
@@ -32,11 +33,11 @@ gen_zpass_flc_kernel(const HT* __restrict__ Ht, const float2* __restrict__ Hm,
   float2* sm = reinterpret_cast<float2*>(tw + p.pairs);
   const int tile = p.rows * w;
   const int pm = staged_pitch<float2>(hp), pt = staged_pitch<HT>(hp);
-  // staged rows of Hm, of Hm2, of Ht; long lines (W = 0) are read from global memory instead
+  // staged rows of Hm, of Hm2, of Ht (or no rows: read from global memory instead)
   float2* rm = sm + ((3 * tile + 1) & ~1);
   float2* rm2 = rm + rows2 * pm;
   HT* rt = reinterpret_cast<HT*>(rm2 + rows2 * pm);
-  float* best = reinterpret_cast<float*>(W ? rt + rows2 * pt : reinterpret_cast<HT*>(rm));
+  float* best = reinterpret_cast<float*>(STAGED ? rt + rows2 * pt : reinterpret_cast<HT*>(rm));
   uint16_t* arg = reinterpret_cast<uint16_t*>(best + rows2 * zp);
   const int y = blockIdx.x, x0 = blockIdx.y * rows2, nrows = min(rows2, n0 - x0);
   const int64_t off = x0 * hl.sx + y * hl.sr, offt = x0 * ht.sx + y * ht.sr;
@@ -47,7 +48,7 @@ gen_zpass_flc_kernel(const HT* __restrict__ Ht, const float2* __restrict__ Hm,
     stage_rows<HT>(rt, Ht + offt + b * ht.sb, nrows, hp, ht.sx, l, w, slot, p.slots);
     async_commit();
   };
-  if constexpr (W) stage(0);
+  if constexpr (STAGED) stage(0);
   // rows past the edge repeat the last one; their voxels are not stored
   const int ra = min(l, nrows - 1), rb = min(l + w, nrows - 1);
   for (int i = tid; i < p.pairs; i += nt) tw[i] = tw_g[i];
@@ -60,15 +61,15 @@ gen_zpass_flc_kernel(const HT* __restrict__ Ht, const float2* __restrict__ Hm,
     }
   const double eps2 = eps * eps;
   for (int b = 0; b < B; ++b) {
-    if constexpr (W) async_wait_all();
+    if constexpr (STAGED) async_wait_all();
     __syncthreads();  // rotation b's rows are in; the tiles are free
     const int64_t o = off + b * hl.sb;
-    const float2 *ma = W ? rm + ra * pm : Hm + o + ra * hl.sx;
-    const float2 *mb = W ? rm + rb * pm : Hm + o + rb * hl.sx;
-    const float2 *sa = W ? rm2 + ra * pm : Hm2 + o + ra * hl.sx;
-    const float2 *sb = W ? rm2 + rb * pm : Hm2 + o + rb * hl.sx;
-    const HT *ta = W ? rt + ra * pt : Ht + offt + b * ht.sb + ra * ht.sx;
-    const HT *tb = W ? rt + rb * pt : Ht + offt + b * ht.sb + rb * ht.sx;
+    const float2 *ma = STAGED ? rm + ra * pm : Hm + o + ra * hl.sx;
+    const float2 *mb = STAGED ? rm + rb * pm : Hm + o + rb * hl.sx;
+    const float2 *sa = STAGED ? rm2 + ra * pm : Hm2 + o + ra * hl.sx;
+    const float2 *sb = STAGED ? rm2 + rb * pm : Hm2 + o + rb * hl.sx;
+    const HT *ta = STAGED ? rt + ra * pt : Ht + offt + b * ht.sb + ra * ht.sx;
+    const HT *tb = STAGED ? rt + rb * pt : Ht + offt + b * ht.sb + rb * ht.sx;
     TM_RADIX(p.r[0], ({
       first_stage<W, RR, 1, false>(p, sm, tw, l, slot, 0, [&](int q) {
         return [=, lr = p.lr[0]](int r) {
@@ -87,7 +88,7 @@ gen_zpass_flc_kernel(const HT* __restrict__ Ht, const float2* __restrict__ Hm,
       });
     }));
     __syncthreads();
-    if (W && b + 1 < B) stage(b + 1);
+    if (STAGED && b + 1 < B) stage(b + 1);
     for (int s = 1; s < p.ns - 1; ++s) {
       TM_RADIX(p.r[s], ({
         for (int i = 0; i < 3; ++i) mid_stage<W, RR, 1>(p, s, sm + i * tile, tw, l, slot);
