@@ -77,9 +77,12 @@ gen_xpass_kernel(const float2* __restrict__ G, const float2* __restrict__ Ft, in
 }
 
 // FLC statistics: the rotated mask's spectrum times the spectra of f and f^2, two inverse
-// transforms of one forward transform.
+// transforms of one forward transform. Issue and latency bound like the x pass, and the last
+// forward stage holds two butterflies: bounding the block at 512 threads leaves a thread the
+// 128 registers that the slots are chosen for (168 without, and a CTA less on an SM: x pass
+// of 64 rotations at 256 x 256 x 128 3.96 -> 3.62 ms, of 32 at 240 x 240 x 120 1.51 -> 1.38).
 template <int W>
-__global__ void __launch_bounds__(kMaxThreads, 1)
+__global__ void __launch_bounds__(512, 1)
 gen_xstat_kernel(const float2* __restrict__ Gm, const float2* __restrict__ Ft,
                  const float2* __restrict__ Ft2, int B, int per, int t0, int n1, int h2,
                  const Plan p, const float4* __restrict__ tw_g, float scale,
