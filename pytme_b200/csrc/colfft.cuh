@@ -29,7 +29,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 
-#include "fft_smem.cuh"
+#include "dft.cuh"
 
 namespace tmb {
 namespace colfft {

@@ -1,20 +1,6 @@
-// Batched 1D complex FFTs of lines held in shared memory (Stockham autosort).
-//
-// A CTA transforms `nlines` lines of length n in place. Element i of line l
-// lives at buf[l * ls + i * es], so both "interleaved" tiles (lines fastest,
-// es = nlines, ls = 1) and "row-major" tiles (es = 1) are supported. Each pass
-// of radix R loads R elements per butterfly into registers, applies the
-// twiddles, runs an R-point DFT and, after a barrier, stores the outputs in
-// autosorted order, so one buffer suffices. The number of butterflies per
-// thread per pass is bounded at compile time (MAXE / R); launches keep
-// n * nlines <= MAXE * nthreads.
-//
-// The compile-time small DFTs at the end are also the butterflies of linefft.cuh and of the
-// scan's four-step z pass.
-//
-// Twiddles come from a table tw[i] = exp(-2 pi i * i / N) in shared memory,
-// computed on the host in double precision and rounded to float; a line of
-// length n with n | N reads it with stride N / n.
+// Complex arithmetic and the small DFTs in registers that every own transform is built from:
+// the columns of colfft.cuh, the line FFTs of linefft.cuh, the Stockham passes of
+// mixed-precision plans and the scan's four-step z pass.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -22,14 +8,6 @@
 
 namespace tmb {
 namespace fft {
-
-constexpr int kMaxPasses = 12;
-
-struct LinePlan {
-  int n;                    // transform length
-  int npass;                // number of radix passes
-  int radix[kMaxPasses];    // radices, first pass first
-};
 
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
@@ -43,12 +21,6 @@ __device__ __forceinline__ float2 cscale(float2 a, float s) { return make_float2
 template <int DIR>
 __device__ __forceinline__ float2 rot90(float2 a) {
   return DIR < 0 ? make_float2(a.y, -a.x) : make_float2(-a.y, a.x);
-}
-
-template <int DIR>
-__device__ __forceinline__ float2 twiddle(const float2* tw, int idx) {
-  float2 w = tw[idx];
-  return DIR < 0 ? w : cconj(w);
 }
 
 // ---- small DFTs in registers; DIR = -1 computes sum_j v_j exp(-2 pi i jk/R)
@@ -124,104 +96,6 @@ __device__ __forceinline__ void dft8(float2* v) {
   for (int k = 0; k < 4; ++k) {
     v[k] = cadd(e[k], o[k]);
     v[k + 4] = csub(e[k], o[k]);
-  }
-}
-
-// Generic odd radix (7, 11, 13): direct DFT with roots of unity read from the
-// twiddle table; tw_r(k) = exp(-2 pi i k / R) sits at table index k * N / R.
-template <int R, int DIR>
-__device__ __forceinline__ void dft_generic(float2* v, const float2* tw, int root_stride) {
-  float2 out[R];
-#pragma unroll
-  for (int k = 0; k < R; ++k) {
-    float2 acc = v[0];
-#pragma unroll
-    for (int j = 1; j < R; ++j) {
-      int e = (j * k) % R;
-      acc = cadd(acc, cmul(v[j], twiddle<DIR>(tw, e * root_stride)));
-    }
-    out[k] = acc;
-  }
-#pragma unroll
-  for (int k = 0; k < R; ++k) v[k] = out[k];
-}
-
-template <int R, int DIR>
-__device__ __forceinline__ void dft(float2* v, const float2* tw, int table_n) {
-  if constexpr (R == 2) dft2<DIR>(v);
-  else if constexpr (R == 3) dft3<DIR>(v);
-  else if constexpr (R == 4) dft4<DIR>(v);
-  else if constexpr (R == 5) dft5<DIR>(v);
-  else if constexpr (R == 8) dft8<DIR>(v);
-  else dft_generic<R, DIR>(v, tw, table_n / R);
-}
-
-// One Stockham pass of radix R over all lines.
-//   Ns: product of the radices of earlier passes.
-//   tws: table stride for this line length (table_n / n).
-template <int R, int DIR, int MAXE, bool LINES_FAST>
-__device__ __forceinline__ void stockham_pass(float2* buf, int n, int Ns, int nlines, int ls,
-                                              int es, const float2* tw, int tws, int table_n,
-                                              int tid, int nthr) {
-  constexpr int MAXB = (MAXE + R - 1) / R;
-  const int nb = n / R;
-  const int total = nb * nlines;
-  const int tstep = (n / (Ns * R)) * tws;
-  float2 v[MAXB][R];
-#pragma unroll
-  for (int c = 0; c < MAXB; ++c) {
-    int w = tid + c * nthr;
-    if (w < total) {
-      int l, j;
-      if (LINES_FAST) { l = w % nlines; j = w / nlines; } else { j = w % nb; l = w / nb; }
-      const float2* base = buf + l * ls;
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[c][r] = base[(j + r * nb) * es];
-      int k = j % Ns;
-      if (k != 0) {
-#pragma unroll
-        for (int r = 1; r < R; ++r) v[c][r] = cmul(v[c][r], twiddle<DIR>(tw, r * k * tstep));
-      }
-      dft<R, DIR>(v[c], tw, table_n);
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int c = 0; c < MAXB; ++c) {
-    int w = tid + c * nthr;
-    if (w < total) {
-      int l, j;
-      if (LINES_FAST) { l = w % nlines; j = w / nlines; } else { j = w % nb; l = w / nb; }
-      float2* base = buf + l * ls;
-      int k = j % Ns;
-      int o = (j / Ns) * Ns * R + k;
-#pragma unroll
-      for (int r = 0; r < R; ++r) base[(o + r * Ns) * es] = v[c][r];
-    }
-  }
-  __syncthreads();
-}
-
-// Full transform of all lines: runs the plan's passes. Callers must
-// __syncthreads() before (data loaded) — the routine ends synchronised.
-// Radices 2, 3, 4, 5 and 8 are compiled in (every 5-smooth length); plans with
-// other radices are rejected on the host (supported_radices).
-template <int DIR, int MAXE, bool LINES_FAST>
-__device__ __forceinline__ void fft_lines(float2* buf, const LinePlan& p, int nlines, int ls, int es,
-                          const float2* tw, int table_n, int tid, int nthr) {
-  const int tws = table_n / p.n;
-  int Ns = 1;
-  for (int s = 0; s < p.npass; ++s) {
-    const int R = p.radix[s];
-    switch (R) {
-      case 8: stockham_pass<8, DIR, MAXE, LINES_FAST>(buf, p.n, Ns, nlines, ls, es, tw, tws, table_n, tid, nthr); break;
-      case 4: stockham_pass<4, DIR, MAXE, LINES_FAST>(buf, p.n, Ns, nlines, ls, es, tw, tws, table_n, tid, nthr); break;
-      case 2: stockham_pass<2, DIR, MAXE, LINES_FAST>(buf, p.n, Ns, nlines, ls, es, tw, tws, table_n, tid, nthr); break;
-      case 3: stockham_pass<3, DIR, MAXE, LINES_FAST>(buf, p.n, Ns, nlines, ls, es, tw, tws, table_n, tid, nthr); break;
-      case 5: stockham_pass<5, DIR, MAXE, LINES_FAST>(buf, p.n, Ns, nlines, ls, es, tw, tws, table_n, tid, nthr); break;
-      default: break;
-    }
-    Ns *= R;
   }
 }
 

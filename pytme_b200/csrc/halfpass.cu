@@ -7,8 +7,8 @@
 // bit for bit; FP32 plans, and what a mixed plan keeps in FP32 (the FLC statistics), take the
 // line FFTs of genpass.cuh.
 //
-// Power-of-two axes use the register-resident columns of colfft.cuh, other 5-smooth ones the
-// shared-memory Stockham of fft_smem.cuh.
+// Power-of-two axes use the register-resident columns of colfft.cuh, other 5-smooth ones a
+// shared-memory Stockham transform.
 #include "halfpass.cuh"
 
 #include <cuda_fp16.h>
@@ -19,31 +19,11 @@
 
 #include "colfft.cuh"
 #include "common.cuh"
-#include "fft_smem.cuh"
+#include "dft.cuh"
 
 namespace tmb {
 
-using fft::LinePlan;
-
 namespace {
-
-LinePlan make_line_plan(int n) {
-  LinePlan p{};
-  p.n = n;
-  int m = n, e2 = 0;
-  while (m % 2 == 0) { m /= 2; ++e2; }
-  int k = 0;
-  int eights = e2 / 3, rem = e2 % 3;
-  if (rem == 1 && eights > 0) { eights -= 1; p.radix[k++] = 4; p.radix[k++] = 4; }
-  else if (rem == 1) { p.radix[k++] = 2; }
-  else if (rem == 2) { p.radix[k++] = 4; }
-  for (int i = 0; i < eights; ++i) p.radix[k++] = 8;
-  for (int q : {3, 5, 7, 11, 13}) {
-    while (m % q == 0) { m /= q; p.radix[k++] = q; }
-  }
-  p.npass = (m == 1) ? k : -1;
-  return p;
-}
 
 // ------------------------------------------------------------------ storage types
 template <typename T> struct Store;
@@ -62,7 +42,9 @@ template <> struct Store<__half2> {
 template <int BYTES>
 __device__ __forceinline__ void cp_async(void* smem, const void* gmem) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  if constexpr (BYTES == 4)
+  if constexpr (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
+  else if constexpr (BYTES == 4)
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem));
   else
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem));
@@ -73,134 +55,339 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(PENDING));
 }
 
-constexpr int kThreads = 512;
-constexpr int kMaxE = 8;             // complex elements per thread in a line-FFT tile
-constexpr int kTile = kThreads * kMaxE;  // elements per tile (4096)
+// ------------------------------------------------------------------ Stockham passes
+// Lines of 5-smooth lengths, 2^lw neighbouring k2 interleaved: element i of line l at
+// (i << lw) + l. A stage of radix R reads inputs j + r * n / R of butterfly j, applies the
+// twiddles of k = j mod Ns (Ns: the product of the radices before) and writes outputs
+// (j / Ns) * Ns * R + k + r * Ns, from one of two tiles to the other, so a stage ends with one
+// barrier. The first stage reads its inputs, and the last of an inverse transform writes its
+// outputs, wherever the pass has them. The order of the radices, the twiddles and every
+// operation fix the bits of a plan's results; lines, tiles and threads do not.
+//
+// Bound by instruction issue and shared-memory latency. Lines are a power of two and j / Ns is
+// a multiplication: with as many lines as fit 4096 elements and divisions by their number, one
+// CTA of 512 threads an SM and two barriers a stage, the passes of 32 rotations at 160^3 (24^3
+// template, mixed) took @X0@ (x) and @Y0@ us (y), now @X1@ and @Y1@.
+constexpr int kMaxThreads = 512;
+
+// The operations as they round: which product of a sum is fused is written out, as it
+// otherwise depends on the code around.
+__device__ __forceinline__ float2 turn(float2 a, float2 w) {  // a * w, forward twiddles
+  return make_float2(__fmaf_rn(a.x, w.x, -__fmul_rn(a.y, w.y)),
+                     __fmaf_rn(a.y, w.x, __fmul_rn(a.x, w.y)));
+}
+__device__ __forceinline__ float2 turn_back(float2 a, float2 w) {  // a * conj(w)
+  return make_float2(__fmaf_rn(a.x, w.x, __fmul_rn(a.y, w.y)),
+                     __fmaf_rn(a.y, w.x, -__fmul_rn(a.x, w.y)));
+}
+__device__ __forceinline__ float2 filter(float2 a, float2 f) {  // a * f, the target
+  return make_float2(__fmaf_rn(a.x, f.x, -__fmul_rn(a.y, f.y)),
+                     __fmaf_rn(a.x, f.y, __fmul_rn(a.y, f.x)));
+}
+__device__ __forceinline__ float2 axpy(float s, float2 x, float2 y) {
+  return make_float2(__fmaf_rn(s, x.x, y.x), __fmaf_rn(s, x.y, y.y));
+}
+
+template <int R, int DIR>
+__device__ __forceinline__ void butterfly(float2* v) {
+  using fft::cadd;
+  using fft::csub;
+  using fft::rot90;
+  if constexpr (R == 3) {
+    const float s = (DIR < 0 ? -1.f : 1.f) * 0.86602540378443864676f;
+    const float2 t = cadd(v[1], v[2]), d = rot90<1>(csub(v[1], v[2]));
+    const float2 m = axpy(-0.5f, t, v[0]);
+    v[0] = cadd(v[0], t);
+    v[1] = axpy(s, d, m);
+    v[2] = axpy(-s, d, m);
+  } else if constexpr (R == 5) {
+    const float c1 = 0.30901699437494742410f, c2 = -0.80901699437494742410f;
+    const float sg = DIR < 0 ? -1.f : 1.f;
+    const float s1 = sg * 0.95105651629515357212f, s2 = sg * 0.58778525229247312917f;
+    const float2 a1 = cadd(v[1], v[4]), b1 = rot90<1>(csub(v[1], v[4]));
+    const float2 a2 = cadd(v[2], v[3]), b2 = rot90<1>(csub(v[2], v[3]));
+    const float2 m1 = axpy(c2, a2, axpy(c1, a1, v[0])), m2 = axpy(c1, a2, axpy(c2, a1, v[0]));
+    const float2 n1 = axpy(s1, b1, make_float2(__fmul_rn(s2, b2.x), __fmul_rn(s2, b2.y)));
+    const float2 n2 = axpy(s2, b1, make_float2(-__fmul_rn(s1, b2.x), -__fmul_rn(s1, b2.y)));
+    v[0] = cadd(cadd(v[0], a1), a2);
+    v[1] = cadd(m1, n1);
+    v[4] = csub(m1, n1);
+    v[2] = cadd(m2, n2);
+    v[3] = csub(m2, n2);
+  } else if constexpr (R == 8) {
+    const float h = 0.70710678118654752440f;
+    float2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+    fft::dft4<DIR>(e);
+    fft::dft4<DIR>(o);
+    // o[k] *= exp(DIR * 2 pi i k / 8), the factor h of odd k in the sums
+    o[1] = cadd(o[1], rot90<DIR>(o[1]));
+    o[2] = rot90<DIR>(o[2]);
+    o[3] = csub(rot90<DIR>(o[3]), o[3]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      v[k] = k % 2 ? axpy(h, o[k], e[k]) : cadd(e[k], o[k]);
+      v[k + 4] = k % 2 ? axpy(-h, o[k], e[k]) : csub(e[k], o[k]);
+    }
+  } else {
+    fft::dft_small<R, DIR>(v);  // 1, 2 and 4 only add
+  }
+}
+
+template <int R, int DIR, bool FIRST, class In, class Out>
+__device__ __forceinline__ void stage(const HalfLine& p, int s, const float2* tw, int slot, In in,
+                                      Out out) {
+  const int nb = p.n / R, ns = p.before[s];
+  for (int j = slot; j < nb; j += p.slots) {
+    float2 v[R];
+    auto load = in(j);
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = load(r);
+    int o = j * R;
+    if constexpr (!FIRST) {
+      const int q = __umulhi(j, p.recip[s]), k = j - q * ns;
+      o = q * (ns * R) + k;
+      if (k != 0) {
+        const int step = k * p.step[s];
+#pragma unroll
+        for (int r = 1; r < R; ++r) {
+          const float2 w = tw[r * step];
+          v[r] = DIR < 0 ? turn(v[r], w) : turn_back(v[r], w);
+        }
+      }
+    }
+    butterfly<R, DIR>(v);
+    auto store = out(o);
+#pragma unroll
+    for (int r = 0; r < R; ++r) store(r, v[r]);
+  }
+}
+
+// The radices of a plan's stages (1: the copy that ends a one-stage transform).
+#define TM_STAGE(R, CALL)                            \
+  do {                                               \
+    switch (R) {                                     \
+      case 8: { constexpr int RR = 8; CALL; } break; \
+      case 4: { constexpr int RR = 4; CALL; } break; \
+      case 2: { constexpr int RR = 2; CALL; } break; \
+      case 3: { constexpr int RR = 3; CALL; } break; \
+      case 5: { constexpr int RR = 5; CALL; } break; \
+      default: { constexpr int RR = 1; CALL; } break; \
+    }                                                \
+  } while (0)
+
+// Inputs and outputs of butterflies of radix R in a tile.
+template <int R>
+__device__ __forceinline__ auto tile_in(const HalfLine& p, const float2* t, int l) {
+  return [=, step = (p.n / R) << p.lw, lw = p.lw](int j) {
+    return [a = t + (j << lw) + l, step](int r) { return a[r * step]; };
+  };
+}
+__device__ __forceinline__ auto tile_out(const HalfLine& p, int s, float2* t, int l) {
+  return [=, step = p.before[s] << p.lw, lw = p.lw](int o) {
+    return [a = t + (o << lw) + l, step](int r, float2 v) { a[r * step] = v; };
+  };
+}
+
+// Stages [1, last) from the tile at `a` to the one at `b` and back; a is left at the outputs.
+template <int DIR>
+__device__ __forceinline__ void tile_stages(const HalfLine& p, int last, float2*& a, float2*& b,
+                                            const float2* tw, int slot, int l) {
+  for (int s = 1; s < last; ++s) {
+    TM_STAGE(p.radix[s], (stage<RR, DIR, false>(p, s, tw, slot, tile_in<RR>(p, a, l),
+                                                tile_out(p, s, b, l))));
+    __syncthreads();
+    float2* t = a;
+    a = b;
+    b = t;
+  }
+}
 
 // ------------------------------------------------------------------ K1: template z/y
-// grid (ceil(h2/W), t0, B); tile: n1 lines-fast rows x W lines (k2).
-__global__ void __launch_bounds__(kThreads, 1)
-tmpl_zy_kernel(const float* __restrict__ tmpl, int t0, int t1, int t2, int n1, int n2, int h2,
-               int W, LinePlan p1, const float2* __restrict__ tw1_g, const float2* __restrict__ tw2_g,
-               float2* __restrict__ G) {
+// grid (ceil(h2 / lines), t0, B). A template plane too large for shared memory stays where it
+// is (wide = false).
+__global__ void __launch_bounds__(kMaxThreads, 2)
+tmpl_zy_kernel(const float* __restrict__ tmpl, int t0, int t1, int t2, int n2, int h2, bool wide,
+               const HalfLine p, const float2* __restrict__ tw1_g,
+               const float2* __restrict__ tw2_g, float2* __restrict__ G) {
   extern __shared__ float4 smem_raw[];
+  const int w = 1 << p.lw, tid = threadIdx.x, nt = blockDim.x;
+  const int l = tid & (w - 1), slot = tid >> p.lw;
   float2* tw1 = reinterpret_cast<float2*>(smem_raw);
-  float2* tw2 = tw1 + n1;
-  float2* buf = tw2 + n2;
-  float* plane = reinterpret_cast<float*>(buf + (int64_t)n1 * W);
-  const int tid = threadIdx.x;
-  const int k2_0 = blockIdx.x * W;
-  const int x = blockIdx.y;
-  const int b = blockIdx.z;
-  for (int i = tid; i < n1; i += kThreads) tw1[i] = tw1_g[i];
-  for (int i = tid; i < n2; i += kThreads) tw2[i] = tw2_g[i];
-  const float* src = tmpl + ((int64_t)b * t0 + x) * t1 * t2;
-  for (int i = tid; i < t1 * t2; i += kThreads) plane[i] = src[i];
+  float2* tw2 = tw1 + p.n;
+  float2* a = tw2 + n2;
+  float2* b = a + (p.n << p.lw);
+  float* staged = reinterpret_cast<float*>(b + (p.n << p.lw));
+  const int k2 = blockIdx.x * w + l;
+  const bool valid = k2 < h2;
+  for (int i = tid; i < p.n; i += nt) tw1[i] = tw1_g[i];
+  for (int i = tid; i < n2; i += nt) tw2[i] = tw2_g[i];
+  const float* src = tmpl + ((int64_t)blockIdx.z * t0 + blockIdx.y) * t1 * t2;
+  if (wide)
+    for (int i = tid; i < t1 * t2; i += nt) staged[i] = src[i];
+  const float* plane = wide ? staged : src;
   __syncthreads();
-  // G1[y][k2] = sum_z plane[y][z] * exp(-2 pi i z k2 / n2), rows y >= t1 are zero
-  for (int e = tid; e < n1 * W; e += kThreads) {
-    int y = e / W, l = e % W;
-    int k2 = k2_0 + l;
+  // rows[y][k2] = sum_z plane[y][z] * exp(-2 pi i z k2 / n2); rows y >= t1 are zero
+  for (int y = slot; y < t1; y += p.slots) {
     float2 acc = make_float2(0.f, 0.f);
-    if (y < t1 && k2 < h2) {
+    if (valid) {
       const float* row = plane + y * t2;
       int idx = 0;
       for (int z = 0; z < t2; ++z) {
-        float v = row[z];
-        float2 w = tw2[idx];
-        acc.x += v * w.x;
-        acc.y += v * w.y;
+        const float v = row[z];
+        const float2 c = tw2[idx];
+        acc.x += v * c.x;
+        acc.y += v * c.y;
         idx += k2;
         if (idx >= n2) idx -= n2;
       }
     }
-    buf[e] = acc;
+    b[(y << p.lw) + l] = acc;
   }
   __syncthreads();
-  fft::fft_lines<-1, kMaxE, true>(buf, p1, W, 1, W, tw1, n1, tid, kThreads);
-  float2* dst = G + ((int64_t)b * t0 + x) * n1 * h2;
-  for (int e = tid; e < n1 * W; e += kThreads) {
-    int k1 = e / W, l = e % W;
-    int k2 = k2_0 + l;
-    if (k2 < h2) dst[(int64_t)k1 * h2 + k2] = buf[e];
-  }
+  TM_STAGE(p.radix[0], (stage<RR, -1, true>(p, 0, tw1, slot, [&](int j) {
+    return [&, j](int r) {
+      const int y = j + r * (p.n / RR);
+      return y < t1 ? b[(y << p.lw) + l] : make_float2(0.f, 0.f);
+    };
+  }, tile_out(p, 0, a, l))));
+  __syncthreads();
+  tile_stages<-1>(p, p.stages - 1, a, b, tw1, slot, l);
+  float2* dst = G + ((int64_t)blockIdx.z * t0 + blockIdx.y) * p.n * h2 + k2;
+  const int s = p.stages - 1;
+  TM_STAGE(p.radix[s], (stage<RR, -1, false>(p, s, tw1, slot, tile_in<RR>(p, a, l), [&](int o) {
+    return [d = dst + (int64_t)o * h2, step = (int64_t)p.before[s] * h2, valid](int r, float2 v) {
+      if (valid) d[r * step] = v;
+    };
+  })));
 }
 
 // ------------------------------------------------------------------ K2: x pass
-// grid (ceil(h2/W), n1); loops over the B rotations of the group.
-template <typename HT>
-__global__ void __launch_bounds__(kThreads, 1)
-xpass_kernel(const float2* __restrict__ G, const float2* __restrict__ Ft, int B, int t0, int n0,
-             int n1, int h2, int W, LinePlan p0, const float2* __restrict__ tw0_g, float scale,
-             HT* __restrict__ H, int hp) {
+// grid (ceil(h2 / lines), n1, rotation chunks). The target's column times the scale of H stays
+// in shared memory for all rotations of a chunk; the next rotation's inputs are copied in while
+// the current one is transformed.
+__global__ void __launch_bounds__(kMaxThreads, 2)
+xpass_kernel(const float2* __restrict__ G, const float2* __restrict__ Ft, int B, int per, int t0,
+             int n1, int h2, const HalfLine p, const float2* __restrict__ tw0_g, float scale,
+             __half2* __restrict__ H, int hp) {
   extern __shared__ float4 smem_raw[];
-  float2* tw0 = reinterpret_cast<float2*>(smem_raw);
-  float2* buf = tw0 + n0;
-  const int tid = threadIdx.x;
-  const int k2_0 = blockIdx.x * W;
-  const int k1 = blockIdx.y;
-  for (int i = tid; i < n0; i += kThreads) tw0[i] = tw0_g[i];
-  const int tile = n0 * W;
-  // target-spectrum tile: re-read through L1 for every rotation of the group
-  const float2* ft_col = Ft + (int64_t)k1 * h2 + k2_0;
-  const int64_t ft_row = (int64_t)n1 * h2;
-  const int64_t SH = (int64_t)n0 * n1 * hp;
-  for (int b = 0; b < B; ++b) {
-    const float2* g = G + (int64_t)b * t0 * n1 * h2;
-    for (int e = tid; e < tile; e += kThreads) {
-      int x = e / W, l = e % W;
-      int k2 = k2_0 + l;
-      float2 v = make_float2(0.f, 0.f);
-      if (x < t0 && k2 < h2) v = g[((int64_t)x * n1 + k1) * h2 + k2];
-      buf[e] = v;
+  const int w = 1 << p.lw, tid = threadIdx.x, nt = blockDim.x;
+  const int l = tid & (w - 1), slot = tid >> p.lw;
+  const int tile = p.n << p.lw;
+  float2* tw = reinterpret_cast<float2*>(smem_raw);
+  float2* ft = tw + p.n;
+  float2* a = ft + tile;
+  float2* b = a + tile;
+  float2* staged = b + tile;  // t0 rows
+  const int k2 = blockIdx.x * w + l, k1 = blockIdx.y;
+  const bool valid = k2 < h2;
+  const int64_t row = (int64_t)n1 * h2;
+  const float2* g = G + (int64_t)k1 * h2 + k2;
+  const int b0 = blockIdx.z * per, b1 = min(B, b0 + per);
+  auto fetch = [&](int rot) {
+    if (valid) {
+      const float2* src = g + ((int64_t)rot * t0 + slot) * row;
+      for (int x = slot; x < t0; x += p.slots, src += p.slots * row)
+        cp_async<8>(staged + (x << p.lw) + l, src);
     }
+    cp_async_commit();
+  };
+  fetch(b0);
+  if (!valid)
+    for (int x = slot; x < t0; x += p.slots) staged[(x << p.lw) + l] = make_float2(0.f, 0.f);
+  for (int i = tid; i < p.n; i += nt) tw[i] = tw0_g[i];
+  const float2* f_col = Ft + (int64_t)k1 * h2 + k2;
+  for (int x = slot; x < p.n; x += p.slots) {
+    const float2 f = valid ? __ldg(f_col + x * row) : make_float2(0.f, 0.f);
+    ft[(x << p.lw) + l] = make_float2(f.x * scale, f.y * scale);
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+  const int last = p.stages - 1;
+  const int64_t out_row = (int64_t)n1 * hp, SH = out_row * p.n;
+  for (int rot = b0; rot < b1; ++rot) {
+    TM_STAGE(p.radix[0], (stage<RR, -1, true>(p, 0, tw, slot, [&](int j) {
+      return [&, j](int r) {
+        const int x = j + r * (p.n / RR);
+        return x < t0 ? staged[(x << p.lw) + l] : make_float2(0.f, 0.f);
+      };
+    }, tile_out(p, 0, b, l))));
     __syncthreads();
-    fft::fft_lines<-1, kMaxE, true>(buf, p0, W, 1, W, tw0, n0, tid, kThreads);
-    for (int e = tid; e < tile; e += kThreads) {
-      int k0 = e / W, l = e % W;
-      float2 f = make_float2(0.f, 0.f);
-      if (k2_0 + l < h2) f = __ldg(ft_col + k0 * ft_row + l);
-      buf[e] = fft::cmul(buf[e], make_float2(f.x * scale, f.y * scale));
-    }
+    if (rot + 1 < b1) fetch(rot + 1);
+    tile_stages<-1>(p, p.stages, b, a, tw, slot, l);
+    TM_STAGE(p.radix[0], (stage<RR, 1, true>(p, 0, tw, slot, [&](int j) {
+      const int step = (p.n / RR) << p.lw;
+      return [c = b + (j << p.lw) + l, f = ft + (j << p.lw) + l, step](int r) {
+        return filter(c[r * step], f[r * step]);
+      };
+    }, tile_out(p, 0, a, l))));
+    cp_async_wait<0>();  // the next inputs, for every thread after the barrier
     __syncthreads();
-    fft::fft_lines<1, kMaxE, true>(buf, p0, W, 1, W, tw0, n0, tid, kThreads);
-    HT* h = H + (int64_t)b * SH;
-    for (int e = tid; e < tile; e += kThreads) {
-      int x = e / W, l = e % W;
-      int k2 = k2_0 + l;
-      if (k2 < h2) Store<HT>::store(h + ((int64_t)x * n1 + k1) * hp + k2, buf[e]);
-    }
-    __syncthreads();
+    tile_stages<1>(p, last, a, b, tw, slot, l);
+    // the next rotation's first stage writes the tile that this stage does not read
+    __half2* h = H + rot * SH + (int64_t)k1 * hp + k2;
+    TM_STAGE(p.radix[last], (stage<RR, 1, false>(p, last, tw, slot, tile_in<RR>(p, a, l),
+                                                 [&](int o) {
+      return [d = h + o * out_row, step = p.before[last] * out_row, valid](int r, float2 v) {
+        if (valid) Store<__half2>::store(d + r * step, v);
+      };
+    })));
   }
 }
 
 // ------------------------------------------------------------------ K3: y pass
-// grid (ceil(h2/W), n0, B): inverse FFT along axis 1, in place.
-template <typename HT>
-__global__ void __launch_bounds__(kThreads, 1)
-ypass_kernel(HT* __restrict__ H, int n0, int n1, int h2, int W, LinePlan p1,
+// grid (ceil(h2 / lines), ceil(n0 / planes), B): inverse FFT along axis 1, in place; the next
+// plane's columns are copied to shared memory while the current one is transformed.
+__global__ void __launch_bounds__(kMaxThreads, 2)
+ypass_kernel(__half2* __restrict__ H, int planes, int n0, int h2, const HalfLine p,
              const float2* __restrict__ tw1_g, int hp) {
   extern __shared__ float4 smem_raw[];
-  float2* tw1 = reinterpret_cast<float2*>(smem_raw);
-  float2* buf = tw1 + n1;
-  const int tid = threadIdx.x;
-  const int k2_0 = blockIdx.x * W;
-  const int x = blockIdx.y;
-  const int b = blockIdx.z;
-  for (int i = tid; i < n1; i += kThreads) tw1[i] = tw1_g[i];
-  const int tile = n1 * W;
-  HT* h = H + (int64_t)b * n0 * n1 * hp + (int64_t)x * n1 * hp;
-  for (int e = tid; e < tile; e += kThreads) {
-    int y = e / W, l = e % W;
-    int k2 = k2_0 + l;
-    buf[e] = (k2 < h2) ? Store<HT>::load(h + (int64_t)y * hp + k2) : make_float2(0.f, 0.f);
-  }
-  __syncthreads();
-  fft::fft_lines<1, kMaxE, true>(buf, p1, W, 1, W, tw1, n1, tid, kThreads);
-  for (int e = tid; e < tile; e += kThreads) {
-    int y = e / W, l = e % W;
-    int k2 = k2_0 + l;
-    if (k2 < h2) Store<HT>::store(h + (int64_t)y * hp + k2, buf[e]);
+  const int w = 1 << p.lw, tid = threadIdx.x, nt = blockDim.x;
+  const int l = tid & (w - 1), slot = tid >> p.lw;
+  const int tile = p.n << p.lw;
+  float2* a = reinterpret_cast<float2*>(smem_raw);
+  float2* b = a + tile;
+  __half2* staged = reinterpret_cast<__half2*>(b + tile);
+  float2* tw = reinterpret_cast<float2*>(staged + ((tile + 1) & ~1));
+  const int k2_0 = blockIdx.x * w, k2 = k2_0 + l;
+  const bool valid = k2 < h2;
+  const int x0 = blockIdx.y * planes, x1 = min(n0, x0 + planes);
+  const int64_t plane = (int64_t)p.n * hp;
+  __half2* base = H + ((int64_t)blockIdx.z * n0 + x0) * plane;
+  auto fetch = [&](const __half2* src) {
+    if (p.lw >= 2) {  // four values of a row at a time
+      const int lp = p.lw - 2, k = (tid & ((1 << lp) - 1)) * 4;
+      if (k2_0 + k < hp)
+        for (int y = tid >> lp; y < p.n; y += nt >> lp)
+          cp_async<16>(staged + (y << p.lw) + k, src + (int64_t)y * hp + k2_0 + k);
+    } else if (valid) {
+      for (int y = slot; y < p.n; y += p.slots)
+        cp_async<4>(staged + (y << p.lw) + l, src + (int64_t)y * hp + k2);
+    }
+    cp_async_commit();
+  };
+  fetch(base);
+  for (int i = tid; i < p.n; i += nt) tw[i] = tw1_g[i];
+  const int last = p.stages - 1;
+  for (int x = x0; x < x1; ++x, base += plane) {
+    cp_async_wait<0>();
+    __syncthreads();  // plane x is in
+    TM_STAGE(p.radix[0], (stage<RR, 1, true>(p, 0, tw, slot, [&](int j) {
+      const int step = (p.n / RR) << p.lw;
+      return [c = staged + (j << p.lw) + l, step, valid](int r) {
+        return valid ? __half22float2(c[r * step]) : make_float2(0.f, 0.f);
+      };
+    }, tile_out(p, 0, a, l))));
+    __syncthreads();
+    if (x + 1 < x1) fetch(base + plane);
+    tile_stages<1>(p, last, a, b, tw, slot, l);
+    __half2* h = base + k2;
+    TM_STAGE(p.radix[last], (stage<RR, 1, false>(p, last, tw, slot, tile_in<RR>(p, a, l),
+                                                 [&](int o) {
+      return [d = h + (int64_t)o * hp, step = (int64_t)p.before[last] * hp, valid](int r,
+                                                                                   float2 v) {
+        if (valid) Store<__half2>::store(d + r * step, v);
+      };
+    })));
   }
 }
 
@@ -511,17 +698,79 @@ int raise(K kernel) {
 
 }  // namespace
 
-HalfConfig half_config(int n0, int n1, int n2, int h2, int t1, int t2) {
+// Plan of a line of length n: radices in the order that fixes the bits, then lines and slots.
+// Sixteen lines where three CTAs of them fit an SM (64 bytes of half2 a row), else the most,
+// up to eight, that fit; slots with few idle lanes over the stages and enough warps on an SM.
+template <class Size>
+static HalfLine half_line(int n, int h2, Size size) {
+  HalfLine p;
+  p.n = n;
+  int m = n, e2 = 0;
+  while (m % 2 == 0) { m /= 2; ++e2; }
+  int eights = e2 / 3;
+  const int rem = e2 % 3;
+  if (rem == 1 && eights > 0) {
+    eights -= 1;
+    p.radix[p.stages++] = 4;
+    p.radix[p.stages++] = 4;
+  } else if (rem) {
+    p.radix[p.stages++] = 1 << rem;
+  }
+  for (int i = 0; i < eights; ++i) p.radix[p.stages++] = 8;
+  for (int q : {3, 5})
+    for (; m % q == 0; m /= q) p.radix[p.stages++] = q;
+  while (p.stages < 2) p.radix[p.stages++] = 1;
+  int before = 1;
+  for (int s = 0; s < p.stages; ++s) {
+    p.before[s] = before;
+    p.recip[s] = (unsigned)((((uint64_t)1 << 32) + before - 1) / before);
+    before *= p.radix[s];
+    p.step[s] = n / before;
+  }
+  const size_t sm = 227 * 1024, own = 1024;
+  for (p.lw = 4; p.lw > 0; --p.lw) {
+    if (p.lw > 2 && 1 << (p.lw - 1) >= h2) continue;
+    if (size(p) <= (p.lw == 4 ? sm / 3 - own : sm - own)) break;
+  }
+  double most = 0;
+  for (int threads = 32; threads <= kMaxThreads; threads += 32) {
+    const int slots = threads >> p.lw;
+    double spent = 0, work = 0;
+    for (int s = 0; s < p.stages; ++s) {
+      const int nb = n / p.radix[s];
+      spent += (double)ceil_div(nb, slots) * slots * (p.radix[s] + 2);
+      work += (double)nb * (p.radix[s] + 2);
+    }
+    const int ctas = (int)std::min<size_t>(std::min<size_t>(32, sm / (size(p) + own)),
+                                           1024 / threads);
+    const double rate = work / spent * std::min(1.0, (ctas * threads / 32.0 + 4) / 24);
+    if (rate > most * 1.01) { most = rate; p.slots = slots; }
+  }
+  return p;
+}
+
+HalfConfig half_config(int n0, int n1, int n2, int h2, int t0, int t1, int t2) {
   HalfConfig c;
   c.reg0 = reg_supported(n0);
   c.reg1 = reg_supported(n1);
-  c.p0 = make_line_plan(n0);
-  c.p1 = make_line_plan(n1);
-  c.w0 = std::max(1, std::min(h2, kTile / n0));
-  c.w1 = std::max(1, std::min(h2, kTile / n1));
-  c.smt = sizeof(float2) * (n1 + n2 + (size_t)n1 * c.w1) + sizeof(float) * t1 * t2;
-  c.smx = sizeof(float2) * (n0 + (size_t)n0 * c.w0);
-  c.smy = sizeof(float2) * (n1 + (size_t)n1 * c.w1);
+  const size_t plane = sizeof(float) * t1 * t2;
+  const auto zy = [&](const HalfLine& p) {
+    return sizeof(float2) * (p.n + n2 + ((size_t)2 * p.n << p.lw));
+  };
+  const auto x = [&](const HalfLine& p) {
+    return sizeof(float2) * (p.n + ((size_t)(3 * p.n + t0) << p.lw));
+  };
+  const auto y = [&](const HalfLine& p) {
+    return sizeof(float2) * (p.n + ((size_t)2 * p.n << p.lw)) +
+           sizeof(__half2) * ((((size_t)p.n << p.lw) + 1) & ~(size_t)1);
+  };
+  c.t = half_line(n1, h2, [&](const HalfLine& p) { return zy(p) + plane; });
+  c.x = half_line(n0, h2, x);
+  c.y = half_line(n1, h2, y);
+  c.wide = zy(c.t) + plane <= 226 * 1024;
+  c.smt = zy(c.t) + (c.wide ? plane : 0);
+  c.smx = x(c.x);
+  c.smy = y(c.y);
   if (c.reg1) {
     size_t zy = 0;
     TM_DISPATCH_N(n1, (zy = reg_smem_bytes<NN>(n2, t1, t2, true)));
@@ -535,14 +784,14 @@ int half_prepare(const HalfConfig& c, int n0, int n1) {
     TM_DISPATCH_N(n0, TM_TRY((raise(xpass_reg_kernel<NN, reg_lines<NN>(), __half2>))));
     TM_DISPATCH_N(n0, TM_TRY((raise(xpass_reg_kernel<NN, reg_lines<NN>(), __half2, true>))));
   } else {
-    TM_TRY(raise(xpass_kernel<__half2>));
+    TM_TRY(raise(xpass_kernel));
   }
   if (c.reg1) {
     TM_DISPATCH_N(n1, TM_TRY((raise(ypass_reg_kernel<NN, reg_lines<NN>(), __half2>))));
     TM_DISPATCH_N(n1, TM_TRY((raise(tmpl_zy_reg_kernel<NN, reg_lines<NN>(), float2>))));
     TM_DISPATCH_N(n1, TM_TRY((raise(tmpl_zy_reg_kernel<NN, reg_lines<NN>(), __half2>))));
   } else {
-    TM_TRY(raise(ypass_kernel<__half2>));
+    TM_TRY(raise(ypass_kernel));
     TM_TRY(raise(tmpl_zy_kernel));
   }
   return TM_OK;
@@ -564,9 +813,9 @@ int half_template(const HalfConfig& c, const float* tmpl, int nb, int t0, int t1
             tmpl, t0, t1, t2, n2, h2, tw1, tw2, static_cast<float2*>(G));
     }));
   } else {
-    const dim3 g((unsigned)ceil_div(h2, c.w1), t0, nb);
-    tmpl_zy_kernel<<<g, kThreads, c.smt, st>>>(tmpl, t0, t1, t2, n1, n2, h2, c.w1, c.p1, tw1, tw2,
-                                               static_cast<float2*>(G));
+    const dim3 g((unsigned)ceil_div(h2, 1 << c.t.lw), t0, nb);
+    tmpl_zy_kernel<<<g, c.t.threads(), c.smt, st>>>(tmpl, t0, t1, t2, n2, h2, c.wide, c.t, tw1,
+                                                    tw2, static_cast<float2*>(G));
   }
   return check_launch("template pass");
 }
@@ -587,9 +836,12 @@ int half_xpass(const HalfConfig& c, const float2* G, const float2* Ft, int nb, i
             G, Ft, nb, t0, n1, h2, tw0, scale, static_cast<__half2*>(H), hp);
     }));
   } else {
-    const dim3 g((unsigned)ceil_div(h2, c.w0), n1);
-    xpass_kernel<__half2><<<g, kThreads, c.smx, st>>>(G, Ft, nb, t0, n0, n1, h2, c.w0, c.p0, tw0,
-                                                     scale, static_cast<__half2*>(H), hp);
+    const int64_t columns = ceil_div(h2, 1 << c.x.lw);
+    const int64_t chunks = std::min<int64_t>(nb, std::max<int64_t>(1, 148 * 16 / (columns * n1)));
+    const int per = (int)ceil_div(nb, chunks);
+    const dim3 g((unsigned)columns, n1, (unsigned)ceil_div(nb, per));
+    xpass_kernel<<<g, c.x.threads(), c.smx, st>>>(G, Ft, nb, per, t0, n1, h2, c.x, tw0, scale,
+                                                  static_cast<__half2*>(H), hp);
   }
   return check_launch("x pass");
 }
@@ -605,8 +857,11 @@ int half_ypass(const HalfConfig& c, void* H, int nb, int n0, int n1, int h2, int
           h, n0, h2, tw1, hp, seg ? 1 : 0);
     }));
   } else {
-    const dim3 g((unsigned)ceil_div(h2, c.w1), n0, nb);
-    ypass_kernel<__half2><<<g, kThreads, c.smy, st>>>(h, n0, n1, h2, c.w1, c.p1, tw1, hp);
+    const int64_t columns = ceil_div(h2, 1 << c.y.lw);
+    int planes = 8;
+    while (planes > 1 && columns * nb * ceil_div(n0, planes) < 148 * 8) planes /= 2;
+    const dim3 g((unsigned)columns, (unsigned)ceil_div(n0, planes), nb);
+    ypass_kernel<<<g, c.y.threads(), c.smy, st>>>(h, planes, n0, h2, c.y, tw1, hp);
   }
   return check_launch("y pass");
 }

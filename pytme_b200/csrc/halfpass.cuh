@@ -4,18 +4,27 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 
-#include "fft_smem.cuh"
-
 namespace tmb {
 
-struct HalfConfig {
-  bool reg0 = false, reg1 = false;  // register-resident columns along x / y
-  fft::LinePlan p0{}, p1{};
-  int w0 = 1, w1 = 1;               // lines of a tile of the other lengths
-  size_t smt = 0, smx = 0, smy = 0;  // their shared memory
+// Stockham transforms of 2^lw interleaved lines of length n by slots x 2^lw threads.
+struct HalfLine {
+  static constexpr int kStages = 12;
+  int n = 0, stages = 0, lw = 0, slots = 1;
+  int radix[kStages] = {};
+  int before[kStages] = {};     // product of the radices before a stage
+  unsigned recip[kStages] = {};  // ceil(2^32 / before)
+  int step[kStages] = {};       // n / (before * radix): steps of the roots of unity
+  int threads() const { return slots << lw; }
 };
 
-HalfConfig half_config(int n0, int n1, int n2, int h2, int t1, int t2);
+struct HalfConfig {
+  bool reg0 = false, reg1 = false;   // register-resident columns along x / y
+  HalfLine t, x, y;                  // of the other lengths: template, x and y pass
+  size_t smt = 0, smx = 0, smy = 0;  // their shared memory
+  bool wide = true;                  // the template pass stages a template plane
+};
+
+HalfConfig half_config(int n0, int n1, int n2, int h2, int t0, int t1, int t2);
 int half_prepare(const HalfConfig& c, int n0, int n1);
 // G[b][x][k1][h2] as complex64 or (register-resident y columns) half2.
 int half_template(const HalfConfig& c, const float* tmpl, int nb, int t0, int t1, int t2, int n1,

@@ -31,7 +31,7 @@
 #include <cstdint>
 #include <vector>
 
-#include "fft_smem.cuh"
+#include "dft.cuh"
 
 namespace tmb {
 namespace linefft {

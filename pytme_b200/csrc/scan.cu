@@ -28,7 +28,7 @@
 // are computed once by set_target; the denominator and the target mean are
 // evaluated in double precision.
 #include "common.cuh"
-#include "fft_smem.cuh"
+#include "dft.cuh"
 #include "genpass.cuh"
 #include "halfpass.cuh"
 #include "ops.cuh"
@@ -861,7 +861,7 @@ int scan_create(const tm_scan_desc* desc, Scan** out, bool any_length) {
       }
       int st = gen_prepare(s->gen, d.score == TM_SCORE_FLC, s->half);
       if (st == TM_OK && s->half) {
-        s->hc = half_config(s->n0, s->n1, s->n2, s->h2, s->t1, s->t2);
+        s->hc = half_config(s->n0, s->n1, s->n2, s->h2, s->t0, s->t1, s->t2);
         st = half_prepare(s->hc, s->n0, s->n1);
       }
       if (st != TM_OK) { destroy(s); return st; }

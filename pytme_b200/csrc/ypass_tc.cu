@@ -34,7 +34,7 @@
 // leave, the copies and MMAs in flight are waited for and the tensor memory is freed.
 // No load here uses cluster multicast.
 #include "common.cuh"
-#include "fft_smem.cuh"
+#include "dft.cuh"
 #include "tc_common.cuh"
 #include "ypass_tc.cuh"
 
