@@ -451,59 +451,140 @@ __device__ __forceinline__ void dif_rest(float2 (&v)[8], float2* sm, const float
   }
 }
 
-// K1': template rows -> G. grid (ceil(h2/W), t0, B); N = n1.
-template <int N, int W, typename GT = float2>
-__global__ void __launch_bounds__(N / 8 * W, 1)
-tmpl_zy_reg_kernel(const float* __restrict__ tmpl, int t0, int t1, int t2, int n2, int h2,
-                   const float2* __restrict__ tw1_g, const float2* __restrict__ tw2_g,
+// Stages 1.. of the template rows' columns and the first one of rows [0, t1) > T, with the
+// operations as they round (see butterfly): the stages of colfft.cuh.
+template <int N, int S>
+__device__ __forceinline__ void template_stage(float2 (&v)[8], int t, const float2* tw) {
+  constexpr int L = colfft::stage_size(N, S), R = colfft::stage_radix(N, S);
+  constexpr int NB = 8 / R, LR = L / R;
+#pragma unroll
+  for (int i = 0; i < NB; ++i) {
+    butterfly<R, -1>(&v[i * R]);
+    if constexpr (LR > 1) {
+      const float2 w1 = tw[(t * NB + i) % LR * (N / L)];
+      float2 w = w1;
+#pragma unroll
+      for (int j = 1; j < R; ++j) {
+        v[i * R + j] = turn(v[i * R + j], w);
+        if (j + 1 < R) w = filter(w, w1);
+      }
+    }
+  }
+}
+
+template <int N, int W, int S>
+__device__ __forceinline__ void template_stages(float2 (&v)[8], float2* sm, const float2* tw,
+                                                int l, int t) {
+  if constexpr (S < colfft::num_stages(N)) {
+    colfft::store_stage<N, W, S - 1>(v, sm, l, t);
+    __syncthreads();
+    colfft::load_stage<N, W, S>(v, sm, l, t);
+    template_stage<N, S>(v, t, tw);
+    template_stages<N, W, S + 1>(v, sm, tw, l, t);
+  }
+}
+
+// K1': template rows -> G. grid (ceil(h2/W), ceil(t0/planes), B); N = n1. Shared-memory
+// wavefronts of the direct DFT along z bound the pass: with one plane a turn each product
+// reads its value and its root, the latter from a table of n2 with three to four wavefronts a
+// read. Templates of at most T rows (P = 4) are taken four planes a turn, a value of each in
+// one read, with the tile's columns of roots in order of use: 512 x 512 x 200, 48^3 template,
+// 32 rotations 436 -> 253 us; 256 x 256 x 128, 32^3 template, 32 rotations 110 -> 59.
+template <int N, int W, int P, typename GT = float2>
+__global__ void __launch_bounds__(N / 8 * W, 1024 / (N / 8 * W))
+tmpl_zy_reg_kernel(const float* __restrict__ tmpl, int planes, int t0, int t1, int t2, int n2,
+                   int h2, const float2* __restrict__ tw1_g, const float2* __restrict__ tw2_g,
                    GT* __restrict__ G) {
   constexpr int T = N / 8;
   constexpr int NT = T * W;
   extern __shared__ float4 smem_raw[];
-  float2* tw1 = reinterpret_cast<float2*>(smem_raw);
+  float* plane = reinterpret_cast<float*>(smem_raw);  // t1 x t2 x P
+  float2* tw1 = reinterpret_cast<float2*>(plane + ((t1 * t2 * P + 1) & ~1));
   float2* sm = tw1 + N;
-  float2* tw2 = sm + colfft::smem_elems<N>(W);
-  float* plane = reinterpret_cast<float*>(tw2 + n2);
+  float2* tw2 = sm + colfft::smem_elems<N>(W);  // P > 1: t2 x W, else n2
   const int tid = threadIdx.x, l = tid % W, t = tid / W;
   const int k2 = blockIdx.x * W + l;
-  const int x = blockIdx.y, b = blockIdx.z;
+  const bool valid = k2 < h2;
   for (int i = tid; i < N; i += NT) tw1[i] = tw1_g[i];
-  for (int i = tid; i < n2; i += NT) tw2[i] = tw2_g[i];
-  const float* src = tmpl + ((int64_t)b * t0 + x) * t1 * t2;
-  for (int i = tid; i < t1 * t2; i += NT) plane[i] = src[i];
-  __syncthreads();
-  float2 v[8];
+  if constexpr (P > 1) {
+    for (int z = t; z < t2; z += T)
+      tw2[z * W + l] = tw2_g[(unsigned)(z * min(k2, h2 - 1)) % (unsigned)n2];
+  } else {
+    for (int i = tid; i < n2; i += NT) tw2[i] = tw2_g[i];
+  }
+  const int area = t1 * t2;
+  const int x1 = min(t0, (int)(blockIdx.y + 1) * planes);
+  for (int x = blockIdx.y * planes; x < x1; x += P) {
+    const float* src = tmpl + ((int64_t)blockIdx.z * t0 + x) * area;
+    const int np = min(P, x1 - x);
+    for (int i = tid; i < area; i += NT) {
+      if constexpr (P > 1)
+        reinterpret_cast<float4*>(plane)[i] =
+            make_float4(src[i], np > 1 ? src[area + i] : 0.f, np > 2 ? src[2 * area + i] : 0.f,
+                        np > 3 ? src[3 * area + i] : 0.f);
+      else
+        plane[i] = src[i];
+    }
+    __syncthreads();
+    float2 v[8], acc[P];
+    if constexpr (P > 1) {
+      static_assert(P == 4, "four planes a read");
 #pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    const int y = t + T * r;
-    float2 acc = make_float2(0.f, 0.f);
-    if (y < t1 && k2 < h2) {
-      const float* row = plane + y * t2;
-      int idx = 0;
-      for (int z = 0; z < t2; ++z) {
-        const float a = row[z];
-        const float2 w = tw2[idx];
-        acc.x += a * w.x;
-        acc.y += a * w.y;
-        idx += k2;
-        if (idx >= n2) idx -= n2;
+      for (int p = 0; p < P; ++p) acc[p] = make_float2(0.f, 0.f);
+      if (t < t1 && valid) {
+        const float4* row = reinterpret_cast<const float4*>(plane) + t * t2;
+#pragma unroll 4
+        for (int z = 0; z < t2; ++z) {
+          const float4 a = row[z];
+          const float2 w = tw2[z * W + l];
+          acc[0] = axpy(a.x, w, acc[0]);
+          acc[1] = axpy(a.y, w, acc[1]);
+          acc[2] = axpy(a.z, w, acc[2]);
+          acc[3] = axpy(a.w, w, acc[3]);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const int y = t + T * r;
+        float2 sum = make_float2(0.f, 0.f);
+        if (y < t1 && valid) {
+          const float* row = plane + y * t2;
+          int idx = 0;
+          for (int z = 0; z < t2; ++z) {
+            sum = axpy(row[z], tw2[idx], sum);
+            idx += k2;
+            if (idx >= n2) idx -= n2;
+          }
+        }
+        v[r] = sum;
       }
     }
-    v[r] = acc;
-  }
-  if (t1 <= T) stage0_single<N>(v, t, tw1);
-  else colfft::dif_stage_regs<N, 0, -1>(v, t, tw1);
-  dif_rest<N, W, -1>(v, sm, tw1, l, t);
-  if (k2 < h2) {
-    GT* dst = G + ((int64_t)b * t0 + x) * N * h2;
-    constexpr int R = colfft::stage_radix(N, colfft::num_stages(N) - 1);
 #pragma unroll
-    for (int i = 0; i < 8 / R; ++i)
+    for (int p = 0; p < P; ++p) {
+      if (p < np) {
+        if (P > 1 || t1 <= T) {
+          // one non-zero input a butterfly: output j is x[t] * W_N^(j*t)
+          if constexpr (P > 1) v[0] = acc[p];
+          const float2 w1 = tw1[t];
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int k1 = colfft::out_index<N>(t, i, r);
-        Store<GT>::store(dst + (int64_t)k1 * h2 + k2, v[i * R + r]);
+          for (int j = 1; j < 8; ++j) v[j] = turn(v[j - 1], w1);
+        } else {
+          template_stage<N, 0>(v, t, tw1);
+        }
+        template_stages<N, W, 1>(v, sm, tw1, l, t);
+        if (valid) {
+          GT* dst = G + (((int64_t)blockIdx.z * t0 + x + p) * N) * h2 + k2;
+          constexpr int R = colfft::stage_radix(N, colfft::num_stages(N) - 1);
+#pragma unroll
+          for (int i = 0; i < 8 / R; ++i)
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+              Store<GT>::store(dst + (int64_t)colfft::out_index<N>(t, i, r) * h2, v[i * R + r]);
+        }
+        __syncthreads();  // the next plane's first exchange, the next planes' values
       }
+    }
   }
 }
 
@@ -663,6 +744,12 @@ size_t reg_smem_bytes(int n2, int t1, int t2, bool with_plane) {
   return b;
 }
 
+template <int N>
+size_t template_smem_bytes(int p, int n2, int t1, int t2) {
+  return reg_smem_bytes<N>(0, 0, 0, false) + sizeof(float) * ((t1 * t2 * p + 1) & ~1) +
+         sizeof(float2) * (p > 1 ? t2 * reg_lines<N>() : n2);
+}
+
 template <int N, typename HT>
 size_t ypass_smem_bytes() {
   return reg_smem_bytes<N>(0, 0, 0, false) + kYStages * sizeof(HT) * N * reg_lines<N>();
@@ -788,8 +875,10 @@ int half_prepare(const HalfConfig& c, int n0, int n1) {
   }
   if (c.reg1) {
     TM_DISPATCH_N(n1, TM_TRY((raise(ypass_reg_kernel<NN, reg_lines<NN>(), __half2>))));
-    TM_DISPATCH_N(n1, TM_TRY((raise(tmpl_zy_reg_kernel<NN, reg_lines<NN>(), float2>))));
-    TM_DISPATCH_N(n1, TM_TRY((raise(tmpl_zy_reg_kernel<NN, reg_lines<NN>(), __half2>))));
+    TM_DISPATCH_N(n1, TM_TRY((raise(tmpl_zy_reg_kernel<NN, reg_lines<NN>(), 1, float2>))));
+    TM_DISPATCH_N(n1, TM_TRY((raise(tmpl_zy_reg_kernel<NN, reg_lines<NN>(), 4, float2>))));
+    TM_DISPATCH_N(n1, TM_TRY((raise(tmpl_zy_reg_kernel<NN, reg_lines<NN>(), 1, __half2>))));
+    TM_DISPATCH_N(n1, TM_TRY((raise(tmpl_zy_reg_kernel<NN, reg_lines<NN>(), 4, __half2>))));
   } else {
     TM_TRY(raise(ypass_kernel));
     TM_TRY(raise(tmpl_zy_kernel));
@@ -803,14 +892,27 @@ int half_template(const HalfConfig& c, const float* tmpl, int nb, int t0, int t1
   if (c.reg1) {
     TM_DISPATCH_N(n1, ({
       constexpr int W = reg_lines<NN>();
-      const dim3 g((unsigned)ceil_div(h2, W), t0, nb);
-      const size_t smem = reg_smem_bytes<NN>(n2, t1, t2, true);
-      if (half_g)
-        tmpl_zy_reg_kernel<NN, W, __half2><<<g, NN / 8 * W, smem, st>>>(
-            tmpl, t0, t1, t2, n2, h2, tw1, tw2, static_cast<__half2*>(G));
-      else
-        tmpl_zy_reg_kernel<NN, W, float2><<<g, NN / 8 * W, smem, st>>>(
-            tmpl, t0, t1, t2, n2, h2, tw1, tw2, static_cast<float2*>(G));
+      // Four planes a turn where the rows are few, two CTAs (of 1024 threads one) still fit an
+      // SM and enough CTAs are left; eight planes a CTA where that leaves several an SM.
+      const int64_t columns = ceil_div(h2, W) * nb;
+      const size_t wide = template_smem_bytes<NN>(4, n2, t1, t2);
+      const bool four = t1 <= NN / 8 && columns * ceil_div(t0, 4) >= 148 * 2 &&
+                        wide <= (NN / 8 * W > 512 ? 226 : 113) * 1024;
+      const int planes = !four ? 1 : columns * ceil_div(t0, 8) >= 148 * 8 ? 8 : 4;
+      const dim3 g((unsigned)ceil_div(h2, W), (unsigned)ceil_div(t0, planes), nb);
+      const size_t smem = four ? wide : template_smem_bytes<NN>(1, n2, t1, t2);
+      auto run = [&](auto kernel, auto* out) {
+        kernel<<<g, NN / 8 * W, smem, st>>>(tmpl, planes, t0, t1, t2, n2, h2, tw1, tw2, out);
+      };
+      if (half_g) {
+        __half2* out = static_cast<__half2*>(G);
+        if (four) run(tmpl_zy_reg_kernel<NN, W, 4, __half2>, out);
+        else run(tmpl_zy_reg_kernel<NN, W, 1, __half2>, out);
+      } else {
+        float2* out = static_cast<float2*>(G);
+        if (four) run(tmpl_zy_reg_kernel<NN, W, 4, float2>, out);
+        else run(tmpl_zy_reg_kernel<NN, W, 1, float2>, out);
+      }
     }));
   } else {
     const dim3 g((unsigned)ceil_div(h2, 1 << c.t.lw), t0, nb);

@@ -48,16 +48,10 @@ def test_any_length_matches_oracle(shape, score, order):
     assert np.all(best - np.where(res[2] < 0, 0.0, picked) <= 2 * tol)
 
 
-@pytest.mark.gpu
-@pytest.mark.parametrize("shape", [(8, 40, 32), (40, 9, 18), (320, 320, 20), (160, 64, 60),
-                                   (64, 100, 48), (810, 48, 30), (20, 1500, 24), (3000, 24, 20),
-                                   (18, 4050, 20)])
-def test_mixed_passes_of_smooth_lengths(shape):
-    """Mixed-precision plans whose x or y length is 5-smooth but no power of two: one to seven
-    stages, tiles of sixteen lines down to one, a last tile with idle lines, chunks of
-    rotations and planes, next to register-resident axes. The spectra are stored twice as half2,
-    so a score is off by about 2^-11 of the map's RMS at most of the time and by a few of that
-    at worst; 2e-3 of it, or 1e-4 where scores are small, is the bound of such plans."""
+def _mixed_against_fp32(shape, rotations, batch):
+    """A mixed-precision plan against an FP32 one. The spectra are stored twice as half2, so a
+    score is off by about 2^-11 of the map's RMS at most of the time and by a few of that at
+    worst; 2e-3 of it, or 1e-4 where scores are small, is the bound of such plans."""
     import torch
 
     from pytme_b200 import synthetic as syn
@@ -69,12 +63,12 @@ def test_mixed_passes_of_smooth_lengths(shape):
     tmpl = syn.blob_template(t, rng, radius=2.0, sigma=1.0)
     mask = syn.spherical_mask((t,) * 3, 3.5, center=(3.0,) * 3)
     target, _, _ = syn.make_tomogram(shape, tmpl, 2, rng, scale=0.5)
-    rots = syn.random_rotation_matrices(5, rng)
+    rots = syn.random_rotation_matrices(rotations, rng)
     mats = torch.as_tensor(rigid_transform_matrices(
         rots, (np.asarray(tmpl.shape) - 1) / 2), device="cuda")
     maps = {}
     for precision in ("fp32", "mixed"):
-        plan = ScanPlan("FLCSphericalMask", shape, tmpl.shape, batch=3, precision=precision)
+        plan = ScanPlan("FLCSphericalMask", shape, tmpl.shape, batch=batch, precision=precision)
         assert plan.precision == precision and not (precision == "mixed" and plan.plain)
         plan.set_template(tmpl[::-1, ::-1, ::-1], mask[::-1, ::-1, ::-1])
         plan.set_target(target)
@@ -85,6 +79,24 @@ def test_mixed_passes_of_smooth_lengths(shape):
     rms = np.sqrt(np.mean(maps["fp32"] ** 2))
     assert rms > 0
     assert np.abs(maps["mixed"] - maps["fp32"]).max() <= max(1e-4, 2e-3 * rms)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(8, 40, 32), (40, 9, 18), (320, 320, 20), (160, 64, 60),
+                                   (64, 100, 48), (810, 48, 30), (20, 1500, 24), (3000, 24, 20),
+                                   (18, 4050, 20)])
+def test_mixed_passes_of_smooth_lengths(shape):
+    """Axes whose x or y length is 5-smooth but no power of two: one to seven stages, tiles of
+    sixteen lines down to one, a last tile with idle lines, chunks of rotations and planes,
+    next to register-resident axes."""
+    _mixed_against_fp32(shape, 5, 3)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(16, 64, 100), (64, 256, 60), (16, 512, 200), (16, 1024, 100)])
+def test_mixed_template_four_planes(shape):
+    """Launch groups large enough for four template planes a turn, the last one of three."""
+    _mixed_against_fp32(shape, 70, 64)
 
 
 @pytest.mark.gpu
