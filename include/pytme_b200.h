@@ -144,7 +144,8 @@ typedef struct {
 typedef struct tm_scan tm_scan;
 
 /* Creates a plan and allocates its device scratch. Returns TM_E_UNSUPPORTED for
- * shapes the fused path does not handle (the plain path handles every shape). */
+ * shapes its fused passes do not handle (tm_scan_create_any_length takes most of
+ * them, the plain path every shape). */
 int tm_scan_create(const tm_scan_desc* desc, tm_scan** plan);
 /* A fused FP32 plan for shapes tm_scan_create refuses with TM_E_UNSUPPORTED: axes of any
  * length 2^a 3^b 5^c 7^d 11^e 13^f up to 4096 (odd ones along z too, and FLC at any of

@@ -9,6 +9,9 @@ namespace {
 // ------------------------------------------------------------------ template pass
 // grid (hp / w, ceil(t0 / planes), nb). Direct real DFT along z of the t1 x t2 plane for
 // the tile's w columns (t2 of n2 inputs are non-zero), then the zero-padded FFT along y.
+// Bound by the shared-memory reads of the DFT: the tile's columns of roots lie in order of
+// use, and several planes share them. 64 rotations at 320 x 320 x 160 with a 40^3 template
+// 0.37 ms (1.2 with a table of n2 roots and a generic Stockham transform).
 template <int W>
 __global__ void __launch_bounds__(kMaxThreads, 2)
 gen_template_kernel(const float* __restrict__ tmpl, int planes, int t0, int t1, int t2, int n2, int h2,
@@ -112,7 +115,9 @@ line_fft_test_kernel(const float2* x, float2* y, const Plan p, const float4* tw_
 // ------------------------------------------------------------------ y pass
 // grid (hp / w, ceil(n0 / planes), nb): inverse FFT along y, in place. The next plane's
 // columns are copied to shared memory (16 bytes at a time) while the later stages of the
-// current one run.
+// current one run: bound by the memory, 5.3 TB/s (64 rotations at 320 x 320 x 160 1.65 ms;
+// 2.66 with the first stage reading global memory itself, 10.1 as a generic Stockham
+// transform of one 512-thread CTA an SM).
 template <int W>
 __global__ void __launch_bounds__(kMaxThreads, 2)
 gen_ypass_kernel(float2* __restrict__ H, int planes, int n0, const Plan p, const float4* __restrict__ tw_g,

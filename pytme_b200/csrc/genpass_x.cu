@@ -9,6 +9,11 @@ namespace {
 // with the target spectrum, inverse FFT, H written. The column of the target, times the scale
 // of H, stays in shared memory for all rotations, in the order of the tile: the product reads
 // it at constant offsets. The next rotation's few input rows are copied in meanwhile.
+// Bound by instruction issue (60 to 71 % of the slots) and the latency of the exchanges: the
+// radices are as large as fit the registers, so that most lengths exchange once each way, and
+// the last forward stage, the product and the first inverse stage share them. 64 rotations at
+// 320 x 320 x 160 with a 40^3 template 2.61 ms (3.06 with the target read from the L2 for every
+// rotation, 14.9 as generic Stockham transforms of one 512-thread CTA an SM).
 template <int W>
 __global__ void __launch_bounds__(kMaxThreads, 2)
 gen_xpass_kernel(const float2* __restrict__ G, const float2* __restrict__ Ft, int B, int per,

@@ -10,19 +10,20 @@
 //    straightforward FP32 GPU port of the reference loop and serves as the
 //    "plain" baseline.
 //
-//  * fused: B rotations per launch group through four kernels of this library.
-//      K1 tmpl_zy    template rows: direct real DFT along axis 2 (only t2 of n2
-//                    inputs are non-zero) and a zero-padded FFT along axis 1,
-//                    producing G[b][x < t0][k1][k2]
-//      K2 xpass      per (k1, k2-tile) column block: forward FFT along axis 0 of
-//                    the zero-padded G columns, product with the target spectrum
-//                    (held in registers for all B rotations), inverse FFT along
-//                    axis 0 -> H[b][x'][k1][k2]
-//      K3 ypass      inverse FFT along axis 1, in place on H
-//      K4 zpass      c2r along axis 2 (half-length complex FFT), score scaling and
-//                    the strict-> max/argmax over the B rotations in registers,
-//                    merged into the caller's state once per launch group
-//    H is complex64 ("fp32") or half2 with a fixed scale ("mixed").
+//  * fused: B rotations per launch group through four passes of this library.
+//      template  rows: direct real DFT along axis 2 (only t2 of n2 inputs are
+//                non-zero) and a zero-padded FFT along axis 1, producing
+//                G[b][x < t0][k1][k2]
+//      x pass    per (k1, k2-tile) column block: forward FFT along axis 0 of the
+//                zero-padded G columns, product with the target spectrum (held on
+//                chip for the rotations of a CTA), inverse FFT along axis 0 -> H
+//      y pass    inverse FFT along axis 1, in place on H
+//      z pass    c2r along axis 2, score scaling and the strict-> max/argmax over
+//                the B rotations, merged into the caller's state once per group
+//    H is complex64 ("fp32") or half2 with a fixed scale ("mixed"). FP32 passes are
+//    line FFTs of any length (genpass.cuh), mixed ones register or Stockham columns
+//    (halfpass.cuh) or the tensor-core kernels; z4 below is the four-step z pass of
+//    some half-lengths.
 //
 // Target-side quantities (target spectra and the FLCSphericalMask denominator)
 // are computed once by set_target; the denominator and the target mean are
