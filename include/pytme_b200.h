@@ -123,8 +123,9 @@ int tm_fft_c2r(tm_fft_plan* plan, void* in, void* out, double scale, void* strea
 /* Template filter at template shape (_apply_filter_subset of _create_filter_func,
  * tme/matching_scores.py:90-135): x = irfftn(rfftn(x) * filter) in place for every
  * batch item of a single-precision plan. `filter` holds one real value per rfft
- * element of one item and is shared by all items; `spectrum` holds the plan's
- * complex output (batch x rfft elements). */
+ * element of one item and is shared by all items; `spectrum` has room for the plan's
+ * complex output (batch x rfft elements) and is scratch: small 3-D items are filtered in
+ * shared memory and leave it alone. */
 int tm_fft_filter(tm_fft_plan* plan, float* x, void* spectrum, const float* filter,
                   void* stream);
 

@@ -2,6 +2,7 @@
 // argument checking lives here and in the ops.
 #include "common.cuh"
 #include "diagnostics.h"
+#include "fftfilter.cuh"
 #include "ops.cuh"
 #include "peaks.cuh"
 #include "refine.cuh"
@@ -10,6 +11,7 @@
 
 #include <cufft.h>
 
+#include <algorithm>
 #include <string>
 
 struct tm_fft_plan {
@@ -19,6 +21,7 @@ struct tm_fft_plan {
   int64_t n_item = 0;   // real elements per batch item
   int64_t n_ft = 0;     // complex elements per batch item
   int batch = 1;
+  int n[3] = {0, 0, 0};  // the shape of 3-D plans
 };
 
 struct tm_scan {
@@ -133,6 +136,7 @@ int tm_fft_plan_create(int ndim, const int* shape, int batch, int double_precisi
   p->n_item = nr;
   p->n_ft = nr / n[ndim - 1] * (n[ndim - 1] / 2 + 1);
   p->batch = batch;
+  if (ndim == 3) std::copy(n, n + 3, p->n);
   cufftResult r = cufftPlanMany(&p->fwd, ndim, n, nullptr, 1, 0, nullptr, 1, 0,
                                 p->dbl ? CUFFT_D2Z : CUFFT_R2C, batch);
   if (r == CUFFT_SUCCESS)
@@ -363,6 +367,8 @@ int tm_line_fft_test(const void* x, void* y, int n, int lines, int dir, void* st
 int tm_fft_filter(tm_fft_plan* p, float* x, void* spectrum, const float* filter, void* stream) {
   TM_REQUIRE(p && x && spectrum && filter, "tm_fft_filter: null pointer");
   TM_REQUIRE(!p->dbl, "tm_fft_filter: single-precision plans only");
+  if (p->n[0] && tmb::fft_filter_supported(p->n, p->batch))
+    return tmb::fft_filter(x, filter, p->n, p->batch, S(stream));
   TM_TRY(tm_fft_r2c(p, x, spectrum, stream));
   // the inverse transform's scale goes in with the filter
   TM_TRY(tmb::apply_real_filter(spectrum, filter, p->n_ft, p->batch, S(stream),
