@@ -30,6 +30,7 @@
 // evaluated in double precision.
 #include "common.cuh"
 #include "dft.cuh"
+#include "fftfilter.cuh"
 #include "genpass.cuh"
 #include "halfpass.cuh"
 #include "ops.cuh"
@@ -888,6 +889,13 @@ static int need_inv(Scan* s) {
   return TM_OK;
 }
 
+// Template filter in shared memory, one launch where cuFFT takes five or more. Mixed plans keep
+// cuFFT: its rounding reaches their half spectra, where a last bit becomes one of 2^-11.
+static bool own_filter(const Scan* s) {
+  const int shape[3] = {s->t0, s->t1, s->t2};
+  return !s->half && fft_filter_supported(shape, s->B);
+}
+
 static int need_template_plans(Scan* s) {
   if (s->have_tfwd) return TM_OK;
   int ts[3] = {s->t0, s->t1, s->t2};
@@ -1125,7 +1133,7 @@ int scan_set_template(Scan* s, const float* tmpl, const float* mask, const float
   TM_REQUIRE(s->d.score == TM_SCORE_CC || mask, "scan_set_template: this score needs a mask");
   cudaMemcpyAsync(s->tmpl, tmpl, sizeof(float) * s->T, cudaMemcpyDeviceToDevice, stream);
   if (mask) cudaMemcpyAsync(s->mask, mask, sizeof(float) * s->T, cudaMemcpyDeviceToDevice, stream);
-  if (filt) TM_TRY(need_template_plans(s));
+  if (filt && !own_filter(s)) TM_TRY(need_template_plans(s));
   s->d.has_template_filter = filt != nullptr;
   if (filt) cudaMemcpyAsync(s->tfilter, filt, sizeof(float) * s->TS, cudaMemcpyDeviceToDevice, stream);
   if (mask) {
@@ -1184,12 +1192,17 @@ static int prepare_templates(Scan* s, int nb, cudaStream_t stream) {
                            s->rot_t, flc ? s->rot_m : nullptr, s->t0, s->t1, s->t2, stream));
   if (s->d.has_template_filter) {
     // _apply_filter_subset (tme/matching_scores.py:125-135): rfftn -> * filter -> irfftn
-    cufftSetStream(s->tfwd, stream);
-    cufftSetStream(s->tinv, stream);
-    TM_TRY(cufft_status(cufftExecR2C(s->tfwd, s->rot_t, (cufftComplex*)s->tspec), "filter r2c"));
-    TM_TRY(apply_real_filter(s->tspec, s->tfilter, s->TS, s->B, stream));
-    TM_TRY(cufft_status(cufftExecC2R(s->tinv, (cufftComplex*)s->tspec, s->rot_t), "filter c2r"));
-    TM_TRY(scale_real(s->rot_t, (float)(1.0 / (double)s->T), s->T * s->B, stream));
+    const int shape[3] = {s->t0, s->t1, s->t2};
+    if (own_filter(s)) {
+      TM_TRY(fft_filter(s->rot_t, s->tfilter, shape, nb, stream));
+    } else {
+      cufftSetStream(s->tfwd, stream);
+      cufftSetStream(s->tinv, stream);
+      TM_TRY(cufft_status(cufftExecR2C(s->tfwd, s->rot_t, (cufftComplex*)s->tspec), "filter r2c"));
+      TM_TRY(apply_real_filter(s->tspec, s->tfilter, s->TS, s->B, stream));
+      TM_TRY(cufft_status(cufftExecC2R(s->tinv, (cufftComplex*)s->tspec, s->rot_t), "filter c2r"));
+      TM_TRY(scale_real(s->rot_t, (float)(1.0 / (double)s->T), s->T * s->B, stream));
+    }
   }
   if (s->d.score == TM_SCORE_FLCSM) {
     TM_TRY(normalize_template(s->rot_t, s->mask, 0, s->t0, s->t1, s->t2, s->t1, s->t2, s->T, nb,
