@@ -630,10 +630,11 @@ int refine_backward(const RefineArgs& a, const float* Tf, const float* gTr, cons
   float4* q = nullptr;
   if (grad_tmpl) {
     q = static_cast<float4*>(workspace);
-    if (!q)
+    if (!q) {
       TM_TRY(cuda_status(cudaMallocAsync((void**)&q, sizeof(float4) * (size_t)nv, st),
                          "refine_backward: workspace"));
-    cudaMemsetAsync(q, 0, sizeof(float4) * (size_t)nv, st);
+      cudaMemsetAsync(q, 0, sizeof(float4) * (size_t)nv, st);
+    }
   }
   auto fn = Tf ? refine_backward_kernel<true> : refine_backward_kernel<false>;
   const int g = resident_grid((const void*)fn, kRefThreads, 0, a.P);

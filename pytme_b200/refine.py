@@ -285,14 +285,16 @@ class FLCRefineFunction(torch.autograd.Function):
         P = int(sums.shape[0])
         dev = sums.device
         g = grad_scores.detach().to(dtype=torch.float32).contiguous()
-        g_ang = torch.zeros((P, 3), dtype=torch.float64, device=dev)
-        g_sh = torch.zeros((P, 3), dtype=torch.float64, device=dev)
-        g_t = torch.zeros(tmpl.shape, dtype=torch.float32, device=dev) \
-            if ctx.needs_input_grad[0] else None
+        g_pose = torch.zeros((2, P, 3), dtype=torch.float64, device=dev)
+        g_ang, g_sh = g_pose
+        g_t = work = None
+        if ctx.needs_input_grad[0]:  # the template gradient and its workspace, zeroed at once
+            n = tmpl.numel()
+            work, g_t = torch.zeros((5 * n,), dtype=torch.float32, device=dev).split((4 * n, n))
         st = N.stream_ptr()
-        work = None if g_t is None else torch.empty((tmpl.numel(), 4), dtype=torch.float32,
-                                                    device=dev)
         for lo, hi in problem.chunks(P):
+            if lo and work is not None:
+                work.zero_()
             d = problem.desc(tmpl, rot, sh, cor, lo, hi)
             tf = gbuf = None
             if problem.filtered:
@@ -312,7 +314,8 @@ class FLCRefineFunction(torch.autograd.Function):
                                                 N.ptr(g_ang[lo:hi]), N.ptr(g_t), N.ptr(work),
                                                 st), "tm_refine_backward_ws")
         gt = None if g_t is None else g_t.reshape(ctx.template_shape)
-        return gt, g_ang.to(torch.float32), g_sh.to(torch.float32), None, None
+        g_ang, g_sh = g_pose.to(torch.float32)
+        return gt, g_ang, g_sh, None, None
 
 
 def refine_score(problem: RefineProblem, corners, angles, shifts=None,
