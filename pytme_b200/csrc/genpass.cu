@@ -17,8 +17,8 @@ size_t even_tile(const Plan& p, int w, int tiles) {
   return 16 * p.pairs + sizeof(float2) * (((size_t)w * p.rows * tiles + 1) & ~(size_t)1);
 }
 size_t smem_y(const Plan& p, int w) { return even_tile(p, w, 1) + sizeof(float2) * w * p.n; }
-// z pass: tiles, the staged rows (for FLC see flc_staged), and per voxel of 2 w rows the maximum, its rotation and (not
-// for FLC) the inverse denominator
+// z pass: tiles, the staged rows (for FLC see flc_staged), and per voxel of 2 w rows the
+// maximum, its rotation and (not for FLC) the inverse denominator
 size_t smem_z(const Plan& p, int w, int hp, bool flc, bool half) {
   const size_t wide = sizeof(float2) * staged_pitch<float2>(hp);
   const size_t own = half ? sizeof(__half2) * staged_pitch<__half2>(hp) : wide;

@@ -4,7 +4,8 @@
 // holds all radices; genpass.cu chooses plans and tiles.
 //
 // Every pass moves tiles of W = 8 neighbouring k2 columns (one 64-byte segment of complex64,
-// 32 bytes of half2). Tiles of fewer lines serve the lengths whose eight-line tile does not fit in shared memory.
+// 32 bytes of half2). Tiles of fewer lines serve the lengths whose eight-line tile does not fit
+// in shared memory.
 #pragma once
 
 #include <cuda_fp16.h>

@@ -20,8 +20,8 @@
 // Twiddles come from tables in shared memory (no recurrences: a value is one rounding from
 // the exact root), for each stage a row of R roots, padded to an even count, per q: a
 // butterfly reads two of its roots at a time, at constant offsets. Lanes of a warp cover W = 8
-// lines and 4 neighbouring butterflies, so a table read is a broadcast, and rows of the tile (8 complex values, 16
-// banks) are grouped by R_last with an odd group pitch, which lets the four butterflies
+// lines and 4 neighbouring butterflies, so a table read is a broadcast, and rows of the tile
+// (8 complex values, 16 banks) are grouped by R_last with an odd group pitch, which lets the four butterflies
 // alternate between the two halves of the banks in every stage.
 #pragma once
 
@@ -277,8 +277,9 @@ inline void search(int n, int left, int hi, int* cur, int depth, int stages, int
 }
 }  // namespace detail
 
-// The plan of a length (ns = 0 where the length is not supported), but for its slots. Radices ascend, so the first stage, which reads global memory, has
-// the most butterflies and the shortest non-zero part of a zero-padded input.
+// The plan of a length (ns = 0 where the length is not supported), but for its slots. Radices
+// ascend, so the first stage, which reads global memory, has the most butterflies and the
+// shortest non-zero part of a zero-padded input.
 inline Plan make_plan(int n) {
   Plan p;
   if (n < 2 || n > kMaxLength) return p;
