@@ -11,11 +11,12 @@ namespace {
 // it at constant offsets. The next rotation's few input rows are copied in meanwhile.
 // Bound by instruction issue (60 to 71 % of the slots) and the latency of the exchanges: the
 // radices are as large as fit the registers, so that most lengths exchange once each way, and
-// the last forward stage, the product and the first inverse stage share them. 64 rotations at
-// 320 x 320 x 160 with a 40^3 template 2.61 ms (3.06 with the target read from the L2 for every
-// rotation, 14.9 as generic Stockham transforms of one 512-thread CTA an SM).
+// the last forward stage, the product and the first inverse stage share them. 64 registers a
+// thread, some of the largest radices' spilled, for more warps: 64 rotations at 320 x 320 x
+// 160 with a 40^3 template 2.37 ms (2.61 with 80 registers, 14.9 as generic Stockham transforms
+// of one 512-thread CTA an SM), 32 at 468 x 480 x 150 2.82 (3.25).
 template <int W>
-__global__ void __launch_bounds__(kMaxThreads, 2)
+__global__ void __launch_bounds__(512, 2)
 gen_xpass_kernel(const float2* __restrict__ G, const float2* __restrict__ Ft, int B, int per,
                  int t0, int n1, int h2, const Plan p, const float4* __restrict__ tw_g,
                  float scale, float2* __restrict__ H, const HLayout hl) {
